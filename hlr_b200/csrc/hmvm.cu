@@ -26,6 +26,7 @@
 #include "common.hpp"
 #include "hlrc.h"
 #include "kernels_bfp8.cuh"
+#include "kernels_dw.cuh"
 #include "kernels_f64.cuh"
 #include "kernels_mr.cuh"
 #include "kernels_q.cuh"
@@ -94,6 +95,13 @@ struct DevTTPass {
     const TGroup* groups1 = nullptr;  // first finish level (long outputs), into the partial array
     int ngroups1 = 0;
     int64_t npart = 0;
+    // group T-form (products of more than 8 vectors of an FP64 store)
+    const GTSeg* gsegs = nullptr;
+    const GTChunk* gchunks = nullptr;
+    const GTTile* gtiles = nullptr;
+    const TGroup *ggroups = nullptr, *ggroups1 = nullptr;
+    int ngsegs = 0, nggroups = 0, nggroups1 = 0;
+    int64_t gnpart = 0;
     int in = V_X, out = V_T, mode = OUT_SET;
     int64_t bytes = 0, alg_bytes = 0;
     int launches() const {
@@ -108,12 +116,14 @@ struct DevTTPass {
 
 // Scratch used by one product: the coefficient vectors and the partial sums
 // of a one-vector product, and (when present) the same arrays as row-major
-// blocks of MR_RB vectors for the multi-vector kernels.  A product reads
+// blocks of MR_RB (FP64 stores: up to DW_MAXNT * MR_RB) vectors for the
+// multi-vector kernels.  A product reads
 // every scratch entry only after writing it in the same product.
 struct Workspace {
     double* t = nullptr;
     double* t2 = nullptr;
     double* part = nullptr;
+    int mr_nt = 0;               // the multi-vector arrays hold blocks of 8 * mr_nt vectors
     double* mr_x = nullptr;      // null: no multi-vector arrays
     double* mr_t = nullptr;
     double* mr_t2 = nullptr;
@@ -185,6 +195,8 @@ struct hlrc_hmat_s {
     double* ws_t2 = nullptr;
     double* part = nullptr;
     int64_t n_t = 0, n_t2 = 0, n_part = 0;
+    bool blocks = false;               // the plan has the group T-forms (products of more than 8 vectors at a time)
+    int64_t n_gpart = 0;               // their partials, and those of the unit T-forms
     std::vector<DevTPass> t;
     std::vector<DevNPass> n;
     std::vector<DevTTPass> tt;
@@ -194,9 +206,10 @@ struct hlrc_hmat_s {
     bool nf_multi = false;             // multi-vector products take stages_nf too
     Workspace side_ws;                 // the handle's side stream and events (side stages only)
     hlrc_info info{};
-    // multi-RHS workspace (FP64 plans, allocated at upload when max_nrhs > 1):
-    // row-major blocks of MR_RB vectors
+    // multi-RHS workspace (allocated at upload when max_nrhs > 1): row-major
+    // blocks of MR_RB * mr_nt vectors
     char* mr_arena = nullptr;
+    int mr_nt = 0;
     double *mr_x = nullptr, *mr_t = nullptr, *mr_t2 = nullptr, *mr_part = nullptr;
     char* mr_tables = nullptr;   // column streams of reduced-precision stores (MSeg / MCol)
     // one-pass 64-vector products of 16-bit H stores (op N): eligibility and
@@ -727,8 +740,14 @@ hlrc_status enable_tc_smem(int dev) {
 // on DMMA, FP32 columns on DMMA, 16-bit and BFP columns on FP16 MMA).
 bool has_multi_kernels(hlrc_hmat) { return true; }
 
+// Tiles of 8 vectors per pass of a multi-vector product: FP64 handles uploaded
+// for more than 8 vectors take up to DW_MAXNT (kernels_dw.cuh), the others one.
+int mr_tiles(hlrc_hmat M, int max_nrhs) {
+    return M->blocks ? std::max(1, std::min(DW_MAXNT, (max_nrhs + MR_RB - 1) / MR_RB)) : 1;
+}
+
 // Sizes of the multi-vector scratch of a handle: x, t, t2 and the partial
-// sums as row-major blocks of MR_RB vectors, each array 256-byte aligned.
+// sums as row-major blocks of MR_RB * nt vectors, each array 256-byte aligned.
 struct MrSizes {
     size_t nx = 0, nt = 0, nt2 = 0, np = 0, bytes = 0;
     void carve(char* base, double*& x, double*& t, double*& t2, double*& part) const {
@@ -745,12 +764,15 @@ struct MrSizes {
     }
 };
 
-MrSizes mr_sizes(hlrc_hmat M) {
+MrSizes mr_sizes(hlrc_hmat M, int nt) {
+    const size_t rb = size_t(MR_RB) * size_t(nt);
     MrSizes z;
-    z.nx = size_t(std::max(M->nrows, M->ncols)) * MR_RB;
-    z.nt = size_t(std::max<int64_t>(1, M->n_t)) * MR_RB;
-    z.nt2 = size_t(std::max<int64_t>(1, M->n_t2)) * MR_RB;
-    z.np = size_t(std::max<int64_t>(1, M->n_part)) * MR_RB;
+    z.nx = size_t(std::max(M->nrows, M->ncols)) * rb;
+    z.nt = size_t(std::max<int64_t>(1, M->n_t)) * rb;
+    z.nt2 = size_t(std::max<int64_t>(1, M->n_t2)) * rb;
+    // a product whose last pass has one tile runs in the same arrays
+    z.np = std::max(size_t(std::max<int64_t>(1, M->n_part)) * MR_RB,
+                    nt > 1 ? size_t(std::max<int64_t>(1, M->n_gpart)) * rb : 0);
     z.bytes = (z.nx + z.nt + z.nt2 + z.np) * sizeof(double) + 4 * 256;
     return z;
 }
@@ -953,6 +975,67 @@ hlrc_status plan_h_leaves(const hlrc_h_desc& d, hlrc_options o, Plan& p, double 
     const hlrc_h_desc hd{d.nrows, d.ncols, d.nblocks, hl.blocks.data()};
     o.leaves_on_device = 0;
     return plan_h(hd, o, p, area);
+}
+
+// The group T-form tables of an FP64 plan, in an allocation of their own.
+hlrc_status upload_groups(const Plan& p, hlrc_hmat_s* h) {
+    size_t bytes = 0;
+    auto take = [&](size_t b) { const size_t o = bytes; bytes = align_up(bytes + b, 256); return o; };
+    std::vector<std::array<size_t, 5>> off;
+    for (const TTPass& t : p.ttpasses)
+        off.push_back({take(t.gsegs.size() * sizeof(GTSeg)), take(t.gchunks.size() * sizeof(GTChunk)),
+                       take(t.gtiles.size() * sizeof(GTTile)), take(t.ggroups.size() * sizeof(TGroup)),
+                       take(t.ggroups1.size() * sizeof(TGroup))});
+    cudaError_t e = cudaMalloc(&h->mr_tables, std::max<size_t>(bytes, 256));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(HLRC_ERR_OOM, "group T-form tables of %zu bytes: %s", bytes, cudaGetErrorString(e));
+    }
+    auto put = [&](size_t o, const auto& v) {
+        if (e == cudaSuccess && !v.empty())
+            e = cudaMemcpy(h->mr_tables + o, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice);
+    };
+    for (size_t i = 0; i < p.ttpasses.size(); ++i) {
+        const TTPass& t = p.ttpasses[i];
+        DevTTPass& d = h->tt[i];
+        put(off[i][0], t.gsegs);
+        put(off[i][1], t.gchunks);
+        put(off[i][2], t.gtiles);
+        put(off[i][3], t.ggroups);
+        put(off[i][4], t.ggroups1);
+        d.gsegs = reinterpret_cast<const GTSeg*>(h->mr_tables + off[i][0]);
+        d.gchunks = reinterpret_cast<const GTChunk*>(h->mr_tables + off[i][1]);
+        d.gtiles = reinterpret_cast<const GTTile*>(h->mr_tables + off[i][2]);
+        d.ggroups = reinterpret_cast<const TGroup*>(h->mr_tables + off[i][3]);
+        d.ggroups1 = reinterpret_cast<const TGroup*>(h->mr_tables + off[i][4]);
+        d.ngsegs = int(t.gsegs.size());
+        d.nggroups = int(t.ggroups.size());
+        d.nggroups1 = int(t.ggroups1.size());
+        d.gnpart = t.gnpart;
+        h->n_gpart = std::max(h->n_gpart, t.gnpart);
+    }
+    for (const TPass& t : p.tpasses) h->n_gpart = std::max(h->n_gpart, int64_t(t.nslots) * 32);
+    if (e != cudaSuccess) return fail(HLRC_ERR_CUDA, "group T-form table upload failed: %s", cudaGetErrorString(e));
+    h->blocks = true;
+    h->info.device_bytes += int64_t(bytes);
+    return HLRC_OK;
+}
+
+// The group T-forms stage x in more than 48 KB of shared memory; raised once
+// per device, as for the tensor-core kernels.
+hlrc_status enable_dw_smem(int dev) {
+    static std::mutex mu;
+    static std::vector<int> done;
+    std::lock_guard<std::mutex> lock(mu);
+    if (std::find(done.begin(), done.end(), dev) != done.end()) return HLRC_OK;
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<2>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<3>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<4>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<2>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<3>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<4>()));
+    done.push_back(dev);
+    return HLRC_OK;
 }
 
 hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
@@ -1171,13 +1254,31 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
     }
 
     fill_info(p, L, hp->info);
+    if (p.blocks) {
+        hlrc_status st = enable_dw_smem(dev);
+        if (st == HLRC_OK) st = upload_groups(p, hp);
+        if (st != HLRC_OK) {
+            cudaFree(hp->mr_tables);
+            cleanup();
+            return st;
+        }
+    }
     // the 8-vector kernels take FP64, FP32 and FP16/BF16 columns; block
     // floating point (BFP) stores loop the one-vector kernels instead
     if (o.max_nrhs > 1 && has_multi_kernels(hp)) {
-        const MrSizes z = mr_sizes(hp);
-        e = cudaMalloc(&hp->mr_arena, z.bytes);
+        // where the arrays of the widest blocks do not fit, narrower ones do
+        // the same product in more passes
+        MrSizes z;
+        for (int nt = mr_tiles(hp, o.max_nrhs); nt >= 1; --nt) {
+            z = mr_sizes(hp, nt);
+            hp->mr_nt = nt;
+            e = cudaMalloc(&hp->mr_arena, z.bytes);
+            if (e != cudaErrorMemoryAllocation) break;
+            if (nt > 1) cudaGetLastError();
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
+            cudaFree(hp->mr_tables);
             cleanup();
             return fail(HLRC_ERR_OOM, "multi-RHS workspace of %zu bytes: %s", z.bytes, cudaGetErrorString(e));
         }
@@ -1315,6 +1416,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
 Workspace handle_workspace(hlrc_hmat M) {
     Workspace w;
     w.t = M->ws_t; w.t2 = M->ws_t2; w.part = M->part;
+    w.mr_nt = M->mr_nt;
     w.mr_x = M->mr_x; w.mr_t = M->mr_t; w.mr_t2 = M->mr_t2; w.mr_part = M->mr_part;
     w.w_xs = M->wws.w_xs; w.w_ts = M->wws.w_ts; w.w_part = M->wws.w_part;
     w.w_xmax = M->wws.w_xmax; w.w_g = M->wws.w_g;
@@ -1640,20 +1742,156 @@ const std::vector<Stage>& mr_stages(hlrc_hmat M, int op) {
     return M->stages_nf[op].empty() || !M->nf_multi ? M->stages[op] : M->stages_nf[op];
 }
 
-// Can the product for `op` run in blocks of MR_RB right-hand sides?  Needs
-// the multi-RHS workspace and no unit T-form stage (the uniform-H adjoint
-// coupling runs per vector).
-bool multi_rhs_ok(hlrc_hmat M, const Workspace& ws, int op, int nrhs) {
-    if (nrhs < 2 || nrhs < M->mr_min_nrhs || !ws.mr_x) return false;
-    for (const Stage& st : mr_stages(M, op))
-        if (st.kind == 0) return false;
-    return true;
+// Can the product run in blocks of MR_RB or more right-hand sides?  Needs
+// the multi-RHS workspace.
+bool multi_rhs_ok(hlrc_hmat M, const Workspace& ws, int nrhs) {
+    return nrhs >= 2 && nrhs >= M->mr_min_nrhs && ws.mr_x;
 }
 
-// y := y + alpha op(M) X for nrhs column vectors, MR_RB at a time: the matrix
-// is streamed once per block instead of once per vector.
+// One pass of an FP64 matrix over the vectors [r0, r0 + nr), nr <= 8 NT:
+// one tile of vectors on the kernels of kernels_mr.cuh, more on those of
+// kernels_dw.cuh.
+template <int NT>
+hlrc_status run_dw(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, const double* X, int64_t ldx, double* Y,
+                   int64_t ldy, int r0, int nr, cudaStream_t s0) {
+    constexpr int RB = MR_RB * NT, NG = (NT + 1) / 2;
+    const int64_t nx = op == HLRC_OP_N ? M->ncols : M->nrows;
+    // side stages read the block of x staged below and add into Y; the
+    // next block overwrites it only after the join
+    SideFork side{M, ws, s0};
+    const bool ov = M->overlap != 0;
+    cudaError_t le = cudaSuccess;   // the first failed launch
+    auto L = [&](cudaError_t e) { if (le == cudaSuccess) le = e; };
+    {
+        const cudaStream_t s = s0;
+        if (nx > 0) L(launch_k(ov, k_dw_rows<NT>, unsigned((nx + 31) / 32), 256, 0, s, X, ldx, nx, r0, nr, ws.mr_x));
+        M->launches += nx > 0;
+        HLRC_AFTER_LAUNCH("rows_from_cols");
+    }
+    int nl = 0;   // kernels launched below, counted at their launch sites
+    auto vec = [&](int name) -> double* { return name == V_X ? ws.mr_x : (name == V_T ? ws.mr_t : ws.mr_t2); };
+    auto omap = [&](int name) -> OutMap {
+        if (name == V_Y) return OutMap{Y + int64_t(r0) * ldy, 1, ldy, nr};
+        return OutMap{vec(name), RB, 1, RB};
+    };
+    const double* A = reinterpret_cast<const double*>(M->store);
+    const std::vector<Stage>& stl = mr_stages(M, op);
+    thread_local std::vector<int> order;
+    for (const int oi : stage_order(M, stl, order)) {
+        const Stage& st = stl[size_t(oi)];
+        const cudaStream_t s = side.before(st);
+        if (st.kind == 0) {
+            const DevTPass& tp = M->t[size_t(st.idx)];
+            const int add = tp.mode != OUT_SET;
+            const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
+            const OutMap om = omap(tp.out);
+            const int nu = tp.cls_begin[3];
+            if (ws.profile) prof_begin(M, stage_name(M, 0, st.idx), tp.alg_bytes, s);
+            if (nu > 0) {
+                L(launch_k(ov, k_tform_dw<NT>, unsigned((nu * NG + 7) / 8), 256, 0, s, tp.units, nu, tp.slabs, A,
+                           vec(tp.in), om, ws.mr_part, alpha, add));
+                ++nl;
+            }
+            if (tp.ngroups > 0) {
+                const int64_t th = int64_t(tp.ngroups) * TCOLS * RB;
+                L(launch_k(ov, k_tfinish_dw<NT>, unsigned((th + 255) / 256), 256, 0, s, tp.groups, tp.ngroups,
+                           ws.mr_part, om, alpha, add));
+                ++nl;
+            }
+            if (ws.profile) prof_end(M, s);
+            HLRC_AFTER_LAUNCH(stage_name(M, 0, st.idx));
+        } else if (st.kind == 2) {
+            const DevTTPass& tp = M->tt[size_t(st.idx)];
+            const int add = tp.mode != OUT_SET;
+            const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;
+            const OutMap om = omap(tp.out);
+            if (ws.profile) prof_begin(M, stage_name(M, 2, st.idx), tp.alg_bytes, s);
+            if constexpr (NT == 1) {
+                if (tp.nsegs[FMT_F64] > 0)
+                    L(launch_k(ov, k_ttform_dmma<DMMA_WARPS>, unsigned(tp.nsegs[FMT_F64]), DMMA_WARPS * 32, 0, s,
+                               tp.segs[FMT_F64], static_cast<const TTChunk*>(tp.chunks), A, vec(tp.in), om, ws.mr_part,
+                               alpha, add));
+                nl += tp.nsegs[FMT_F64] > 0;
+            } else {
+                // launched plainly: with programmatic dependent launch its waiting
+                // CTAs cost the 16-vector adjoint product of an n = 50021 matrix
+                // 50 us of 875
+                if (tp.ngsegs > 0)
+                    L(launch_k(false, k_gtform_dw<NT>, unsigned(tp.ngsegs), DW_GWARPS * 32, dw_gsmem<NT>(), s, tp.gsegs,
+                               tp.gchunks, tp.gtiles, A, vec(tp.in), om, ws.mr_part, alpha, add));
+                nl += tp.ngsegs > 0;
+            }
+            if (ws.profile) prof_end(M, s);
+            const TGroup *gr = NT == 1 ? tp.groups : tp.ggroups, *gr1 = NT == 1 ? tp.groups1 : tp.ggroups1;
+            const int ng = NT == 1 ? tp.ngroups : tp.nggroups, ng1 = NT == 1 ? tp.ngroups1 : tp.nggroups1;
+            if (ng > 0) {
+                if (ws.profile) prof_begin(M, "ttfinish", (NT == 1 ? tp.npart : tp.gnpart) * RB * 8, s);
+                // first level: runs of slots into the scratch part of the partials
+                const OutMap pm{ws.mr_part, RB, 1, RB};
+                const int b1 = fin_gpb(ng1), b2 = fin_gpb(ng);
+                if (ng1 > 0)
+                    L(launch_k(ov, k_ttfinish_flat<RB, double, false>, unsigned((ng1 + b1 - 1) / b1), 256, 0, s, gr1, ng1,
+                               b1, ws.mr_part, pm, static_cast<double*>(nullptr), 1.0, 0));
+                L(launch_k(ov, k_ttfinish_flat<RB, double, false>, unsigned((ng + b2 - 1) / b2), 256, 0, s, gr, ng, b2,
+                           ws.mr_part, om, static_cast<double*>(nullptr), alpha, add));
+                nl += 1 + (ng1 > 0 ? 1 : 0);
+                if (ws.profile) prof_end(M, s);
+            }
+            HLRC_AFTER_LAUNCH(stage_name(M, 2, st.idx));
+        } else {
+            const DevNPass& np = M->n[size_t(st.idx)];
+            if (np.launches() == 0) continue;
+            if (np.ncta > 0) return fail(HLRC_ERR_INTERNAL, "tree sweep in a multi-vector product");
+            if (ws.profile) prof_begin(M, stage_name(M, 1, st.idx), np.alg_bytes, s);
+            const int add = np.mode != OUT_SET;
+            const double alpha = np.mode == OUT_ADD ? 1.0 : alpha_in;
+            const NChunk* ch = static_cast<const NChunk*>(np.chunks);
+            if constexpr (NT == 1)
+                L(launch_k(ov, k_nform_dmma<DMMA_WARPS>, unsigned(np.nsegs[FMT_F64]), DMMA_WARPS * 32, 0, s,
+                           np.segs[FMT_F64], ch, A, vec(np.vx), vec(np.vt), omap(np.out), alpha, add));
+            else
+                L(launch_k(ov, k_nform_dw<NT>, unsigned(np.nsegs[FMT_F64]), DW_WARPS * 32, dw_nsmem<NT>(), s,
+                           np.segs[FMT_F64], ch, A, vec(np.vx), vec(np.vt), omap(np.out), alpha, add));
+            ++nl;
+            if (ws.profile) prof_end(M, s);
+            HLRC_AFTER_LAUNCH(stage_name(M, 1, st.idx));
+        }
+    }
+    M->launches += nl;
+    L(side.end());
+    if (le != cudaSuccess) return fail(HLRC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(le));
+    return HLRC_OK;
+}
+
+// An FP64 product of nrhs vectors in the fewest passes of at most ws.mr_nt
+// 8-vector tiles, their tiles spread evenly (40 vectors: 24 + 16, not 32 + 8,
+// whose second pass would read the matrix for a quarter of the arithmetic).
+hlrc_status run_multi_f64(hlrc_hmat M, const Workspace& ws, double alpha, int op, const double* X, int64_t ldx,
+                          double* Y, int64_t ldy, int nrhs, cudaStream_t s) {
+    int tiles = (nrhs + MR_RB - 1) / MR_RB;
+    int passes = (tiles + ws.mr_nt - 1) / ws.mr_nt;
+    for (int r0 = 0; r0 < nrhs; --passes) {
+        const int nt = (tiles + passes - 1) / passes, nr = std::min(nt * MR_RB, nrhs - r0);
+        hlrc_status st;
+        if (nt == 1) st = run_dw<1>(M, ws, alpha, op, X, ldx, Y, ldy, r0, nr, s);
+        else if (nt == 2) st = run_dw<2>(M, ws, alpha, op, X, ldx, Y, ldy, r0, nr, s);
+        else if (nt == 3) st = run_dw<3>(M, ws, alpha, op, X, ldx, Y, ldy, r0, nr, s);
+        else st = run_dw<DW_MAXNT>(M, ws, alpha, op, X, ldx, Y, ldy, r0, nr, s);
+        if (st != HLRC_OK) return st;
+        tiles -= nt;
+        r0 += nr;
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(HLRC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+    return HLRC_OK;
+}
+
+// y := y + alpha op(M) X for nrhs column vectors, MR_RB at a time (FP64
+// stores: up to MR_RB * ws.mr_nt): the matrix is streamed once per block
+// instead of once per vector.
 hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, const double* X, int64_t ldx,
                       double* Y, int64_t ldy, int nrhs, cudaStream_t s0) {
+    if (M->precision == HLRC_PREC_F64) return run_multi_f64(M, ws, alpha_in, op, X, ldx, Y, ldy, nrhs, s0);
     const int64_t nx = op == HLRC_OP_N ? M->ncols : M->nrows;
     for (int r0 = 0; r0 < nrhs; r0 += MR_RB) {
         const cudaStream_t s = s0;
@@ -1673,7 +1911,6 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
             if (name == V_Y) return OutMap{Y + int64_t(r0) * ldy, 1, ldy, nr};
             return OutMap{vec(name), MR_RB, 1, MR_RB};
         };
-        const double* A = reinterpret_cast<const double*>(M->store);
         const std::vector<Stage>& stl = mr_stages(M, op);
         thread_local std::vector<int> order;
         for (const int oi : stage_order(M, stl, order)) {
@@ -1685,15 +1922,7 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
                 const OutMap om = omap(tp.out);
                 if (ws.profile) prof_begin(M, stage_name(M, 2, st.idx), tp.alg_bytes, s);
-                constexpr int TW = DMMA_WARPS;
-                if (M->precision == HLRC_PREC_F64) {
-                    if (tp.nsegs[FMT_F64] > 0) {
-                        k_ttform_dmma<TW><<<tp.nsegs[FMT_F64], TW * 32, 0, s>>>(
-                            tp.segs[FMT_F64], static_cast<const TTChunk*>(tp.chunks), A, vec(tp.in), om, ws.mr_part,
-                            alpha, add);
-                        ++nl;
-                    }
-                } else if (M->precision == HLRC_PREC_BFP) {
+                if (M->precision == HLRC_PREC_BFP) {
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     if (tp.nmseg[FMT_I24] > 0) {
                         k_ttform_bfp<true><<<tp.nmseg[FMT_I24], TC_WARPS * 32, bq_smem_t(true), s>>>(
@@ -1722,27 +1951,18 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 }
                 if (ws.profile) prof_end(M, s);
                 if (tp.ngroups > 0) {
-                    if (ws.profile)
-                        prof_begin(M, "ttfinish", tp.npart * MR_RB * (M->precision == HLRC_PREC_F64 ? 8 : 4), s);
+                    if (ws.profile) prof_begin(M, "ttfinish", tp.npart * MR_RB * 4, s);
                     // first level: runs of slots into the scratch part of the partials
                     const OutMap pm{ws.mr_part, MR_RB, 1, MR_RB};
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     const int b1 = fin_gpb(tp.ngroups1), b2 = fin_gpb(tp.ngroups);
                     const unsigned fg1 = unsigned((tp.ngroups1 + b1 - 1) / b1);
                     const unsigned fg = unsigned((tp.ngroups + b2 - 1) / b2);
-                    if (M->precision == HLRC_PREC_F64) {
-                        if (tp.ngroups1 > 0)
-                            k_ttfinish_flat<MR_RB, double, false><<<fg1, 256, 0, s>>>(
-                                tp.groups1, tp.ngroups1, b1, ws.mr_part, pm, static_cast<double*>(nullptr), 1.0, 0);
-                        k_ttfinish_flat<MR_RB, double, false><<<fg, 256, 0, s>>>(
-                            tp.groups, tp.ngroups, b2, ws.mr_part, om, static_cast<double*>(nullptr), alpha, add);
-                    } else {
-                        if (tp.ngroups1 > 0)
-                            k_ttfinish_flat<MR_RB, float, true><<<fg1, 256, 0, s>>>(tp.groups1, tp.ngroups1, b1, fpart,
-                                                                                    pm, fpart, 1.0, 0);
-                        k_ttfinish_flat<MR_RB, float, false><<<fg, 256, 0, s>>>(
-                            tp.groups, tp.ngroups, b2, fpart, om, static_cast<float*>(nullptr), alpha, add);
-                    }
+                    if (tp.ngroups1 > 0)
+                        k_ttfinish_flat<MR_RB, float, true><<<fg1, 256, 0, s>>>(tp.groups1, tp.ngroups1, b1, fpart, pm,
+                                                                                fpart, 1.0, 0);
+                    k_ttfinish_flat<MR_RB, float, false><<<fg, 256, 0, s>>>(tp.groups, tp.ngroups, b2, fpart, om,
+                                                                            static_cast<float*>(nullptr), alpha, add);
                     nl += 1 + (tp.ngroups1 > 0 ? 1 : 0);
                     if (ws.profile) prof_end(M, s);
                 }
@@ -1755,39 +1975,31 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 const int add = np.mode != OUT_SET;
                 const double alpha = np.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
                 const OutMap om = omap(np.out);
-                constexpr int NW = DMMA_WARPS;
-                const bool f64plan = M->precision == HLRC_PREC_F64;
                 // the formats of one output tile run as separate grids, each
                 // adding its share to the output in a fixed launch order
-                if (f64plan && np.nsegs[FMT_F64] > 0) {
-                    k_nform_dmma<NW><<<np.nsegs[FMT_F64], NW * 32, 0, s>>>(
-                        np.segs[FMT_F64], static_cast<const NChunk*>(np.chunks), A, vec(np.vx), vec(np.vt), om, alpha,
-                        add);
-                    ++nl;
-                }
-                if (!f64plan && np.nmseg[FMT_F32] > 0) {
+                if (np.nmseg[FMT_F32] > 0) {
                     k_nform_d32<<<np.nmseg[FMT_F32], TC_WARPS * 32, tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32), s>>>(
                         np.mseg[FMT_F32], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
                     ++nl;
                 }
-                if (!f64plan && np.nmseg[FMT_F16] > 0) {
+                if (np.nmseg[FMT_F16] > 0) {
                     k_nform_tc<FMT_F16><<<np.nmseg[FMT_F16], TC_WARPS * 32,
                                           tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s>>>(
                         np.mseg[FMT_F16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
                     ++nl;
                 }
-                if (!f64plan && np.nmseg[FMT_BF16] > 0) {
+                if (np.nmseg[FMT_BF16] > 0) {
                     k_nform_tc<FMT_BF16><<<np.nmseg[FMT_BF16], TC_WARPS * 32,
                                            tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s>>>(
                         np.mseg[FMT_BF16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
                     ++nl;
                 }
-                if (!f64plan && np.nmseg[FMT_I24] > 0) {
+                if (np.nmseg[FMT_I24] > 0) {
                     k_nform_bfp<true><<<np.nmseg[FMT_I24], TC_WARPS * 32, bq_smem_n(true), s>>>(
                         np.mseg[FMT_I24], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
                     ++nl;
                 }
-                if (!f64plan && np.nmseg[FMT_I16] > 0) {
+                if (np.nmseg[FMT_I16] > 0) {
                     k_nform_bfp<false><<<np.nmseg[FMT_I16], TC_WARPS * 32, bq_smem_n(false), s>>>(
                         np.mseg[FMT_I16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
                     ++nl;
@@ -2061,7 +2273,7 @@ extern "C" hlrc_status hlrc_mvm(hlrc_hmat M, double alpha, int op, const double*
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Workspace ws = handle_workspace(M);
     if (wide_ok(M, ws, op, nrhs)) return run_wide(M, ws, alpha, x, ldx, y, ldy, nrhs, s);
-    if (multi_rhs_ok(M, ws, op, nrhs)) return run_multi(M, ws, alpha, op, x, ldx, y, ldy, nrhs, s);
+    if (multi_rhs_ok(M, ws, nrhs)) return run_multi(M, ws, alpha, op, x, ldx, y, ldy, nrhs, s);
     for (int r = 0; r < nrhs; ++r) {
         st = run_single(M, ws, alpha, op, x + size_t(r) * size_t(ldx), y + size_t(r) * size_t(ldy), s);
         if (st != HLRC_OK) return st;
@@ -2101,7 +2313,7 @@ extern "C" hlrc_status hlrc_mvm_host(hlrc_hmat M, double alpha, int op, const do
     if (wide_ok(M, ws, op, nrhs)) {
         st = run_wide(M, ws, alpha, M->hx, nx, M->hy, ny, nrhs, nullptr);
         if (st != HLRC_OK) return st;
-    } else if (multi_rhs_ok(M, ws, op, nrhs)) {
+    } else if (multi_rhs_ok(M, ws, nrhs)) {
         st = run_multi(M, ws, alpha, op, M->hx, nx, M->hy, ny, nrhs, nullptr);
         if (st != HLRC_OK) return st;
     } else {
@@ -2289,6 +2501,7 @@ struct hlrc_workspace_s {
     int device = 0;
     int64_t n_t = 0, n_t2 = 0, n_part = 0;   // one-vector capacities (doubles)
     size_t mr_nx = 0, mr_nt = 0, mr_nt2 = 0, mr_np = 0;   // multi-vector capacities (0: none)
+    int mr_tiles = 0;                                     // and the 8-vector tiles they were made for
     size_t w_xs = 0, w_ts = 0, w_part = 0;                // 64-vector capacities in bytes (0: none)
     char* arena = nullptr;
     size_t bytes = 0;
@@ -2310,13 +2523,6 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     size_t off = 0;
     auto take = [&](size_t elems) { const size_t o_ = off; off = align_up(off + elems * sizeof(double), 256); return o_; };
     const size_t o_t = take(size_t(W->n_t)), o_t2 = take(size_t(W->n_t2)), o_p = take(size_t(W->n_part));
-    MrSizes z;
-    size_t o_mr = 0;
-    if (max_nrhs > 1 && has_multi_kernels(M)) {
-        z = mr_sizes(M);
-        o_mr = take(z.bytes / sizeof(double) + 1);
-        W->mr_nx = z.nx; W->mr_nt = z.nt; W->mr_nt2 = z.nt2; W->mr_np = z.np;
-    }
     WideSizes zw;
     size_t o_w = 0;
     if (max_nrhs > MR_RB && M->wide) {
@@ -2326,8 +2532,24 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
         o_w = take(zw.bytes / sizeof(double) + 1);
         W->w_xs = zw.xs; W->w_ts = zw.ts; W->w_part = zw.part;
     }
-    W->bytes = off;
-    const cudaError_t e = cudaMalloc(&W->arena, W->bytes);
+    // the multi-vector arrays come last: narrower blocks where the widest do
+    // not fit (the same product in more passes)
+    MrSizes z;
+    const size_t o_mr = off;
+    cudaError_t e = cudaSuccess;
+    for (int nt = max_nrhs > 1 && has_multi_kernels(M) ? mr_tiles(M, max_nrhs) : 0;; --nt) {
+        off = o_mr;
+        if (nt > 0) {
+            z = mr_sizes(M, nt);
+            take(z.bytes / sizeof(double) + 1);
+            W->mr_nx = z.nx; W->mr_nt = z.nt; W->mr_nt2 = z.nt2; W->mr_np = z.np;
+            W->mr_tiles = W->ws.mr_nt = nt;
+        }
+        W->bytes = off;
+        e = cudaMalloc(&W->arena, W->bytes);
+        if (e != cudaErrorMemoryAllocation || nt <= 1) break;
+        cudaGetLastError();
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(HLRC_ERR_OOM, "hlrc_workspace_create: cudaMalloc of %zu bytes failed: %s", W->bytes,
@@ -2377,17 +2599,21 @@ extern "C" hlrc_status hlrc_mvm_ws(hlrc_hmat M, hlrc_workspace W, double alpha, 
     if (!g.ok) return fail(HLRC_ERR_CUDA, "cannot select device %d", M->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Workspace ws = W->ws;
-    if (ws.mr_x) {   // the multi-vector arrays serve only handles they fit
-        const MrSizes z = mr_sizes(M);
-        if (!has_multi_kernels(M) || z.nx > W->mr_nx || z.nt > W->mr_nt || z.nt2 > W->mr_nt2 || z.np > W->mr_np)
-            ws.mr_x = nullptr;
+    if (ws.mr_x) {   // the multi-vector arrays serve only handles they fit, in blocks that fit
+        ws.mr_nt = std::min(W->mr_tiles, mr_tiles(M, DW_MAXNT * MR_RB));
+        auto fits = [&](int nt) {
+            const MrSizes z = mr_sizes(M, nt);
+            return z.nx <= W->mr_nx && z.nt <= W->mr_nt && z.nt2 <= W->mr_nt2 && z.np <= W->mr_np;
+        };
+        while (ws.mr_nt > 0 && !fits(ws.mr_nt)) --ws.mr_nt;
+        if (!has_multi_kernels(M) || ws.mr_nt < 1) ws.mr_x = nullptr;
     }
     if (ws.w_xs) {
         const WideSizes z = wide_sizes(M);
         if (!M->wide || z.xs > W->w_xs || z.ts > W->w_ts || z.part > W->w_part) ws.w_xs = nullptr;
     }
     if (wide_ok(M, ws, op, nrhs)) return run_wide(M, ws, alpha, x, ldx, y, ldy, nrhs, s);
-    if (multi_rhs_ok(M, ws, op, nrhs)) return run_multi(M, ws, alpha, op, x, ldx, y, ldy, nrhs, s);
+    if (multi_rhs_ok(M, ws, nrhs)) return run_multi(M, ws, alpha, op, x, ldx, y, ldy, nrhs, s);
     for (int r = 0; r < nrhs; ++r) {
         st = run_single(M, ws, alpha, op, x + size_t(r) * size_t(ldx), y + size_t(r) * size_t(ldy), s);
         if (st != HLRC_OK) return st;

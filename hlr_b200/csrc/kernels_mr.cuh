@@ -166,6 +166,7 @@ __global__ void __launch_bounds__(W * 32, 2)
 k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
              const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
     __shared__ double red[W][TILE][MR_RB];
+    pdl_trigger();
     const NSeg sg = segs[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -200,6 +201,7 @@ k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, c
             }
     };
     uint32_t c = sg.cb + warp;
+    pdl_wait();
     if (c < sg.ce) {
         const NChunk none{0, 0, 0, 0};
         double2 mA[2][4], mB[2][4];
@@ -245,9 +247,11 @@ template <int W>
 __global__ void __launch_bounds__(W * 32, 2)
 k_ttform_dmma(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks, const double* __restrict__ A,
               const double* __restrict__ vin, OutMap om, double* __restrict__ part, double alpha, int add) {
+    pdl_trigger();
     const TTSeg sg = segs[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
+    pdl_wait();
     // x of the lane: rows 8j + 2t + b (j < 8, b < 2), right-hand side g
     double xv[16];
 #pragma unroll

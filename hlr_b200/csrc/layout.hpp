@@ -101,6 +101,34 @@ struct TTSeg {
 };
 static_assert(sizeof(TTSeg) == 16, "TTSeg must be 16 bytes");
 
+// Group T-form of FP64 products of more than 8 vectors: one CTA per group of
+// GT_TILES consecutive input tiles (or a piece of its chunks).  A chunk is
+// <= TCOLS columns of one object over all the group's tiles: clusters inside
+// one group need no partials, longer ones one partial per group instead of
+// one per tile.
+constexpr int GT_TILES = 4;
+constexpr uint32_t GT_NONE = 0xffffffffu;   // the object has no slab in this tile
+struct GTTile {
+    uint32_t v_off;        // first row of the tile in the input vector
+    uint16_t rows;
+    uint16_t ld;           // leading dimension of all slabs of the tile
+};
+static_assert(sizeof(GTTile) == 8, "GTTile must be 8 bytes");
+struct GTChunk {
+    uint32_t a[GT_TILES];  // (element offset - the segment's base) / 2 of the chunk's first column, per tile
+    uint32_t out;          // TT_DIRECT: output offset; else offset in the partial array
+    uint16_t nc;           // columns (<= TCOLS)
+    uint16_t flags;
+};
+static_assert(sizeof(GTChunk) == 24, "GTChunk must be 24 bytes");
+struct GTSeg {
+    uint64_t base;         // element offset the chunks' offsets are relative to
+    uint32_t cb, ce;       // chunk range
+    uint32_t tile0;        // tiles [tile0, tile0 + ntiles) of the tile table
+    uint32_t ntiles;
+};
+static_assert(sizeof(GTSeg) == 24, "GTSeg must be 24 bytes");
+
 // ------------------------------------------------------ reduced precision
 // Storage formats of a chunk.  Scaled formats store value / scale; the
 // scale (one FP32 per chunk = per block, tile and <= 8 columns) is folded

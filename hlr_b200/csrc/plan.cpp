@@ -4,6 +4,7 @@
 #include "plan.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -478,6 +479,7 @@ struct PlanKnobs {
     // the near field on a side stream (every kind of plan: 0 H, 1 uniform-H,
     // 2 H^2), unless the caller asks for it fused
     bool side_dense(int /*kind*/) const { return near_field != 1; }
+    bool blocks = false;           // build the group T-forms (FP64, max_nrhs > 8)
 };
 thread_local PlanKnobs g_knobs;
 struct KnobScope {
@@ -486,6 +488,7 @@ struct KnobScope {
         g_knobs.finish_slots = o.finish_slots > 0 ? uint32_t(o.finish_slots) : FINISH_SLOTS;
         g_knobs.piece_tiles = o.piece_tiles > 0 ? o.piece_tiles : WT_MAXT;
         g_knobs.near_field = o.near_field;
+        g_knobs.blocks = o.precision == HLRC_PREC_F64 && o.max_nrhs > 8;
     }
     ~KnobScope() { g_knobs = saved; }
 };
@@ -509,7 +512,15 @@ struct TTBuilder {
     std::vector<uint32_t> oout;
     uint32_t cb = 0, voff = 0;
     int64_t bytes = 0, rows = 0;
-    TTBuilder(TTPass& p, const Store& s, size_t nobj) : P(p), S(s), pbase(nobj, -2), ncol(nobj, 0), oout(nobj, 0) {}
+    // group T-form: per object its slots so far, the group of the last one
+    // and that slot's first chunk; per group chunk its object, column and slot
+    struct GObj { int64_t nslots = 0, group = -1; uint32_t first = 0; };
+    struct GRef { uint32_t id, j, slot, group; };
+    std::vector<GObj> gobj;
+    std::vector<GRef> gref;
+    std::vector<std::array<uint64_t, GT_TILES>> goff;   // element offsets (~0: none)
+    TTBuilder(TTPass& p, const Store& s, size_t nobj)
+        : P(p), S(s), pbase(nobj, -2), ncol(nobj, 0), oout(nobj, 0), gobj(g_knobs.blocks ? nobj : 0) {}
 
     void object(size_t id, uint32_t out, int64_t ncols, int64_t nslabs) {
         ncol[id] = ncols;
@@ -528,6 +539,92 @@ struct TTBuilder {
         voff = uint32_t(v_off);
         rows = tile_rows;
         bytes = 0;
+        if (g_knobs.blocks) P.gtiles.push_back(GTTile{voff, uint16_t(rows), uint16_t(pad_rows(rows))});
+    }
+    // slab `sid` (columns [lo, lo + ncol[id])) as one slot of object `id` in
+    // the current group of tiles
+    void group_slab(int sid, size_t id, int64_t lo) {
+        const SSlab& s = S.slabs[size_t(sid)];
+        const int64_t tile = int64_t(P.gtiles.size()) - 1, group = tile / GT_TILES;
+        const size_t at = size_t(tile % GT_TILES);
+        GObj& o = gobj[id];
+        // the slab's chunks of these columns follow one another
+        int32_t c0 = s.c0, c1 = s.c0 + s.nch;
+        while (c0 < c1 && S.chunks[size_t(c0)].col0 < lo) ++c0;
+        while (c1 > c0 && S.chunks[size_t(c1 - 1)].col0 >= lo + ncol[id]) --c1;
+        const SChunk* cols = S.chunks.data() + c0;
+        const size_t nc = size_t(c1 - c0);
+        // the slot of an earlier tile of the group takes the slab when it has
+        // the same chunks and none of this tile yet
+        bool same = o.group == group && o.first + nc <= gref.size();
+        for (size_t q = 0; same && q < nc; ++q) {
+            const GRef& r = gref[o.first + q];
+            same = r.id == id && r.j == uint32_t(cols[q].col0 - lo) && P.gchunks[o.first + q].nc == cols[q].nc &&
+                   goff[o.first + q][at] == ~uint64_t(0);
+        }
+        if (!same) {
+            o.group = group;
+            o.first = uint32_t(gref.size());
+            for (size_t q = 0; q < nc; ++q) {
+                gref.push_back(GRef{uint32_t(id), uint32_t(cols[q].col0 - lo), uint32_t(o.nslots), uint32_t(group)});
+                P.gchunks.push_back(GTChunk{{GT_NONE, GT_NONE, GT_NONE, GT_NONE}, 0, uint16_t(cols[q].nc), 0});
+                goff.push_back({~uint64_t(0), ~uint64_t(0), ~uint64_t(0), ~uint64_t(0)});
+            }
+            ++o.nslots;
+        }
+        for (size_t q = 0; q < nc; ++q) goff[o.first + q][at] = uint64_t(cols[q].byte_off) / sizeof(double);
+    }
+    // Outputs and partial slots of the group chunks, and the segments: a
+    // group's chunks in pieces of about equal bytes, so that some 148 x 8
+    // CTAs share the work whatever the number of tiles; a piece stages the
+    // x rows of its tiles again (32 KB a vector group of 16), hence not below
+    // 64 KB of matrix.
+    void group_finish() {
+        std::vector<int64_t> gbase(gobj.size(), -1);
+        for (size_t id = 0; id < gobj.size(); ++id) {
+            if (gobj[id].nslots <= 1) continue;
+            gbase[id] = P.gnpart;
+            P.ggroups.push_back({uint32_t(P.gnpart), uint32_t(gobj[id].nslots), oout[id], uint32_t(ncol[id])});
+            P.gnpart += gobj[id].nslots * ncol[id];
+        }
+        for (size_t c = 0; c < gref.size(); ++c) {
+            const GRef& r = gref[c];
+            GTChunk& g = P.gchunks[c];
+            if (gbase[r.id] < 0) { g.out = oout[r.id] + r.j; g.flags = TT_DIRECT; }
+            else g.out = uint32_t(gbase[r.id] + int64_t(r.slot) * ncol[r.id] + r.j);
+        }
+        int64_t total = 0;
+        std::vector<int32_t> by(gref.size(), 0);
+        for (size_t c = 0; c < gref.size(); ++c) {
+            for (size_t a = 0; a < GT_TILES; ++a)
+                if (goff[c][a] != ~uint64_t(0))
+                    by[c] += 8 * int32_t(P.gchunks[c].nc) * P.gtiles[size_t(gref[c].group) * GT_TILES + a].ld;
+            total += by[c];
+        }
+        const int64_t target = std::min<int64_t>(768 << 10, std::max<int64_t>(64 << 10, total / (148 * 8)));
+        std::vector<std::pair<int64_t, GTSeg>> segs;
+        for (size_t c = 0; c < gref.size();) {
+            size_t e = c;
+            int64_t b = 0;
+            uint64_t base = ~uint64_t(0);
+            for (; e < gref.size() && gref[e].group == gref[c].group && (e == c || b < target); ++e) {
+                b += by[e];
+                for (size_t a = 0; a < GT_TILES; ++a) base = std::min(base, goff[e][a]);
+            }
+            const size_t t0 = size_t(gref[c].group) * GT_TILES;
+            segs.push_back({b, GTSeg{base, uint32_t(c), uint32_t(e), uint32_t(t0),
+                                     uint32_t(std::min<size_t>(GT_TILES, P.gtiles.size() - t0))}});
+            for (size_t k = c; k < e; ++k)
+                for (size_t a = 0; a < GT_TILES; ++a) {
+                    const uint64_t o = goff[k][a];
+                    if (o == ~uint64_t(0)) continue;
+                    P.gchunks[k].a[a] = uint32_t(std::min<uint64_t>((o - base) / 2, GT_NONE));
+                }
+            c = e;
+        }
+        std::stable_sort(segs.begin(), segs.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+        for (const auto& e : segs) P.gsegs.push_back(e.second);
+        two_levels(P.ggroups, P.ggroups1, P.gnpart);
     }
     // columns [lo, lo + ncol[id]) of slab `sid` feed object `id` as its slab number `k`
     void slab(int sid, size_t id, int64_t k, int64_t lo = 0) {
@@ -544,6 +641,7 @@ struct TTBuilder {
             bytes += pad_fmt(s.rows, ch.fmt) * ch.nc * fmt_bytes(ch.fmt);
             P.alg_bytes += rows * ch.nc * fmt_bytes(ch.fmt);
         }
+        if (g_knobs.blocks) group_slab(sid, id, lo);
     }
     void end() {
         const uint32_t ce = uint32_t(P.chunks.size());
@@ -570,22 +668,26 @@ struct TTBuilder {
                 P.bytes += e.first;
             }
         }
-        // Outputs with more than FINISH_SLOTS tiles are summed in two levels,
-        // so that no warp adds more than FINISH_SLOTS slots in a row: the
-        // slots are cut into runs whose sums go to a scratch region appended
-        // to the partial array (layout [run][column], like the slots), and
-        // the output's group then sums the runs.  The order of all additions
-        // depends on the shapes only.
-        for (TGroup& g : P.groups) {
+        two_levels(P.groups, P.groups1, P.npart);
+        if (g_knobs.blocks) group_finish();
+    }
+    // Outputs with more than FINISH_SLOTS slots are summed in two levels,
+    // so that no warp adds more than FINISH_SLOTS slots in a row: the
+    // slots are cut into runs whose sums go to a scratch region appended
+    // to the partial array (layout [run][column], like the slots), and
+    // the output's group then sums the runs.  The order of all additions
+    // depends on the shapes only.
+    static void two_levels(std::vector<TGroup>& groups, std::vector<TGroup>& groups1, int64_t& npart) {
+        for (TGroup& g : groups) {
             const uint32_t FS = g_knobs.finish_slots;
             if (g.nslots <= FS) continue;
             const uint32_t nrun = (g.nslots + FS - 1) / FS;
-            const uint32_t scratch = uint32_t(P.npart);
+            const uint32_t scratch = uint32_t(npart);
             for (uint32_t r = 0; r < nrun; ++r) {
                 const uint32_t s0 = r * FS;
-                P.groups1.push_back({g.slot0 + s0 * g.nc, std::min(FS, g.nslots - s0), scratch + r * g.nc, g.nc});
+                groups1.push_back({g.slot0 + s0 * g.nc, std::min(FS, g.nslots - s0), scratch + r * g.nc, g.nc});
             }
-            P.npart += int64_t(nrun) * g.nc;
+            npart += int64_t(nrun) * g.nc;
             g.slot0 = scratch;
             g.nslots = nrun;
         }
@@ -803,6 +905,36 @@ hlrc_status validate_plan(const Plan& p) {
             if (int64_t(g.slot0) + int64_t(g.nslots) * g.nc > tp.npart || int64_t(g.out) + g.nc > tp.npart)
                 return fail(HLRC_ERR_INTERNAL, "T-pass %zu: first-level finish group outside the partials", pi);
     }
+    // group T-forms: offsets inside the store and on 16 bytes, tiles inside the
+    // input, outputs inside their arrays
+    for (size_t pi = 0; pi < p.ttpasses.size(); ++pi) {
+        const TTPass& tp = p.ttpasses[pi];
+        for (const GTTile& t : tp.gtiles)
+            if (t.rows > TILE || t.ld != pad_rows(t.rows) || int64_t(t.v_off) + t.rows > vec_len(tp.in))
+                return fail(HLRC_ERR_INTERNAL, "T-pass %zu: bad group tile", pi);
+        for (const GTSeg& s : tp.gsegs) {
+            if (s.ce < s.cb || s.ce > tp.gchunks.size() || s.ntiles < 1 || s.ntiles > GT_TILES ||
+                size_t(s.tile0) + s.ntiles > tp.gtiles.size() || s.base % 2 != 0)
+                return fail(HLRC_ERR_INTERNAL, "T-pass %zu: bad group segment", pi);
+            for (uint32_t c = s.cb; c < s.ce; ++c) {
+                const GTChunk& g = tp.gchunks[c];
+                const int64_t lim = (g.flags & TT_DIRECT) ? vec_len(tp.out) : tp.gnpart;
+                bool ok = g.nc >= 1 && g.nc <= TCOLS && int64_t(g.out) + g.nc <= lim, any = false;
+                for (uint32_t a = 0; a < GT_TILES && ok; ++a) {
+                    if (g.a[a] == GT_NONE) continue;
+                    any = true;
+                    ok = a < s.ntiles &&
+                         int64_t(8 * (s.base + 2 * uint64_t(g.a[a]))) + 8 * int64_t(g.nc) * tp.gtiles[s.tile0 + a].ld <= store;
+                }
+                if (!ok || !any) return fail(HLRC_ERR_INTERNAL, "T-pass %zu: bad group chunk %u", pi, c);
+            }
+        }
+        for (const std::vector<TGroup>* gs : {&tp.ggroups, &tp.ggroups1})
+            for (const TGroup& g : *gs)
+                if (int64_t(g.slot0) + int64_t(g.nslots) * g.nc > tp.gnpart ||
+                    int64_t(g.out) + g.nc > (gs == &tp.ggroups ? vec_len(tp.out) : tp.gnpart))
+                    return fail(HLRC_ERR_INTERNAL, "T-pass %zu: group finish outside its arrays", pi);
+    }
     // side stages lead their list and are plain N-form passes adding into y
     // from x and the store only: they run beside the stages after them
     for (int op = 0; op < 3; ++op) {
@@ -961,6 +1093,7 @@ hlrc_status plan_h(const hlrc_h_desc& d, const hlrc_options& o, Plan& p, double 
     if (valr && !(o.mixed_eps > 0))
         return fail(HLRC_ERR_ARG, "HLRC_PREC_MIXED / HLRC_PREC_BFP need mixed_eps > 0");
     p = Plan();
+    p.blocks = g_knobs.blocks;
     p.kind = 0;
     p.precision = o.precision;
     p.nrows = d.nrows;
@@ -1268,6 +1401,7 @@ hlrc_status plan_uniform(const hlrc_uniform_desc& d, const hlrc_options& o, Plan
     if (o.precision != HLRC_PREC_F64)
         return fail(HLRC_ERR_ARG, "precision %d not supported for uniform-H (FP64 only)", o.precision);
     p = Plan();
+    p.blocks = g_knobs.blocks;
     p.kind = 1;
     p.precision = o.precision;
     p.nrows = d.nrows;
@@ -1579,6 +1713,7 @@ hlrc_status plan_h2(const hlrc_h2_desc& d, const hlrc_options& o, Plan& p) {
     if (o.precision != HLRC_PREC_F64)
         return fail(HLRC_ERR_ARG, "precision %d not supported for H2 (FP64 only)", o.precision);
     p = Plan();
+    p.blocks = g_knobs.blocks;
     p.kind = 2;
     p.precision = o.precision;
     p.nrows = d.nrows;

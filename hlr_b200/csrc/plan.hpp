@@ -92,6 +92,13 @@ struct TTPass {
     int64_t npart = 0;             // partial array length (doubles), scratch region included
     int in = V_X, out = V_T, mode = OUT_SET;
     int64_t bytes = 0, alg_bytes = 0;
+    // group T-form (FP64 plans for more than 8 vectors): segments by cost
+    // (descending), the finish of objects in several groups, partials
+    std::vector<GTSeg> gsegs;
+    std::vector<GTChunk> gchunks;
+    std::vector<GTTile> gtiles;
+    std::vector<TGroup> ggroups, ggroups1;
+    int64_t gnpart = 0;
 };
 
 // The one-pass 64-vector product of a 16-bit H store (op N): the
@@ -160,6 +167,7 @@ struct Plan {
     // profile names per pass (static strings), per stage kind; empty = the
     // fixed names of kinds 0 and 1
     std::vector<const char*> names[3];
+    bool blocks = false;           // FP64 plan with the group T-forms of products of more than 8 vectors
     WidePlan wide;                 // 16-bit H stores: the 64-vector op N product
 };
 
