@@ -28,6 +28,7 @@
 #include "kernels_bfp8.cuh"
 #include "kernels_dw.cuh"
 #include "kernels_f64.cuh"
+#include "kernels_flow.cuh"
 #include "kernels_mr.cuh"
 #include "kernels_q.cuh"
 #include "kernels_tc.cuh"
@@ -123,6 +124,7 @@ struct Workspace {
     double* t = nullptr;
     double* t2 = nullptr;
     double* part = nullptr;
+    unsigned* ctr = nullptr;     // counters of one-launch products (FLOW_CTRS, zero between products)
     int mr_nt = 0;               // the multi-vector arrays hold blocks of 8 * mr_nt vectors
     double* mr_x = nullptr;      // null: no multi-vector arrays
     double* mr_t = nullptr;
@@ -206,6 +208,14 @@ struct hlrc_hmat_s {
     bool nf_multi = false;             // multi-vector products take stages_nf too
     Workspace side_ws;                 // the handle's side stream and events (side stages only)
     hlrc_info info{};
+    // one-vector products as one launch (kernels_flow.cuh), per op; nst 0:
+    // a launch per pass
+    struct Flow {
+        FlowStage st[FLOW_MAXST];
+        int nst = 0, side = -1, main_items = 0, side_items = 0;
+    };
+    Flow flow[3];
+    unsigned* ctr = nullptr;           // counters of the handle's own workspace
     // multi-RHS workspace (allocated at upload when max_nrhs > 1): row-major
     // blocks of MR_RB * mr_nt vectors
     char* mr_arena = nullptr;
@@ -333,7 +343,7 @@ struct ArenaLayout {
     std::vector<size_t> tu, ts, tg, nc, ttc, ttg, ttg1, n2;
     std::vector<std::array<size_t, 7>> ntree;   // per N-pass: the tree sweep's seven arrays
     std::vector<std::array<size_t, NFMT>> ns, tts;   // per pass, per StoreFmt
-    size_t t = 0, t2 = 0, part = 0, err = 0, total = 0;
+    size_t t = 0, t2 = 0, part = 0, ctr = 0, err = 0, total = 0;
     size_t part_elems = 0;
 };
 
@@ -379,6 +389,7 @@ ArenaLayout arena_layout(const Plan& p) {
     L.t = take(size_t(std::max<int64_t>(1, p.n_t)) * sizeof(double));
     L.t2 = take(size_t(std::max<int64_t>(1, p.n_t2)) * sizeof(double));
     L.part = take(part_elems * sizeof(double));
+    L.ctr = take(FLOW_CTRS * sizeof(unsigned));
     L.err = take(sizeof(int));
     L.part_elems = part_elems;
     L.total = off;
@@ -977,6 +988,81 @@ hlrc_status plan_h_leaves(const hlrc_h_desc& d, hlrc_options o, Plan& p, double 
     return plan_h(hd, o, p, area);
 }
 
+// The passes of one-launch products (kernels_flow.cuh): the one-vector stages
+// of each op, with the finishes as passes of their own.  Only products whose
+// passes have at most FLOW_TILES tiles run this way, and none with tree sweeps:
+// a hand-over between passes costs about 2 us on the device, as between
+// launches; what is saved are the host's calls (B200, one vector, eager
+// launches, separate -> one: 1D log n = 2048 20 -> 11 us, n = 8192 28 -> 14 us,
+// n = 16384 (256 tiles) 22 -> 19 us; exponential n = 13001 117 -> 113 us; but 512
+// tiles of a uniform-H matrix 55 -> 75 us, 2048 tiles 66 -> 124 us).
+constexpr int FLOW_TILES = 296;
+void plan_flow(hlrc_hmat_s* h) {
+    if (h->precision != HLRC_PREC_F64) return;
+    for (int op = 0; op < 3; ++op) {
+        const std::vector<Stage>& list = h->stages_nf[op].empty() ? h->stages[op] : h->stages_nf[op];
+        hlrc_hmat_s::Flow F;
+        bool ok = !list.empty();
+        int prev = -1;
+        bool joined = false;
+        auto push = [&](int kind, const void* items, const void* data, int n, bool side, int in, int vt, int out, int mode) {
+            if (n <= 0) return;
+            if (F.nst == FLOW_MAXST || (side && F.side >= 0)) ok = false;
+            if (!ok) return;
+            // a tile is an item; groups and units come one per warp, in rounds
+            // so that the pass has at most one item per resident CTA
+            const bool tiles = kind == FLOW_N || kind == FLOW_TT;
+            const int most = 8 * FLOW_CTAS * h->sms;
+            ok = !tiles || n <= FLOW_TILES;
+            FlowStage& f = F.st[F.nst];
+            f = FlowStage{};
+            f.items = items;
+            f.data = data;
+            f.kind = kind;
+            f.n = n;
+            f.per = tiles ? 1 : 8 * std::max(1, (n + most - 1) / most);
+            f.nitems = (n + f.per - 1) / f.per;
+            f.dep = side ? -1 : prev;
+            f.join = -1;
+            f.in = int8_t(in);
+            f.vt = int8_t(vt);
+            f.out = int8_t(out);
+            f.add = int8_t(mode == OUT_SET ? 0 : (mode == OUT_ADD ? 2 : 1));
+            int& items_of = side ? F.side_items : F.main_items;
+            f.first = items_of;
+            items_of += f.nitems;
+            if (side) {
+                F.side = F.nst;
+            } else {
+                if (out == V_Y && F.side >= 0 && !joined) {
+                    f.join = F.side;
+                    joined = true;
+                }
+                prev = F.nst;
+            }
+            ++F.nst;
+        };
+        for (const Stage& st : list) {
+            if (st.kind == 1) {
+                const DevNPass& np = h->n[size_t(st.idx)];
+                ok = ok && np.ncta == 0;
+                push(FLOW_N, np.segs[FMT_F64], np.chunks, np.nsegs[FMT_F64], st.side, np.vx, np.vt, np.out, np.mode);
+            } else if (st.kind == 2) {
+                const DevTTPass& tp = h->tt[size_t(st.idx)];
+                push(FLOW_TT, tp.segs[FMT_F64], tp.chunks, tp.nsegs[FMT_F64], st.side, tp.in, tp.in, tp.out, tp.mode);
+                push(FLOW_FINISH, tp.groups1, nullptr, tp.ngroups1, st.side, tp.in, tp.in, 4, OUT_SET);
+                push(FLOW_FINISH, tp.groups, nullptr, tp.ngroups, st.side, tp.in, tp.in, tp.out, tp.mode);
+            } else {
+                const DevTPass& tp = h->t[size_t(st.idx)];
+                ok = ok && tp.cls_begin[1] == tp.cls_begin[3];   // 8-column units only
+                push(FLOW_T, tp.units, tp.slabs, tp.cls_begin[3], st.side, tp.in, tp.in, tp.out, tp.mode);
+                push(FLOW_TFINISH, tp.groups, nullptr, tp.ngroups, st.side, tp.in, tp.in, tp.out, tp.mode);
+            }
+        }
+        if (ok && F.nst > 0) h->flow[op] = F;
+    }
+}
+
 // The group T-form tables of an FP64 plan, in an allocation of their own.
 hlrc_status upload_groups(const Plan& p, hlrc_hmat_s* h) {
     size_t bytes = 0;
@@ -1049,6 +1135,8 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (st != HLRC_OK) return st;
     }
     h->device = dev;
+    cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, dev);
+    if (h->sms <= 0) h->sms = 148;
     h->kind = p.kind;
     for (int k = 0; k < 3; ++k) h->names[k] = p.names[k];
     h->precision = p.precision;
@@ -1223,6 +1311,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         hp->tt.push_back(d);
     }
     if (e == cudaSuccess) e = cudaMemset(hp->arena + L.err, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(hp->arena + L.ctr, 0, FLOW_CTRS * sizeof(unsigned));
     if (e != cudaSuccess) {
         cleanup();
         return fail(HLRC_ERR_CUDA, "upload copy failed: %s", cudaGetErrorString(e));
@@ -1240,6 +1329,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
     hp->ws_t2 = reinterpret_cast<double*>(hp->arena + o_t2);
     hp->part = reinterpret_cast<double*>(hp->arena + o_part);
     hp->dev_err = reinterpret_cast<int*>(hp->arena + L.err);
+    hp->ctr = reinterpret_cast<unsigned*>(hp->arena + L.ctr);
     for (int op = 0; op < 3; ++op) {
         hp->stages[op] = p.stages[op];
         hp->stages_mr[op] = p.stages_mr[op];
@@ -1254,6 +1344,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
     }
 
     fill_info(p, L, hp->info);
+    plan_flow(hp);
     if (p.blocks) {
         hlrc_status st = enable_dw_smem(dev);
         if (st == HLRC_OK) st = upload_groups(p, hp);
@@ -1370,8 +1461,6 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         hp->info.device_bytes += int64_t(wb);
     }
     // the store as rows of 128 bytes for the full-tile TMA kernels
-    cudaDeviceGetAttribute(&hp->sms, cudaDevAttrMultiProcessorCount, dev);
-    if (hp->sms <= 0) hp->sms = 148;
     if (!p.wide.empty()) {
         const uint64_t rows = uint64_t(p.store_size()) / 128;
         hp->tma = rows > 0 && make_map(&hp->tm_s16, hp->store, 64, rows, 128, 64, 16) &&
@@ -1416,6 +1505,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
 Workspace handle_workspace(hlrc_hmat M) {
     Workspace w;
     w.t = M->ws_t; w.t2 = M->ws_t2; w.part = M->part;
+    w.ctr = M->ctr;
     w.mr_nt = M->mr_nt;
     w.mr_x = M->mr_x; w.mr_t = M->mr_t; w.mr_t2 = M->mr_t2; w.mr_part = M->mr_part;
     w.w_xs = M->wws.w_xs; w.w_ts = M->wws.w_ts; w.w_part = M->wws.w_part;
@@ -1593,8 +1683,46 @@ const std::vector<int>& stage_order(hlrc_hmat M, const std::vector<Stage>& stl, 
     return order;
 }
 
+// Does the product run as one launch?  Not under capture (n = 8192: a replay of
+// the separate launches takes 9.3 us, one launch 13.3 us, and the host's calls
+// are paid once), not with per-pass profiling or debugging, nor with launch
+// shapes other than the default (its CTAs have 8 warps, which gives the sums
+// of the default shapes).
+bool flow_ok(hlrc_hmat M, const Workspace& ws, int op, cudaStream_t s) {
+    return M->flow[op].nst > 0 && ws.ctr && !ws.profile && M->nform_warps == 8 && M->ttform_warps == 8 &&
+           !debug_sync() && !capturing(s);
+}
+hlrc_status run_flow(hlrc_hmat M, const Workspace& ws, double alpha, int op, const double* x, double* y,
+                     cudaStream_t s) {
+    const hlrc_hmat_s::Flow& F = M->flow[op];
+    FlowArgs a{};
+    std::copy(F.st, F.st + F.nst, a.st);
+    a.nst = F.nst;
+    a.side = F.side;
+    a.main_items = F.main_items;
+    a.side_items = F.side_items;
+    a.A = reinterpret_cast<const double*>(M->store);
+    a.v[V_X] = const_cast<double*>(x);
+    a.v[V_Y] = y;
+    a.v[V_T] = ws.t;
+    a.v[V_T2] = ws.t2;
+    a.v[4] = ws.part;
+    a.alpha = alpha;
+    a.ctr = ws.ctr;
+    a.err = M->dev_err;
+    a.wait_ns = M->wait_ns;
+    a.skip = M->wait_skip;
+    const int grid = std::min(FLOW_CTAS * M->sms, F.main_items + F.side_items);
+    a.main_ctas = grid - (F.side >= 0 ? std::min(F.side_items, grid / 2) : 0);
+    M->launches += 1;
+    const cudaError_t e = launch_k(M->overlap != 0, k_flow_f64, unsigned(grid), 256, 0, s, a);
+    if (e != cudaSuccess) return fail(HLRC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+    return HLRC_OK;
+}
+
 hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, const double* x, double* y,
                        cudaStream_t s0) {
+    if (flow_ok(M, ws, op, s0)) return run_flow(M, ws, alpha_in, op, x, y, s0);
     // FP64 plans carry 16-byte FP64 descriptors, reduced-precision plans
     // 32-byte packs: each kind of kernel only ever sees its own kind
     const bool f64plan = M->precision == HLRC_PREC_F64;
@@ -2435,26 +2563,31 @@ extern "C" hlrc_status hlrc_check_device_error(hlrc_hmat M, int* code) {
 // per device with cudaGetSymbolAddress while that device is current.
 constexpr size_t NOALLOC_SCRATCH_DOUBLES = size_t(1) << 20;  // 8 MiB
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_SCRATCH_DOUBLES];
+static __device__ __align__(256) unsigned g_noalloc_ctr[FLOW_CTRS];   // one-launch products: zero between calls
 
 namespace {
 constexpr int NOALLOC_MAX_DEVICES = 128;
 std::mutex g_noalloc_mu;
 double* g_noalloc_ptr[NOALLOC_MAX_DEVICES] = {};
+unsigned* g_noalloc_ctr_ptr[NOALLOC_MAX_DEVICES] = {};
 
 // device address of the scratch on `dev` (which must be current)
-hlrc_status noalloc_scratch(int dev, double** out) {
+hlrc_status noalloc_scratch(int dev, double** out, unsigned** ctr) {
     if (dev < 0 || dev >= NOALLOC_MAX_DEVICES)
         return fail(HLRC_ERR_ARG, "hlrc_mvm_noalloc: device ordinal %d outside 0..%d", dev, NOALLOC_MAX_DEVICES - 1);
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
     if (!g_noalloc_ptr[dev]) {
-        void* p = nullptr;
-        const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+        void *p = nullptr, *c = nullptr;
+        cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+        if (e == cudaSuccess) e = cudaGetSymbolAddress(&c, g_noalloc_ctr);
         if (e != cudaSuccess)
             return fail(HLRC_ERR_CUDA, "hlrc_mvm_noalloc: cudaGetSymbolAddress on device %d failed: %s", dev,
                         cudaGetErrorString(e));
         g_noalloc_ptr[dev] = static_cast<double*>(p);
+        g_noalloc_ctr_ptr[dev] = static_cast<unsigned*>(c);
     }
     *out = g_noalloc_ptr[dev];
+    *ctr = g_noalloc_ctr_ptr[dev];
     return HLRC_OK;
 }
 }  // namespace
@@ -2475,7 +2608,8 @@ extern "C" hlrc_status hlrc_mvm_noalloc(hlrc_hmat M, double alpha, int op, const
     DeviceGuard g(M->device);
     if (!g.ok) return fail(HLRC_ERR_CUDA, "cannot select device %d", M->device);
     double* base = nullptr;
-    st = noalloc_scratch(M->device, &base);
+    unsigned* ctr = nullptr;
+    st = noalloc_scratch(M->device, &base, &ctr);
     if (st != HLRC_OK) return st;
     // every scratch entry a product reads is written earlier in the same
     // product (coefficients with OUT_SET, each partial by its chunk), so the
@@ -2484,6 +2618,7 @@ extern "C" hlrc_status hlrc_mvm_noalloc(hlrc_hmat M, double alpha, int op, const
     ws.t = base;
     ws.t2 = base + std::max<int64_t>(1, M->n_t);
     ws.part = base + std::max<int64_t>(1, M->n_t) + std::max<int64_t>(1, M->n_t2);
+    ws.ctr = ctr;
     return run_single(M, ws, alpha, op, x, y, static_cast<cudaStream_t>(stream));
 }
 
@@ -2522,7 +2657,8 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     W->n_part = std::max<int64_t>(1, M->n_part);
     size_t off = 0;
     auto take = [&](size_t elems) { const size_t o_ = off; off = align_up(off + elems * sizeof(double), 256); return o_; };
-    const size_t o_t = take(size_t(W->n_t)), o_t2 = take(size_t(W->n_t2)), o_p = take(size_t(W->n_part));
+    const size_t o_t = take(size_t(W->n_t)), o_t2 = take(size_t(W->n_t2)), o_p = take(size_t(W->n_part)),
+                 o_ctr = take(FLOW_CTRS * sizeof(unsigned) / sizeof(double) + 1);
     WideSizes zw;
     size_t o_w = 0;
     if (max_nrhs > MR_RB && M->wide) {
@@ -2558,6 +2694,11 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     W->ws.t = reinterpret_cast<double*>(W->arena + o_t);
     W->ws.t2 = reinterpret_cast<double*>(W->arena + o_t2);
     W->ws.part = reinterpret_cast<double*>(W->arena + o_p);
+    W->ws.ctr = reinterpret_cast<unsigned*>(W->arena + o_ctr);
+    if (const cudaError_t me = cudaMemset(W->ws.ctr, 0, FLOW_CTRS * sizeof(unsigned)); me != cudaSuccess) {
+        cudaFree(W->arena);
+        return fail(HLRC_ERR_CUDA, "hlrc_workspace_create: %s", cudaGetErrorString(me));
+    }
     if (W->mr_nx) z.carve(W->arena + o_mr, W->ws.mr_x, W->ws.mr_t, W->ws.mr_t2, W->ws.mr_part);
     if (W->w_xs) {
         zw.carve(W->arena + o_w, W->ws);

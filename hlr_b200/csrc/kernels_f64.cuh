@@ -56,6 +56,14 @@ template <> struct Log2<8> { static constexpr int v = 3; };
 template <> struct Log2<16> { static constexpr int v = 4; };
 template <> struct Log2<32> { static constexpr int v = 5; };
 
+// A vector entry: through L2 when another CTA of the same launch may have
+// written it (CG), else through the read-only path.
+template <bool CG>
+__device__ __forceinline__ double ld_vec(const double* p) {
+    if constexpr (CG) return __ldcg(p);
+    else return __ldg(p);
+}
+
 // N-form: one CTA (W warps) per output tile; chunk c goes to warp c % W;
 // lane l owns rows 2l, 2l+1; warps are summed in index order.
 template <int W>
@@ -318,17 +326,10 @@ k_ntree_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, Tr
 
 // T-form: one warp per unit; lane l owns rows 2l, 2l+1 of every slab and
 // keeps NC column partials in registers; one transpose-reduction per unit.
-template <int NC>
-__global__ void __launch_bounds__(256)
-k_tform_f64(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict__ slabs,
-            const double* __restrict__ A, const double* __restrict__ vin, double* __restrict__ out,
-            double* __restrict__ part, double alpha, int add) {
-    pdl_trigger();
-    const int wid = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (wid >= nunits) return;
-    const int lane = threadIdx.x & 31;
-    const TUnit u = units[wid];
-    pdl_wait();
+template <int NC, bool CG>
+__device__ __forceinline__ void tform_unit(const TUnit& u, const TSlab* __restrict__ slabs,
+                                           const double* __restrict__ A, const double* vin, double* out, double* part,
+                                           double alpha, int add, int lane) {
     double p[NC];
 #pragma unroll
     for (int j = 0; j < NC; ++j) p[j] = 0.0;
@@ -340,8 +341,8 @@ k_tform_f64(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict
         const TSlab cur = sl;
         if (s + 1 < u.se) sl = slabs[s + 1];
         if (r < cur.ld) {
-            const double v0 = (r < cur.rows) ? __ldg(vin + cur.v_off + r) : 0.0;
-            const double v1 = (r + 1 < cur.rows) ? __ldg(vin + cur.v_off + r + 1) : 0.0;
+            const double v0 = (r < cur.rows) ? ld_vec<CG>(vin + cur.v_off + r) : 0.0;
+            const double v1 = (r + 1 < cur.rows) ? ld_vec<CG>(vin + cur.v_off + r + 1) : 0.0;
             const double* a = A + cur.a_off + size_t(u.c0) * cur.ld + r;
             double2 m[NC];
 #pragma unroll
@@ -356,12 +357,25 @@ k_tform_f64(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict
     if ((lane & ((1 << SH) - 1)) == 0 && c < u.nc) {
         if (u.flags & TU_DIRECT) {
             double* o = out + u.out + c;
-            if (add) *o += alpha * p[0];
+            if (add) *o = (CG ? __ldcg(o) : *o) + alpha * p[0];
             else *o = p[0];
         } else {
             part[size_t(u.out) * 32 + c] = p[0];
         }
     }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256)
+k_tform_f64(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict__ slabs,
+            const double* __restrict__ A, const double* __restrict__ vin, double* __restrict__ out,
+            double* __restrict__ part, double alpha, int add) {
+    pdl_trigger();
+    const int wid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (wid >= nunits) return;
+    const TUnit u = units[wid];
+    pdl_wait();
+    tform_unit<NC, false>(u, slabs, A, vin, out, part, alpha, add, threadIdx.x & 31);
 }
 
 // Tile T-form: one CTA (W warps) per input tile; x restricted to the tile
@@ -421,15 +435,10 @@ k_ttform_f64(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks,
 
 // Sums the per-tile partials of multi-tile tile-T-form outputs in tile order
 // (one-vector products; a warp per output, lanes over its columns).
-__global__ void __launch_bounds__(256)
-k_ttfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* __restrict__ part,
-               double* __restrict__ out, double alpha, int add) {
-    pdl_trigger();
-    const int gid = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (gid >= ngroups) return;
-    const int lane = threadIdx.x & 31;
-    const TGroup g = groups[gid];
-    pdl_wait();
+template <bool CG>
+__device__ __forceinline__ void ttfinish_group(const TGroup& g, const double* part, double* out, double alpha, int add,
+                                               int lane) {
+    auto ld = [](const double* p) { return CG ? __ldcg(p) : *p; };
     for (uint32_t j = lane; j < g.nc; j += 32) {
         // four interleaved partial sums keep four loads in flight; they are
         // combined in a fixed order, so the result is deterministic
@@ -440,7 +449,7 @@ k_ttfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* __r
         for (; i + 16 <= g.nslots; i += 16) {
             double v[16];
 #pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = p[size_t(i + q) * g.nc];
+            for (int q = 0; q < 16; ++q) v[q] = ld(p + size_t(i + q) * g.nc);
 #pragma unroll
             for (int q = 0; q < 16; q += 4) {
                 s0 += v[q];
@@ -450,35 +459,52 @@ k_ttfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* __r
             }
         }
         for (; i + 4 <= g.nslots; i += 4) {
-            s0 += p[size_t(i) * g.nc];
-            s1 += p[size_t(i + 1) * g.nc];
-            s2 += p[size_t(i + 2) * g.nc];
-            s3 += p[size_t(i + 3) * g.nc];
+            s0 += ld(p + size_t(i) * g.nc);
+            s1 += ld(p + size_t(i + 1) * g.nc);
+            s2 += ld(p + size_t(i + 2) * g.nc);
+            s3 += ld(p + size_t(i + 3) * g.nc);
         }
-        for (; i < g.nslots; ++i) s0 += p[size_t(i) * g.nc];
+        for (; i < g.nslots; ++i) s0 += ld(p + size_t(i) * g.nc);
         const double s = (s0 + s1) + (s2 + s3);
         double* o = out + g.out + j;
-        if (add) *o += alpha * s;
+        if (add) *o = ld(o) + alpha * s;
         else *o = s;
     }
 }
 
+__global__ void __launch_bounds__(256)
+k_ttfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* __restrict__ part,
+               double* __restrict__ out, double alpha, int add) {
+    pdl_trigger();
+    const int gid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (gid >= ngroups) return;
+    const TGroup g = groups[gid];
+    pdl_wait();
+    ttfinish_group<false>(g, part, out, alpha, add, threadIdx.x & 31);
+}
+
 // Sums the partial slots of multi-unit T-form outputs in slot order.
+template <bool CG>
+__device__ __forceinline__ void tfinish_group(const TGroup& g, const double* part, double* out, double alpha, int add,
+                                              int lane) {
+    if (lane >= int(g.nc)) return;
+    auto ld = [](const double* p) { return CG ? __ldcg(p) : *p; };
+    double s = 0.0;
+    for (uint32_t i = 0; i < g.nslots; ++i) s += ld(part + size_t(g.slot0 + i) * 32 + lane);
+    double* o = out + g.out + lane;
+    if (add) *o = ld(o) + alpha * s;
+    else *o = s;
+}
+
 __global__ void __launch_bounds__(256)
 k_tfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* __restrict__ part,
               double* __restrict__ out, double alpha, int add) {
     pdl_trigger();
     const int gid = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gid >= ngroups) return;
-    const int lane = threadIdx.x & 31;
     const TGroup g = groups[gid];
     pdl_wait();
-    if (lane >= int(g.nc)) return;
-    double s = 0.0;
-    for (uint32_t i = 0; i < g.nslots; ++i) s += part[size_t(g.slot0 + i) * 32 + lane];
-    double* o = out + g.out + lane;
-    if (add) *o += alpha * s;
-    else *o = s;
+    tfinish_group<false>(g, part, out, alpha, add, threadIdx.x & 31);
 }
 
 }  // namespace hlrc

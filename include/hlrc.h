@@ -227,7 +227,9 @@ typedef struct hlrc_info {
     int32_t kind;                      /* 0 = H, 1 = uniform-H                  */
     int32_t max_rank;
     int32_t launches[3];               /* kernel launches per product, op N/T/C
-                                          (0 = op unsupported)                  */
+                                          (0 = op unsupported); small FP64
+                                          products outside captures run these
+                                          passes in one launch                  */
     int64_t scratch_bytes;             /* scratch of one one-vector product:
                                           low-rank coefficients and per-tile
                                           partial sums (what hlrc_mvm_noalloc
@@ -443,7 +445,8 @@ hlrc_status hlrc_fp64_peak(int device, double* tflops);
 /* Reads and clears the handle's device error word (synchronous).  Kernels
  * that wait with a bound set it when a wait runs out; the products launched
  * since then are incomplete.  0 means no error; bit 0 (value 1): a copy wait
- * of an H^2 tree sweep ran out; bit 1 (value 2): a stage hand-over of the
+ * of an H^2 tree sweep, or a wait between the passes of a product that runs
+ * as one launch, ran out; bit 1 (value 2): a stage hand-over of the
  * 64-vector kernels ran out.                                                 */
 hlrc_status hlrc_check_device_error(hlrc_hmat M, int* code);
 
@@ -452,8 +455,8 @@ hlrc_status hlrc_check_device_error(hlrc_hmat M, int* code);
  * products (0 restores it).  skip_handover != 0 makes the next products
  * leave one hand-over undone in every CTA that waits: an H^2 tree sweep
  * announces 16 bytes more on its first level's barrier than its copies
- * deliver, and the producers of the 64-vector kernels never signal their
- * first stage.  The waiting kernel then gives up after the bound, records
+ * deliver, the producers of the 64-vector kernels never signal their first
+ * stage, and a product that runs as one launch never counts its first item.  The waiting kernel then gives up after the bound, records
  * the error bit, finishes its copies and MMAs, frees its tensor memory and
  * returns; the product is incomplete and hlrc_check_device_error reports
  * it, and the context stays usable.  Not for use during captures.           */
