@@ -1744,17 +1744,10 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
             const int add = tp.mode != OUT_SET;
             const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
             if (ws.profile) prof_begin(M, stage_name(M, 0, st.idx), tp.alg_bytes, s);
-            for (int c = 0; c < 3; ++c) {
-                const int nu = tp.cls_begin[c + 1] - tp.cls_begin[c];
-                if (nu <= 0) continue;
-                const TUnit* u = tp.units + tp.cls_begin[c];
-                const int grid = (nu + 7) / 8;
-                static_assert(TCOLS == 8, "T-form units are launched with the 8-column kernel");
-                const double* A = reinterpret_cast<const double*>(M->store);  // unit T-form: FP64 plans only
-                if (c == 0) L(launch_k(ov, k_tform_f64<8>, grid, 256, 0, s, u, nu, tp.slabs, A, vin, vout, ws.part, alpha, add));
-                else if (c == 1) L(launch_k(ov, k_tform_f64<16>, grid, 256, 0, s, u, nu, tp.slabs, A, vin, vout, ws.part, alpha, add));
-                else L(launch_k(ov, k_tform_f64<32>, grid, 256, 0, s, u, nu, tp.slabs, A, vin, vout, ws.part, alpha, add));
-            }
+            static_assert(TCOLS == 8, "T-form units are launched with the 8-column kernel");
+            if (const int nu = tp.cls_begin[3]; nu > 0)   // unit T-form: FP64 plans only
+                L(launch_k(ov, k_tform_f64<TCOLS>, unsigned((nu + 7) / 8), 256, 0, s, tp.units, nu, tp.slabs,
+                           reinterpret_cast<const double*>(M->store), vin, vout, ws.part, alpha, add));
             if (tp.ngroups > 0)
                 L(launch_k(ov, k_tfinish_f64, unsigned((tp.ngroups + 7) / 8), 256, 0, s, tp.groups, tp.ngroups,
                            static_cast<const double*>(ws.part), vout, alpha, add));

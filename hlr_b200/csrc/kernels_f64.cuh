@@ -334,21 +334,51 @@ __device__ __forceinline__ void tform_unit(const TUnit& u, const TSlab* __restri
 #pragma unroll
     for (int j = 0; j < NC; ++j) p[j] = 0.0;
     const int r = 2 * lane;
-    // the next slab's descriptor is fetched one iteration ahead so that its
-    // latency overlaps the current slab's loads
-    TSlab sl = u.sb < u.se ? slabs[u.sb] : TSlab{0, 0, 0, 0};
-    for (uint32_t s = u.sb; s < u.se; ++s) {
-        const TSlab cur = sl;
-        if (s + 1 < u.se) sl = slabs[s + 1];
-        if (r < cur.ld) {
-            const double v0 = (r < cur.rows) ? ld_vec<CG>(vin + cur.v_off + r) : 0.0;
-            const double v1 = (r + 1 < cur.rows) ? ld_vec<CG>(vin + cur.v_off + r + 1) : 0.0;
-            const double* a = A + cur.a_off + size_t(u.c0) * cur.ld + r;
-            double2 m[NC];
+    // the next slab is loaded before the current one is added, and its
+    // descriptor a slab earlier: a unit is a chain of short slabs (couplings
+    // of 20 to 40 rows), each a round trip otherwise.  Two operand sets take
+    // 120 registers; with one (and 40 warps per SM) the transposed couplings of
+    // a uniform-H sphere of 32768 triangles (56 MB) took 95 us against 32 us
+    struct Ops {
+        double2 m[NC];
+        double v0, v1;
+    };
+    auto load = [&](const TSlab& q, Ops& o) {
+        const bool in = r < q.ld;
+        o.v0 = r < q.rows ? ld_vec<CG>(vin + q.v_off + r) : 0.0;
+        o.v1 = r + 1 < q.rows ? ld_vec<CG>(vin + q.v_off + r + 1) : 0.0;
+        const double* a = A + q.a_off + size_t(u.c0) * q.ld + r;
 #pragma unroll
-            for (int j = 0; j < NC; ++j) m[j] = (j < u.nc) ? ld_stream(a + size_t(j) * cur.ld) : make_double2(0.0, 0.0);
+        for (int j = 0; j < NC; ++j) o.m[j] = in && j < u.nc ? ld_stream(a + size_t(j) * q.ld) : make_double2(0.0, 0.0);
+    };
+    auto add_slab = [&](const Ops& o) {
 #pragma unroll
-            for (int j = 0; j < NC; ++j) p[j] = fma(m[j].y, v1, fma(m[j].x, v0, p[j]));
+        for (int j = 0; j < NC; ++j) p[j] = fma(o.m[j].y, o.v1, fma(o.m[j].x, o.v0, p[j]));
+    };
+    const TSlab none{0, 0, 0, 0};
+    auto desc = [&](uint32_t s) { return s < u.se ? slabs[s] : none; };
+    if constexpr (CG) {   // inside a launch of several passes: one operand set, for its registers
+        TSlab nx = desc(u.sb);
+        for (uint32_t s = u.sb; s < u.se; ++s) {
+            const TSlab cur = nx;
+            nx = desc(s + 1);
+            Ops o;
+            load(cur, o);
+            add_slab(o);
+        }
+    } else if (u.sb < u.se) {
+        Ops oA, oB;
+        load(slabs[u.sb], oA);
+        TSlab nx = desc(u.sb + 1);
+        for (uint32_t s = u.sb;; s += 2) {
+            const TSlab n2 = desc(s + 2);
+            if (s + 1 < u.se) load(nx, oB);
+            nx = desc(s + 3);
+            add_slab(oA);
+            if (s + 1 >= u.se) break;
+            if (s + 2 < u.se) load(n2, oA);
+            add_slab(oB);
+            if (s + 2 >= u.se) break;
         }
     }
     TransposeReduce<NC, 16>::run(p, lane);
