@@ -2162,7 +2162,9 @@ hlrc_status run_wide(hlrc_hmat M, const Workspace& ws, double alpha, const doubl
         const double* Xr = X + int64_t(r0) * ldx;
         if (ws.profile) prof_begin(M, "wide_xsplit", nx * int64_t(nr) * 8 + nx * WIDE_ROWB, s);
         HLRC_CUDA(cudaMemsetAsync(ws.w_xmax, 0, WIDE_RHS * sizeof(unsigned long long), s));
-        const unsigned gx = unsigned(std::min<int64_t>((nx + 255) / 256, 4 * 148));
+        // eight entries a thread: few maxima per vector meet in the atomics (64
+        // vectors of 32768: the split of x took 30 us, 22 us so)
+        const unsigned gx = unsigned(std::min<int64_t>((nx + 2047) / 2048, 4 * 148));
         k_wide_xmax<<<dim3(std::max(1u, gx), unsigned(nr)), 256, 0, s>>>(Xr, ldx, nx, nr, ws.w_xmax);
         const unsigned gs = unsigned(std::max<int64_t>(1, (nx + TILE - 1) / TILE));
         if (bf) k_wide_xsplit<FMT_BF16><<<gs, 256, 0, s>>>(Xr, ldx, nx, nr, ws.w_xmax, ws.w_xs, ws.w_g);

@@ -43,7 +43,7 @@
 // y_r += alpha F 2^-g_r (acc_hi + acc_lo).  All factors are fixed at upload
 // (WCol, E per run).  The tensor cores accumulate in FP32 over WIDE_FLUSH
 // stages (64 columns) into one of two TMEM buffers; the epilogue warps add
-// each finished buffer to an FP64 accumulator in shared memory while the
+// each finished buffer to FP64 accumulators in registers while the
 // MMAs fill the other, so long runs keep FP64 sums.
 //
 // Roles (224 threads): warps 0-3 read the accumulators (warp w reads TMEM
@@ -85,18 +85,15 @@ constexpr uint32_t WT_EMPTY = 0xffffffffu;   // stacked column without data
 
 // N-form stage: A (vector terms, 2 M-atoms x 4 K-atoms) 8 KB, B (matrix, 4 K-atoms) 4 KB
 constexpr int WIDE_N_STAGE = 12288;
-// N-form FP64 accumulator in shared memory: [vector][row], rows padded to 65
-// (the 16 lanes that add one row of 16 vectors hit 16 different bank pairs)
-constexpr int WIDE_ACC_LD = TILE + 1;
-constexpr int WIDE_ACC_BYTES = WIDE_RHS * WIDE_ACC_LD * 8;
 constexpr int WIDE_WQ_BYTES = WIDE_WQ * WIDE_PRODUCERS * 8;
 // column-cluster T-form stage: A (split rows of a tile: 2 M-atoms x 8 K-atoms)
 // 16 KB, B (<= 128 stacked V columns: 16 atoms) 16 KB
 constexpr int WIDE_C_STAGE = 32768;
-constexpr int WIDE_C_TABLES = WT_MAXB * 16 + WT_MAXN * 4 + WT_MAXT * WT_MAXB * 4;
+// blocks; stacked columns (block and column, output entry, exponent, scale); slabs
+constexpr int WIDE_C_TABLES = WT_MAXB * 16 + WT_MAXN * 4 * 4 + WT_MAXT * WT_MAXB * 4;
 constexpr int WIDE_BAR_BYTES = 256;   // mbarriers and the TMEM address
 constexpr int wide_smem_n() {
-    return 1024 + WIDE_NS_N * WIDE_N_STAGE + WIDE_ACC_BYTES + WIDE_WQ_BYTES + WIDE_BAR_BYTES;
+    return 1024 + WIDE_NS_N * WIDE_N_STAGE + WIDE_WQ_BYTES + WIDE_BAR_BYTES;
 }
 constexpr int wide_smem_c() { return 1024 + WIDE_NS_C * WIDE_C_STAGE + WIDE_C_TABLES + WIDE_BAR_BYTES; }
 static_assert(WIDE_NS_C * WIDE_C_STAGE >= WT_MAXN * WIDE_TERMS * 4, "T-form epilogue transpose fits the stages");
@@ -195,6 +192,7 @@ __global__ void __launch_bounds__(256)
 k_wide_xmax(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, unsigned long long* xmax) {
     const int r = blockIdx.y;
     double m = 0.0;
+#pragma unroll 8
     for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n; i += int64_t(gridDim.x) * 256)
         m = fmax(m, fabs(X[i + int64_t(r) * ldx]));
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -248,7 +246,8 @@ k_wide_xsplit(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, cons
 // entry; a lane holds vectors 2l, 2l + 1
 template <int FMT>
 __device__ __forceinline__ void wide_store_row(double v0, double v1, int e, uint32_t* __restrict__ row, int lane) {
-    reinterpret_cast<uint2*>(row)[lane] = make_uint2(wide_split<FMT>(ldexp(v0, -e)), wide_split<FMT>(ldexp(v1, -e)));
+    const double f = __hiloint2double((1023 - e) << 20, 0);   // 2^-e, |e| < 128: the products equal ldexp
+    reinterpret_cast<uint2*>(row)[lane] = make_uint2(wide_split<FMT>(v0 * f), wide_split<FMT>(v1 * f));
 }
 
 // Partials of the pieces of long column clusters (FP32, 64 per entry:
@@ -311,7 +310,10 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     WTBlk* sblk = reinterpret_cast<WTBlk*>(sm + WIDE_NS_C * WIDE_C_STAGE);
     uint32_t* scol = reinterpret_cast<uint32_t*>(sblk + WT_MAXB);           // stacked column -> (block << 16) | column
-    uint32_t* sslab = scol + WT_MAXN;                                       // [tile][block] store offsets / 16
+    uint32_t* sdst = scol + WT_MAXN;                                        // its output entry,
+    int* sexp = reinterpret_cast<int*>(sdst + WT_MAXN);                     // static exponent
+    float* sscl = reinterpret_cast<float*>(sexp + WT_MAXN);                 // and scale
+    uint32_t* sslab = reinterpret_cast<uint32_t*>(sscl + WT_MAXN);          // [tile][block] store offsets / 16
     uint64_t* full = reinterpret_cast<uint64_t*>(sslab + WT_MAXT * WT_MAXB);
     uint64_t* empty = full + WIDE_NS_C;
     uint64_t* accf = empty + WIDE_NS_C;
@@ -342,6 +344,20 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
     for (int j = threadIdx.x; j < nb; j += WIDE_THREADS)
         for (int l = 0; l < sblk[j].k; ++l) scol[sblk[j].off + l] = (uint32_t(j) << 16) | uint32_t(l);
     __syncthreads();
+    // outputs of the stacked columns, looked up while the tiles are staged: a
+    // load per column in the epilogue is a round trip per column
+    if (warp < 4) {
+        const int n = threadIdx.x;
+        const uint32_t cm = scol[n];
+        if (cm != WT_EMPTY) {
+            const WTBlk& b = sblk[cm >> 16];
+            const uint32_t l = cm & 0xffffu;
+            const uint32_t e = u.npieces == 1 ? b.toff + l : b.pbase + uint32_t(u.piece) * b.k + l;
+            sdst[n] = e;
+            sexp[n] = u.npieces == 1 ? int(texp[e]) : 0;
+            sscl[n] = b.scale;
+        }
+    }
     const uint32_t tmem = *tslot;
 
     if (warp >= 5) {
@@ -430,21 +446,16 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
         tc_fence_before();
         asm volatile("bar.sync 1, 128;\n" ::: "memory");
         if (__all_sync(0xffffffffu, ok)) {
+            // four columns at a time: their conversions and stores overlap
+#pragma unroll 4
             for (int n = warp; n < nc; n += 4) {
-                const uint32_t cm = scol[n];
-                if (cm == WT_EMPTY) continue;
-                const WTBlk& b = sblk[cm >> 16];
-                const int l = int(cm & 0xffffu);
+                if (scol[n] == WT_EMPTY) continue;
                 const float4 t4 = reinterpret_cast<const float4*>(red + n * WIDE_TERMS)[lane];
-                const double sc = double(b.scale);
+                const double sc = double(sscl[n]);
                 const double v0 = (double(t4.x) + double(t4.y)) * sc, v1 = (double(t4.z) + double(t4.w)) * sc;
-                if (u.npieces == 1) {
-                    const size_t e = size_t(b.toff) + size_t(l);
-                    wide_store_row<FMT>(v0, v1, int(texp[e]), ts + e * (WIDE_TERMS / 2), lane);
-                } else {
-                    const size_t e = size_t(b.pbase) + size_t(u.piece) * b.k + size_t(l);
-                    reinterpret_cast<float2*>(part)[e * 32 + lane] = make_float2(float(v0), float(v1));
-                }
+                const size_t e = sdst[n];
+                if (u.npieces == 1) wide_store_row<FMT>(v0, v1, sexp[n], ts + e * (WIDE_TERMS / 2), lane);
+                else reinterpret_cast<float2*>(part)[e * 32 + lane] = make_float2(float(v0), float(v1));
             }
         }
     }
@@ -471,9 +482,8 @@ k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-    double* acc = reinterpret_cast<double*>(sm + WIDE_NS_N * WIDE_N_STAGE);   // [r][row], ld WIDE_ACC_LD
-    uint2* wq = reinterpret_cast<uint2*>(sm + WIDE_NS_N * WIDE_N_STAGE + WIDE_ACC_BYTES);   // [slot][producer]
-    uint64_t* full = reinterpret_cast<uint64_t*>(sm + WIDE_NS_N * WIDE_N_STAGE + WIDE_ACC_BYTES + WIDE_WQ_BYTES);
+    uint2* wq = reinterpret_cast<uint2*>(sm + WIDE_NS_N * WIDE_N_STAGE);   // [slot][producer]
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm + WIDE_NS_N * WIDE_N_STAGE + WIDE_WQ_BYTES);
     uint64_t* empty = full + WIDE_NS_N;
     uint64_t* tfull = empty + WIDE_NS_N;                // accumulator buffers ready
     uint64_t* tempty = tfull + 2;                       // accumulator buffers drained
@@ -487,7 +497,6 @@ k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (nst == 0) return;
     const int E = int(sg.pad);
-    for (int i = threadIdx.x; i < WIDE_RHS * WIDE_ACC_LD; i += WIDE_THREADS) acc[i] = 0.0;
     if (threadIdx.x == 0) {
         for (int i = 0; i < WIDE_NS_N; ++i) {
             mbar_init(full + i, WIDE_PRODUCERS);
@@ -615,11 +624,15 @@ k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const
         __syncwarp();
     } else {
         // -------------------------------------------------------- epilogue
-        // lane m = term m: vector m / 2, hi (even) or lo (odd); the even lane
-        // adds hi + lo of its vector's 64 rows to the FP64 accumulator
+        // lane m = term m: vector m / 2, hi (even) or lo (odd).  The two
+        // lanes of a vector exchange terms: the even lane keeps the FP64 sums
+        // of rows 0-31 in registers, the odd one those of rows 32-63
         const uint32_t la = tmem + (uint32_t(32 * warp) << 16);
-        const int m = 32 * warp + lane;
-        double* arow = acc + (m >> 1) * WIDE_ACC_LD;
+        const int m = 32 * warp + lane, r = m >> 1;
+        const bool odd = (lane & 1) != 0;
+        double acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[i] = 0.0;
         bool ok = true;
         for (int q = 0; q < ngrp; ++q) {
             const int buf = q & 1;
@@ -628,25 +641,28 @@ k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const
             tc_fence_after();
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                float f[32];
-                tmem_ld32(la + uint32_t(buf) * 64u + uint32_t(32 * h), f);
+                float f0[16], f1[16];   // this term's rows 16h .. and 32 + 16h ..
+                tmem_ld16(la + uint32_t(buf) * 64u + uint32_t(16 * h), f0);
+                tmem_ld16(la + uint32_t(buf) * 64u + uint32_t(32 + 16 * h), f1);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float o = __shfl_xor_sync(0xffffffffu, f[i], 1);
-                    if ((lane & 1) == 0) arow[32 * h + i] += double(f[i]) + double(o);
+                for (int i = 0; i < 16; ++i) {
+                    const float o = __shfl_xor_sync(0xffffffffu, odd ? f0[i] : f1[i], 1);
+                    acc[16 * h + i] += double(odd ? f1[i] : f0[i]) + double(o);
                 }
             }
             tc_fence_before();
             mbar_arrive(tempty + buf);
         }
-        asm volatile("bar.sync 1, 128;\n" ::: "memory");
         ok = __all_sync(0xffffffffu, ok) && !wide_aborted(err);
-        if (ok) {
-            for (int q = threadIdx.x; q < WIDE_RHS * TILE; q += 128) {
-                const int r = q / TILE, row = q % TILE;
-                if (r >= om.nr || row >= int(sg.rows)) continue;
-                const double val = ldexp(acc[r * WIDE_ACC_LD + row], E - g[r]);
-                double* o = om.base + int64_t(sg.vo + row) * om.rs + int64_t(r) * om.cs;
+        if (ok && r < om.nr) {
+            const int rg = g[r];
+            double* y = om.base + int64_t(r) * om.cs;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const int row = (odd ? 32 : 0) + i;
+                if (row >= int(sg.rows)) break;
+                const double val = ldexp(acc[i], E - rg);
+                double* o = y + int64_t(sg.vo + row) * om.rs;
                 if (add) *o += alpha * val;
                 else *o = val;
             }
