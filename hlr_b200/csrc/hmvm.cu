@@ -175,6 +175,13 @@ bool has_side(const std::vector<Stage>* nf) {
     return false;
 }
 
+// Pageable vectors of hlrc_mvm_host pass through pinned slots of the handle:
+// the copy of one slot runs while the host fills or adds the next.  The
+// runtime's own path for pageable memory is synchronous; on n = 100003 (three
+// copies of 0.8 MB) it took 240 us of 320.
+constexpr size_t HOST_SLOT = 128 << 10;
+constexpr int HOST_SLOTS = 16;
+
 struct ProfileRec {
     const char* name;
     cudaEvent_t e0, e1;
@@ -247,6 +254,9 @@ struct hlrc_hmat_s {
     double* hx = nullptr;
     double* hy = nullptr;
     size_t hx_elems = 0, hy_elems = 0;
+    char* pin = nullptr;                   // ring of pinned slots for pageable vectors
+    int pin_slots = 0;
+    cudaEvent_t pin_ev[HOST_SLOTS] = {};   // the slot's last copy
     std::mutex host_mu;
     int* dev_err = nullptr;   // device error word (bounded waits that ran out)
     // bound of the device waits and the test hook of hlrc_debug_waits
@@ -2162,8 +2172,7 @@ hlrc_status run_wide(hlrc_hmat M, const Workspace& ws, double alpha, const doubl
         const double* Xr = X + int64_t(r0) * ldx;
         if (ws.profile) prof_begin(M, "wide_xsplit", nx * int64_t(nr) * 8 + nx * WIDE_ROWB, s);
         HLRC_CUDA(cudaMemsetAsync(ws.w_xmax, 0, WIDE_RHS * sizeof(unsigned long long), s));
-        // eight entries a thread: few maxima per vector meet in the atomics (64
-        // vectors of 32768: the split of x took 30 us, 22 us so)
+        // eight entries a thread: few maxima per vector meet in the atomics
         const unsigned gx = unsigned(std::min<int64_t>((nx + 2047) / 2048, 4 * 148));
         k_wide_xmax<<<dim3(std::max(1u, gx), unsigned(nr)), 256, 0, s>>>(Xr, ldx, nx, nr, ws.w_xmax);
         const unsigned gs = unsigned(std::max<int64_t>(1, (nx + TILE - 1) / TILE));
@@ -2252,6 +2261,84 @@ hlrc_status run_wide(hlrc_hmat M, const Workspace& ws, double alpha, const doubl
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(HLRC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
     return HLRC_OK;
+}
+
+// Is p ordinary host memory, unknown to the driver?
+bool pageable(const void* p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
+}
+
+// The ring holds min(HOST_SLOTS, what `bytes` need) slots or more.
+hlrc_status host_ring(hlrc_hmat M, size_t bytes) {
+    const int want = int(std::min<size_t>(HOST_SLOTS, (bytes + HOST_SLOT - 1) / HOST_SLOT));
+    for (cudaEvent_t& e : M->pin_ev)
+        if (!e) HLRC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (want <= M->pin_slots) return HLRC_OK;
+    if (M->pin) cudaFreeHost(M->pin);
+    M->pin = nullptr;
+    M->pin_slots = 0;
+    HLRC_CUDA(cudaMallocHost(&M->pin, size_t(want) * HOST_SLOT));
+    M->pin_slots = want;
+    return HLRC_OK;
+}
+
+// Visits nrhs columns of n doubles, slot by slot: f(element offset in a
+// packed array, column, first row, elements).
+template <typename F>
+hlrc_status host_pieces(int64_t n, int nrhs, F&& f) {
+    constexpr int64_t per = int64_t(HOST_SLOT / sizeof(double));
+    for (int r = 0; r < nrhs; ++r)
+        for (int64_t i = 0; i < n; i += per)
+            if (const hlrc_status st = f(int64_t(r) * n + i, r, i, std::min(per, n - i)); st != HLRC_OK) return st;
+    return HLRC_OK;
+}
+
+// dev (packed) = v, through the ring, on the legacy default stream
+hlrc_status host_put(hlrc_hmat M, double* dev, const double* v, int64_t n, int nrhs, int64_t ld) {
+    int k = 0;
+    return host_pieces(n, nrhs, [&](int64_t at, int r, int64_t i, int64_t m) -> hlrc_status {
+        const int slot = k % M->pin_slots;
+        char* p = M->pin + size_t(slot) * HOST_SLOT;
+        HLRC_CUDA(cudaEventSynchronize(M->pin_ev[slot]));   // also a copy that a failed call left behind
+        std::memcpy(p, v + int64_t(r) * ld + i, size_t(m) * sizeof(double));
+        HLRC_CUDA(cudaMemcpyAsync(dev + at, p, size_t(m) * sizeof(double), cudaMemcpyHostToDevice, nullptr));
+        HLRC_CUDA(cudaEventRecord(M->pin_ev[slot], nullptr));
+        ++k;
+        return HLRC_OK;
+    });
+}
+
+// v += dev (packed), through the ring; returns when v is complete
+hlrc_status host_add(hlrc_hmat M, const double* dev, double* v, int64_t n, int nrhs, int64_t ld) {
+    struct Piece { double* v; int64_t m; };
+    std::vector<Piece> q;   // pieces in flight, by slot
+    q.resize(size_t(M->pin_slots));
+    auto take = [&](int slot) -> hlrc_status {
+        HLRC_CUDA(cudaEventSynchronize(M->pin_ev[slot]));
+        const double* p = reinterpret_cast<const double*>(M->pin + size_t(slot) * HOST_SLOT);
+        const Piece c = q[size_t(slot)];
+        for (int64_t i = 0; i < c.m; ++i) c.v[i] += p[i];
+        return HLRC_OK;
+    };
+    int k = 0;
+    hlrc_status st = host_pieces(n, nrhs, [&](int64_t at, int r, int64_t i, int64_t m) -> hlrc_status {
+        const int slot = k % M->pin_slots;
+        if (k >= M->pin_slots)
+            if (const hlrc_status ts = take(slot); ts != HLRC_OK) return ts;
+        HLRC_CUDA(cudaMemcpyAsync(M->pin + size_t(slot) * HOST_SLOT, dev + at, size_t(m) * sizeof(double),
+                                  cudaMemcpyDeviceToHost, nullptr));
+        HLRC_CUDA(cudaEventRecord(M->pin_ev[slot], nullptr));
+        q[size_t(slot)] = Piece{v + int64_t(r) * ld + i, m};
+        ++k;
+        return HLRC_OK;
+    });
+    for (int j = std::max(0, k - M->pin_slots); j < k && st == HLRC_OK; ++j) st = take(j % M->pin_slots);
+    return st;
 }
 
 hlrc_status check_mvm_args(hlrc_hmat M, int op, const double* x, double* y, int nrhs, int64_t ldx, int64_t ldy) {
@@ -2430,8 +2517,20 @@ extern "C" hlrc_status hlrc_mvm_host(hlrc_hmat M, double alpha, int op, const do
         M->hy_elems = ey;
     }
     const int64_t lx = nrhs > 1 ? ldx : nx, ly = nrhs > 1 ? ldy : ny;
-    HLRC_CUDA(cudaMemcpy2D(M->hx, size_t(nx) * 8, x, size_t(lx) * 8, size_t(nx) * 8, size_t(nrhs), cudaMemcpyHostToDevice));
-    HLRC_CUDA(cudaMemcpy2D(M->hy, size_t(ny) * 8, y, size_t(ly) * 8, size_t(ny) * 8, size_t(nrhs), cudaMemcpyHostToDevice));
+    // pageable y: the product goes into zeroed device memory and the host adds
+    // it to y, which saves y's way down; vectors the driver knows (pinned,
+    // managed) are copied directly
+    const bool add_y = pageable(y), ring_x = pageable(x);
+    if (add_y || ring_x)
+        if (st = host_ring(M, std::max(ring_x ? ex : 0, add_y ? ey : 0) * sizeof(double)); st != HLRC_OK) return st;
+    if (ring_x) {
+        if (st = host_put(M, M->hx, x, nx, nrhs, lx); st != HLRC_OK) return st;
+    } else {
+        HLRC_CUDA(cudaMemcpy2D(M->hx, size_t(nx) * 8, x, size_t(lx) * 8, size_t(nx) * 8, size_t(nrhs), cudaMemcpyHostToDevice));
+    }
+    if (add_y) HLRC_CUDA(cudaMemsetAsync(M->hy, 0, ey * sizeof(double), nullptr));
+    else
+        HLRC_CUDA(cudaMemcpy2D(M->hy, size_t(ny) * 8, y, size_t(ly) * 8, size_t(ny) * 8, size_t(nrhs), cudaMemcpyHostToDevice));
     const Workspace ws = handle_workspace(M);
     if (wide_ok(M, ws, op, nrhs)) {
         st = run_wide(M, ws, alpha, M->hx, nx, M->hy, ny, nrhs, nullptr);
@@ -2445,6 +2544,7 @@ extern "C" hlrc_status hlrc_mvm_host(hlrc_hmat M, double alpha, int op, const do
             if (st != HLRC_OK) return st;
         }
     }
+    if (add_y) return host_add(M, M->hy, y, ny, nrhs, ly);
     HLRC_CUDA(cudaMemcpy2D(y, size_t(ly) * 8, M->hy, size_t(ny) * 8, size_t(ny) * 8, size_t(nrhs), cudaMemcpyDeviceToHost));
     return HLRC_OK;
 }
@@ -2766,6 +2866,9 @@ extern "C" hlrc_status hlrc_free(hlrc_hmat M) {
     }
     cudaFree(M->hx);
     cudaFree(M->hy);
+    if (M->pin) cudaFreeHost(M->pin);
+    for (cudaEvent_t e : M->pin_ev)
+        if (e) cudaEventDestroy(e);
     cudaFree(M->mr_arena);
     cudaFree(M->mr_tables);
     cudaFree(M->w_arena);
