@@ -75,7 +75,11 @@ constexpr int WIDE_THREADS = 224;     // 4 epilogue warps, 1 MMA warp, 2 produce
 constexpr int WIDE_PRODUCERS = 64;
 constexpr int WIDE_NS_N = 6;          // N-form stages (32 columns each): 2 CTAs per SM
 constexpr int WIDE_FLUSH = 2;         // N-form stages per FP32 accumulation (64 columns), then added in FP64
-constexpr int WIDE_NS_C = 3;          // column-cluster T-form stages (one tile each): 2 CTAs per SM
+// Column-cluster T-form stages (one tile each).  Most units have one tile or a
+// few, so a unit is a chain of latencies and CTAs per SM count for more than
+// stages: 361 us with three stages and two CTAs (n = 20011, BF16, 40 vectors),
+// 258 us with two and three, 216 us with one and four (all of the tensor memory).
+constexpr int WIDE_NS_C = 1;
 constexpr int WIDE_LAG_N = WIDE_NS_N - 2;   // copy groups a producer keeps in flight
 constexpr int WIDE_LAG_C = WIDE_NS_C - 1;
 constexpr int WIDE_PF = WIDE_LAG_N + 1;     // N-form: column-table entries prefetched this many stages ahead
@@ -96,7 +100,9 @@ constexpr int wide_smem_n() {
     return 1024 + WIDE_NS_N * WIDE_N_STAGE + WIDE_WQ_BYTES + WIDE_BAR_BYTES;
 }
 constexpr int wide_smem_c() { return 1024 + WIDE_NS_C * WIDE_C_STAGE + WIDE_C_TABLES + WIDE_BAR_BYTES; }
-static_assert(WIDE_NS_C * WIDE_C_STAGE >= WT_MAXN * WIDE_TERMS * 4, "T-form epilogue transpose fits the stages");
+// the T-form epilogue transposes this many columns at a time through the stages
+constexpr int WIDE_C_ROUND = WIDE_NS_C * WIDE_C_STAGE / (WIDE_TERMS * 4) < WT_MAXN
+                                 ? WIDE_NS_C * WIDE_C_STAGE / (WIDE_TERMS * 4) : WT_MAXN;
 
 template <int FMT> struct WideT;
 template <> struct WideT<FMT_F16> {
@@ -112,6 +118,7 @@ template <> struct WideT<FMT_F16> {
         return *reinterpret_cast<uint32_t*>(&x);
     }
     static constexpr bool bf16 = false;
+    static constexpr uint32_t one = 0x3c003c00u;   // 1.0 twice
 };
 template <> struct WideT<FMT_BF16> {
     using h2 = __nv_bfloat162;
@@ -128,6 +135,7 @@ template <> struct WideT<FMT_BF16> {
         return *reinterpret_cast<uint32_t*>(&x);
     }
     static constexpr bool bf16 = true;
+    static constexpr uint32_t one = 0x3f803f80u;
 };
 
 // the two 16-bit terms of v (already scaled), packed lo-term high
@@ -299,7 +307,7 @@ k_ttfinish_wide(const TGroup* __restrict__ groups, int ngroups, const float* __r
 // x N) accumulates over all tiles.  The epilogue transposes D through shared
 // memory and writes one split row (or FP32 partial) per column.
 template <int FMT>
-__global__ void __launch_bounds__(WIDE_THREADS, 2)
+__global__ void __launch_bounds__(WIDE_THREADS, 4)
 k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, const uint32_t* __restrict__ slabs,
               const WTTile* __restrict__ tiles, const uint8_t* __restrict__ A, const uint32_t* __restrict__ xs,
               uint32_t* __restrict__ ts, const int8_t* __restrict__ texp, float* __restrict__ part, int* err,
@@ -430,34 +438,39 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
         bool ok = __all_sync(0xffffffffu, wide_wait(accf, 0u, err, wc.limit_ns) && !wide_aborted(err));
         tc_fence_after();
         // every stage has been consumed: the stage memory holds the
-        // transpose red[n][m] (FP32, 128 terms per stacked column)
+        // transpose red[n][m] (FP32, 128 terms per stacked column) of
+        // WIDE_C_ROUND columns at a time
         float* red = reinterpret_cast<float*>(sm);
-        if (ok) {
-            const uint32_t la = tmem + (uint32_t(32 * warp) << 16);
-            const int m = 32 * warp + lane;
-            for (int c = 0; c < npad; c += 32) {
-                float f[32];
-                tmem_ld32(la + uint32_t(c), f);
+        const uint32_t la = tmem + (uint32_t(32 * warp) << 16);
+        const int m = 32 * warp + lane;
+        for (int n0 = 0; n0 < nc; n0 += WIDE_C_ROUND) {
+            const int n1 = min(nc, n0 + WIDE_C_ROUND);
+            if (n0 > 0) asm volatile("bar.sync 1, 128;\n" ::: "memory");   // the round before is written out
+            if (ok) {
+                for (int c = n0; c < n1; c += 32) {
+                    float f[32];
+                    tmem_ld32(la + uint32_t(c), f);
 #pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    if (c + i < nc) red[(c + i) * WIDE_TERMS + m] = f[i];
+                    for (int i = 0; i < 32; ++i)
+                        if (c + i < n1) red[(c - n0 + i) * WIDE_TERMS + m] = f[i];
+                }
+            }
+            asm volatile("bar.sync 1, 128;\n" ::: "memory");
+            if (ok) {
+                // four columns at a time: their conversions and stores overlap
+#pragma unroll 4
+                for (int n = n0 + warp; n < n1; n += 4) {
+                    if (scol[n] == WT_EMPTY) continue;
+                    const float4 t4 = reinterpret_cast<const float4*>(red + (n - n0) * WIDE_TERMS)[lane];
+                    const double sc = double(sscl[n]);
+                    const double v0 = (double(t4.x) + double(t4.y)) * sc, v1 = (double(t4.z) + double(t4.w)) * sc;
+                    const size_t e = sdst[n];
+                    if (u.npieces == 1) wide_store_row<FMT>(v0, v1, sexp[n], ts + e * (WIDE_TERMS / 2), lane);
+                    else reinterpret_cast<float2*>(part)[e * 32 + lane] = make_float2(float(v0), float(v1));
+                }
             }
         }
         tc_fence_before();
-        asm volatile("bar.sync 1, 128;\n" ::: "memory");
-        if (__all_sync(0xffffffffu, ok)) {
-            // four columns at a time: their conversions and stores overlap
-#pragma unroll 4
-            for (int n = warp; n < nc; n += 4) {
-                if (scol[n] == WT_EMPTY) continue;
-                const float4 t4 = reinterpret_cast<const float4*>(red + n * WIDE_TERMS)[lane];
-                const double sc = double(sscl[n]);
-                const double v0 = (double(t4.x) + double(t4.y)) * sc, v1 = (double(t4.z) + double(t4.w)) * sc;
-                const size_t e = sdst[n];
-                if (u.npieces == 1) wide_store_row<FMT>(v0, v1, sexp[n], ts + e * (WIDE_TERMS / 2), lane);
-                else reinterpret_cast<float2*>(part)[e * 32 + lane] = make_float2(float(v0), float(v1));
-            }
-        }
     }
     tc_fence_before();
     __syncthreads();
@@ -540,14 +553,18 @@ k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const
         tc5::cp_wait<0>();
         auto finish = [&](int sd) {   // stage sd has landed: scale its matrix column, hand it over
             const uint32_t fb = wq[(sd % WIDE_WQ) * WIDE_PRODUCERS + p].y;
-            const typename W::h2 f = *reinterpret_cast<const typename W::h2*>(&fb);
-            uint8_t* col = sm + (sd % WIDE_NS_N) * WIDE_N_STAGE + 8192 + (k >> 3) * 1024;
+            // factor 1 (every column of a store whose row tiles share one
+            // scale) leaves the column as it is
+            if (fb != W::one) {
+                const typename W::h2 f = *reinterpret_cast<const typename W::h2*>(&fb);
+                uint8_t* col = sm + (sd % WIDE_NS_N) * WIDE_N_STAGE + 8192 + (k >> 3) * 1024;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint4* q = reinterpret_cast<uint4*>(col + swz(k & 7, 4 * half + i));
-                uint4 w = *q;
-                w.x = W::mul(w.x, f); w.y = W::mul(w.y, f); w.z = W::mul(w.z, f); w.w = W::mul(w.w, f);
-                *q = w;
+                for (int i = 0; i < 4; ++i) {
+                    uint4* q = reinterpret_cast<uint4*>(col + swz(k & 7, 4 * half + i));
+                    uint4 w = *q;
+                    w.x = W::mul(w.x, f); w.y = W::mul(w.y, f); w.z = W::mul(w.z, f); w.w = W::mul(w.w, f);
+                    *q = w;
+                }
             }
             fence_async_smem();
             if (!(wc.skip && sd == 0)) mbar_arrive(full + sd % WIDE_NS_N);
