@@ -136,7 +136,7 @@ struct Workspace {
     uint32_t* w_xs = nullptr;
     uint32_t* w_ts = nullptr;
     float* w_part = nullptr;
-    unsigned long long* w_xmax = nullptr;
+    double* w_xmax = nullptr;
     int* w_g = nullptr;
     // TMA views of w_xs (boxes of 16 and 64 split rows) and w_ts (16 rows)
     bool has_tm = false;
@@ -809,7 +809,7 @@ struct WideSizes {
         w.w_xs = reinterpret_cast<uint32_t*>(take(xs));
         w.w_ts = reinterpret_cast<uint32_t*>(take(ts));
         w.w_part = reinterpret_cast<float*>(take(part));
-        w.w_xmax = reinterpret_cast<unsigned long long*>(take(WIDE_RHS * sizeof(unsigned long long)));
+        w.w_xmax = reinterpret_cast<double*>(take(WIDE_RHS * WIDE_XBLOCKS * sizeof(double)));
         w.w_g = reinterpret_cast<int*>(take(WIDE_RHS * sizeof(int)));
     }
 };
@@ -819,7 +819,7 @@ WideSizes wide_sizes(hlrc_hmat M) {
     z.xs = size_t(std::max(M->nrows, M->ncols)) * WIDE_ROWB;
     z.ts = size_t(std::max<int64_t>(1, M->n_t)) * WIDE_ROWB;
     z.part = size_t(std::max<int64_t>(1, M->w_npart)) * WIDE_RHS * sizeof(float);
-    z.bytes = z.xs + z.ts + z.part + 2 * WIDE_RHS * 8 + 6 * 256;
+    z.bytes = z.xs + z.ts + z.part + WIDE_RHS * (WIDE_XBLOCKS + 1) * 8 + 6 * 256;
     return z;
 }
 
@@ -1610,10 +1610,10 @@ bool capturing(cudaStream_t s) {
 // while the preceding kernel of the stream still runs, and waits for it
 // inside (pdl_wait) before it touches the vectors.
 template <typename... P, typename... A>
-cudaError_t launch_k(bool overlap, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+cudaError_t launch_k(bool overlap, void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
                      A... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -2024,6 +2024,9 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                       double* Y, int64_t ldy, int nrhs, cudaStream_t s0) {
     if (M->precision == HLRC_PREC_F64) return run_multi_f64(M, ws, alpha_in, op, X, ldx, Y, ldy, nrhs, s0);
     const int64_t nx = op == HLRC_OP_N ? M->ncols : M->nrows;
+    const bool ov = M->overlap != 0;
+    cudaError_t le = cudaSuccess;   // the first failed launch
+    auto L = [&](cudaError_t e) { if (le == cudaSuccess) le = e; };
     for (int r0 = 0; r0 < nrhs; r0 += MR_RB) {
         const cudaStream_t s = s0;
         // side stages read the block of x staged below and add into Y; the
@@ -2031,7 +2034,7 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
         SideFork side{M, ws, s0};
         const int nr = std::min(MR_RB, nrhs - r0);
         const int64_t tot = nx * MR_RB;
-        k_rows_from_cols<<<unsigned((tot + 255) / 256), 256, 0, s>>>(X, ldx, nx, r0, nr, ws.mr_x);
+        L(launch_k(ov, k_rows_from_cols, unsigned((tot + 255) / 256), 256, 0, s, X, ldx, nx, r0, nr, ws.mr_x));
         M->launches += 1;
         HLRC_AFTER_LAUNCH("rows_from_cols");
         int nl = 0;   // kernels launched below, counted at their launch sites
@@ -2056,27 +2059,29 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 if (M->precision == HLRC_PREC_BFP) {
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     if (tp.nmseg[FMT_I24] > 0) {
-                        k_ttform_bfp<true><<<tp.nmseg[FMT_I24], TC_WARPS * 32, bq_smem_t(true), s>>>(
-                            tp.mseg[FMT_I24], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add);
+                        L(launch_k(ov, k_ttform_bfp<true>, unsigned(tp.nmseg[FMT_I24]), TC_WARPS * 32,
+                                   bq_smem_t(true), s, tp.mseg[FMT_I24], tp.mcol, M->store, vec(tp.in), om, fpart,
+                                   alpha, add));
                         ++nl;
                     }
                     if (tp.nmseg[FMT_I16] > 0) {
-                        k_ttform_bfp<false><<<tp.nmseg[FMT_I16], TC_WARPS * 32, bq_smem_t(false), s>>>(
-                            tp.mseg[FMT_I16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add);
+                        L(launch_k(ov, k_ttform_bfp<false>, unsigned(tp.nmseg[FMT_I16]), TC_WARPS * 32,
+                                   bq_smem_t(false), s, tp.mseg[FMT_I16], tp.mcol, M->store, vec(tp.in), om, fpart,
+                                   alpha, add));
                         ++nl;
                     }
                 } else {
                     const int n32 = tp.nmseg[FMT_F32];
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     if (tp.nmseg[FMT_BF16] > 0) {
-                        k_ttform_mr<FMT_BF16><<<n32 + tp.nmseg[FMT_BF16], TC_WARPS * 32,
-                                               tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s>>>(
-                            tp.mseg[FMT_F32], n32, tp.mseg[FMT_BF16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add);
+                        L(launch_k(ov, k_ttform_mr<FMT_BF16>, unsigned(n32 + tp.nmseg[FMT_BF16]), TC_WARPS * 32,
+                                   tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s, tp.mseg[FMT_F32], n32,
+                                   tp.mseg[FMT_BF16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add));
                         ++nl;
                     } else if (n32 + tp.nmseg[FMT_F16] > 0) {
-                        k_ttform_mr<FMT_F16><<<n32 + tp.nmseg[FMT_F16], TC_WARPS * 32,
-                                               tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s>>>(
-                            tp.mseg[FMT_F32], n32, tp.mseg[FMT_F16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add);
+                        L(launch_k(ov, k_ttform_mr<FMT_F16>, unsigned(n32 + tp.nmseg[FMT_F16]), TC_WARPS * 32,
+                                   tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s, tp.mseg[FMT_F32], n32,
+                                   tp.mseg[FMT_F16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add));
                         ++nl;
                     }
                 }
@@ -2090,10 +2095,10 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                     const unsigned fg1 = unsigned((tp.ngroups1 + b1 - 1) / b1);
                     const unsigned fg = unsigned((tp.ngroups + b2 - 1) / b2);
                     if (tp.ngroups1 > 0)
-                        k_ttfinish_flat<MR_RB, float, true><<<fg1, 256, 0, s>>>(tp.groups1, tp.ngroups1, b1, fpart, pm,
-                                                                                fpart, 1.0, 0);
-                    k_ttfinish_flat<MR_RB, float, false><<<fg, 256, 0, s>>>(tp.groups, tp.ngroups, b2, fpart, om,
-                                                                            static_cast<float*>(nullptr), alpha, add);
+                        L(launch_k(ov, k_ttfinish_flat<MR_RB, float, true>, fg1, 256, 0, s, tp.groups1, tp.ngroups1,
+                                   b1, fpart, pm, fpart, 1.0, 0));
+                    L(launch_k(ov, k_ttfinish_flat<MR_RB, float, false>, fg, 256, 0, s, tp.groups, tp.ngroups, b2,
+                               fpart, om, static_cast<float*>(nullptr), alpha, add));
                     nl += 1 + (tp.ngroups1 > 0 ? 1 : 0);
                     if (ws.profile) prof_end(M, s);
                 }
@@ -2109,30 +2114,31 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 // the formats of one output tile run as separate grids, each
                 // adding its share to the output in a fixed launch order
                 if (np.nmseg[FMT_F32] > 0) {
-                    k_nform_d32<<<np.nmseg[FMT_F32], TC_WARPS * 32, tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32), s>>>(
-                        np.mseg[FMT_F32], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
+                    L(launch_k(ov, k_nform_d32, unsigned(np.nmseg[FMT_F32]), TC_WARPS * 32,
+                               tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32), s, np.mseg[FMT_F32], np.mcol, M->store,
+                               vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_F16] > 0) {
-                    k_nform_tc<FMT_F16><<<np.nmseg[FMT_F16], TC_WARPS * 32,
-                                          tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s>>>(
-                        np.mseg[FMT_F16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
+                    L(launch_k(ov, k_nform_tc<FMT_F16>, unsigned(np.nmseg[FMT_F16]), TC_WARPS * 32,
+                               tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s, np.mseg[FMT_F16], np.mcol, M->store,
+                               vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_BF16] > 0) {
-                    k_nform_tc<FMT_BF16><<<np.nmseg[FMT_BF16], TC_WARPS * 32,
-                                           tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s>>>(
-                        np.mseg[FMT_BF16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
+                    L(launch_k(ov, k_nform_tc<FMT_BF16>, unsigned(np.nmseg[FMT_BF16]), TC_WARPS * 32,
+                               tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s, np.mseg[FMT_BF16], np.mcol, M->store,
+                               vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_I24] > 0) {
-                    k_nform_bfp<true><<<np.nmseg[FMT_I24], TC_WARPS * 32, bq_smem_n(true), s>>>(
-                        np.mseg[FMT_I24], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
+                    L(launch_k(ov, k_nform_bfp<true>, unsigned(np.nmseg[FMT_I24]), TC_WARPS * 32, bq_smem_n(true), s,
+                               np.mseg[FMT_I24], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_I16] > 0) {
-                    k_nform_bfp<false><<<np.nmseg[FMT_I16], TC_WARPS * 32, bq_smem_n(false), s>>>(
-                        np.mseg[FMT_I16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add);
+                    L(launch_k(ov, k_nform_bfp<false>, unsigned(np.nmseg[FMT_I16]), TC_WARPS * 32, bq_smem_n(false),
+                               s, np.mseg[FMT_I16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (ws.profile) prof_end(M, s);
@@ -2143,7 +2149,7 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
         if (const cudaError_t fe = side.end(); fe != cudaSuccess)
             return fail(HLRC_ERR_CUDA, "side stream: %s", cudaGetErrorString(fe));
     }
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = le != cudaSuccess ? le : cudaGetLastError();
     if (e != cudaSuccess) return fail(HLRC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
     return HLRC_OK;
 }
@@ -2167,17 +2173,20 @@ hlrc_status run_wide(hlrc_hmat M, const Workspace& ws, double alpha, const doubl
     const DevNPass& np = M->n[size_t(st[1].idx)];
     const int64_t nx = M->ncols;
     const bool bf = f == FMT_BF16;
+    const bool ov = M->overlap != 0;
+    cudaError_t le = cudaSuccess;   // the first failed launch
+    auto L = [&](cudaError_t e) { if (le == cudaSuccess) le = e; };
     for (int r0 = 0; r0 < nrhs; r0 += WIDE_RHS) {
         const int nr = std::min(WIDE_RHS, nrhs - r0);
         const double* Xr = X + int64_t(r0) * ldx;
         if (ws.profile) prof_begin(M, "wide_xsplit", nx * int64_t(nr) * 8 + nx * WIDE_ROWB, s);
-        HLRC_CUDA(cudaMemsetAsync(ws.w_xmax, 0, WIDE_RHS * sizeof(unsigned long long), s));
-        // eight entries a thread: few maxima per vector meet in the atomics
-        const unsigned gx = unsigned(std::min<int64_t>((nx + 2047) / 2048, 4 * 148));
-        k_wide_xmax<<<dim3(std::max(1u, gx), unsigned(nr)), 256, 0, s>>>(Xr, ldx, nx, nr, ws.w_xmax);
+        // one maximum per vector and block, at most WIDE_XBLOCKS of them
+        const int gx = int(std::max<int64_t>(1, std::min<int64_t>((nx + 2047) / 2048, WIDE_XBLOCKS)));
+        L(launch_k(ov, k_wide_xmax, dim3(unsigned(gx), unsigned(nr)), 256, 0, s, Xr, ldx, nx, ws.w_xmax));
         const unsigned gs = unsigned(std::max<int64_t>(1, (nx + TILE - 1) / TILE));
-        if (bf) k_wide_xsplit<FMT_BF16><<<gs, 256, 0, s>>>(Xr, ldx, nx, nr, ws.w_xmax, ws.w_xs, ws.w_g);
-        else k_wide_xsplit<FMT_F16><<<gs, 256, 0, s>>>(Xr, ldx, nx, nr, ws.w_xmax, ws.w_xs, ws.w_g);
+        if (bf) L(launch_k(ov, k_wide_xsplit<FMT_BF16>, gs, 256, 0, s, Xr, ldx, nx, nr, ws.w_xmax, gx, ws.w_xs,
+                           ws.w_g));
+        else L(launch_k(ov, k_wide_xsplit<FMT_F16>, gs, 256, 0, s, Xr, ldx, nx, nr, ws.w_xmax, gx, ws.w_xs, ws.w_g));
         if (ws.profile) prof_end(M, s);
         M->launches += 2;
         HLRC_AFTER_LAUNCH("wide_xsplit");
@@ -2193,24 +2202,24 @@ hlrc_status run_wide(hlrc_hmat M, const Workspace& ws, double alpha, const doubl
             if (ntma > 0) {
                 const int grid = std::min(ntma, 2 * M->sms);
                 if (bf)
-                    k_ctform_wtma<FMT_BF16><<<grid, WTMA_THREADS_C, wtma_smem_c(), s>>>(
-                        M->w_units_tma, ntma, M->w_blks, M->w_slabs, M->w_tiles, M->w_ctab, M->tm_s8, ws.tm_x64,
-                        ws.w_ts, ws.w_part, M->dev_err, wc);
+                    L(launch_k(ov, k_ctform_wtma<FMT_BF16>, unsigned(grid), WTMA_THREADS_C, wtma_smem_c(), s,
+                               M->w_units_tma, ntma, M->w_blks, M->w_slabs, M->w_tiles, M->w_ctab, M->tm_s8,
+                               ws.tm_x64, ws.w_ts, ws.w_part, M->dev_err, wc));
                 else
-                    k_ctform_wtma<FMT_F16><<<grid, WTMA_THREADS_C, wtma_smem_c(), s>>>(
-                        M->w_units_tma, ntma, M->w_blks, M->w_slabs, M->w_tiles, M->w_ctab, M->tm_s8, ws.tm_x64,
-                        ws.w_ts, ws.w_part, M->dev_err, wc);
+                    L(launch_k(ov, k_ctform_wtma<FMT_F16>, unsigned(grid), WTMA_THREADS_C, wtma_smem_c(), s,
+                               M->w_units_tma, ntma, M->w_blks, M->w_slabs, M->w_tiles, M->w_ctab, M->tm_s8,
+                               ws.tm_x64, ws.w_ts, ws.w_part, M->dev_err, wc));
                 M->launches += 1;
             }
             if (ncp > 0) {
                 if (bf)
-                    k_ctform_wide<FMT_BF16><<<ncp, WIDE_THREADS, wide_smem_c(), s>>>(
-                        ucp, M->w_blks, M->w_slabs, M->w_tiles, M->store, ws.w_xs, ws.w_ts, M->w_texp, ws.w_part,
-                        M->dev_err, wc);
+                    L(launch_k(ov, k_ctform_wide<FMT_BF16>, unsigned(ncp), WIDE_THREADS, wide_smem_c(), s, ucp,
+                               M->w_blks, M->w_slabs, M->w_tiles, M->store, ws.w_xs, ws.w_ts, M->w_texp, ws.w_part,
+                               M->dev_err, wc));
                 else
-                    k_ctform_wide<FMT_F16><<<ncp, WIDE_THREADS, wide_smem_c(), s>>>(
-                        ucp, M->w_blks, M->w_slabs, M->w_tiles, M->store, ws.w_xs, ws.w_ts, M->w_texp, ws.w_part,
-                        M->dev_err, wc);
+                    L(launch_k(ov, k_ctform_wide<FMT_F16>, unsigned(ncp), WIDE_THREADS, wide_smem_c(), s, ucp,
+                               M->w_blks, M->w_slabs, M->w_tiles, M->store, ws.w_xs, ws.w_ts, M->w_texp, ws.w_part,
+                               M->dev_err, wc));
                 M->launches += 1;
             }
             if (ws.profile) prof_end(M, s);
@@ -2219,11 +2228,11 @@ hlrc_status run_wide(hlrc_hmat M, const Workspace& ws, double alpha, const doubl
         if (M->w_ngroups > 0) {
             if (ws.profile) prof_begin(M, "ttfinish", M->w_npart * WIDE_RHS * 4, s);
             if (bf)
-                k_ttfinish_wide<FMT_BF16><<<(M->w_ngroups + 7) / 8, 256, 0, s>>>(M->w_groups, M->w_ngroups, ws.w_part,
-                                                                                  ws.w_ts, M->w_texp);
+                L(launch_k(ov, k_ttfinish_wide<FMT_BF16>, unsigned((M->w_ngroups + 7) / 8), 256, 0, s, M->w_groups,
+                           M->w_ngroups, ws.w_part, ws.w_ts, M->w_texp));
             else
-                k_ttfinish_wide<FMT_F16><<<(M->w_ngroups + 7) / 8, 256, 0, s>>>(M->w_groups, M->w_ngroups, ws.w_part,
-                                                                                 ws.w_ts, M->w_texp);
+                L(launch_k(ov, k_ttfinish_wide<FMT_F16>, unsigned((M->w_ngroups + 7) / 8), 256, 0, s, M->w_groups,
+                           M->w_ngroups, ws.w_part, ws.w_ts, M->w_texp));
             if (ws.profile) prof_end(M, s);
             M->launches += 1;
             HLRC_AFTER_LAUNCH("ttfinish");
@@ -2238,27 +2247,27 @@ hlrc_status run_wide(hlrc_hmat M, const Workspace& ws, double alpha, const doubl
             if (ws.profile) prof_begin(M, stage_name(M, 1, st[1].idx), np.alg_bytes, s);
             if (nwt > 0) {
                 if (bf)
-                    k_nform_wtma<FMT_BF16><<<nwt, WTMA_THREADS, wtma_smem_n(), s>>>(
-                        np.wseg, np.wstage, M->tm_s16, ws.tm_x16, ws.tm_t16, ws.w_g, om, alpha, M->dev_err, wc);
+                    L(launch_k(ov, k_nform_wtma<FMT_BF16>, unsigned(nwt), WTMA_THREADS, wtma_smem_n(), s, np.wseg,
+                               np.wstage, M->tm_s16, ws.tm_x16, ws.tm_t16, ws.w_g, om, alpha, M->dev_err, wc));
                 else
-                    k_nform_wtma<FMT_F16><<<nwt, WTMA_THREADS, wtma_smem_n(), s>>>(
-                        np.wseg, np.wstage, M->tm_s16, ws.tm_x16, ws.tm_t16, ws.w_g, om, alpha, M->dev_err, wc);
+                    L(launch_k(ov, k_nform_wtma<FMT_F16>, unsigned(nwt), WTMA_THREADS, wtma_smem_n(), s, np.wseg,
+                               np.wstage, M->tm_s16, ws.tm_x16, ws.tm_t16, ws.w_g, om, alpha, M->dev_err, wc));
                 M->launches += 1;
             }
             if (nmcp > 0) {
                 if (bf)
-                    k_nform_wide<FMT_BF16><<<nmcp, WIDE_THREADS, wide_smem_n(), s>>>(
-                        mcp, np.wcol, M->store, ws.w_xs, ws.w_ts, ws.w_g, om, alpha, 1, M->dev_err, wc);
+                    L(launch_k(ov, k_nform_wide<FMT_BF16>, unsigned(nmcp), WIDE_THREADS, wide_smem_n(), s, mcp,
+                               np.wcol, M->store, ws.w_xs, ws.w_ts, ws.w_g, om, alpha, 1, M->dev_err, wc));
                 else
-                    k_nform_wide<FMT_F16><<<nmcp, WIDE_THREADS, wide_smem_n(), s>>>(
-                        mcp, np.wcol, M->store, ws.w_xs, ws.w_ts, ws.w_g, om, alpha, 1, M->dev_err, wc);
+                    L(launch_k(ov, k_nform_wide<FMT_F16>, unsigned(nmcp), WIDE_THREADS, wide_smem_n(), s, mcp,
+                               np.wcol, M->store, ws.w_xs, ws.w_ts, ws.w_g, om, alpha, 1, M->dev_err, wc));
                 M->launches += 1;
             }
             if (ws.profile) prof_end(M, s);
             HLRC_AFTER_LAUNCH(stage_name(M, 1, st[1].idx));
         }
     }
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = le != cudaSuccess ? le : cudaGetLastError();
     if (e != cudaSuccess) return fail(HLRC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
     return HLRC_OK;
 }

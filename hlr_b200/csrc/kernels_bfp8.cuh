@@ -144,7 +144,9 @@ k_nform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const 
     constexpr int VOFF = I24 ? BQ_PLANE + 32 * BQ_LO_STRIDE : BQ_PLANE;   // vector part of a stage
     constexpr int NT = I24 ? 3 : 2;                                        // FP16 terms of the vector operand
     extern __shared__ __align__(16) uint8_t smem[];
+    pdl_trigger();
     const MSeg sg = segs[blockIdx.x];
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* ring = smem + warp * (BQ_STAGES * STAGE + (I24 ? BQ_PLANE : 0));
@@ -402,6 +404,8 @@ __global__ void __launch_bounds__(TC_WARPS * 32, HLRC_BQ_MINB)
 k_ttform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
              const double* __restrict__ vin, OutMap om, float* __restrict__ part, double alpha, int add) {
     extern __shared__ __align__(16) uint8_t smem[];
+    pdl_trigger();
+    pdl_wait();
     ttform_bfp<I24>(segs[blockIdx.x], smem, cols, A, vin, om, part, alpha, add);
 }
 

@@ -25,8 +25,10 @@ constexpr int MR_RB = 8;   // right-hand sides per block (kernels, finish, works
 // xr[i * RB + r] = X[i + (r0 + r) * ldx] for r < nr, 0 for nr <= r < RB
 __global__ void k_rows_from_cols(const double* __restrict__ X, int64_t ldx, int64_t n, int r0, int nr,
                                  double* __restrict__ xr) {
+    pdl_trigger();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= n * MR_RB) return;
+    pdl_wait();
     const int64_t i = idx / MR_RB;
     const int r = int(idx % MR_RB);
     xr[idx] = r < nr ? X[i + int64_t(r0 + r) * ldx] : 0.0;

@@ -358,7 +358,9 @@ k_nform_tc(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const u
            const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
     using O = TcOp<FMT>;
     extern __shared__ __align__(16) uint8_t smem[];
+    pdl_trigger();
     const MSeg sg = segs[blockIdx.x];
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* ring = smem + warp * (TC_STAGES_N16 * TC_STAGE_N16);
@@ -523,7 +525,9 @@ __global__ void __launch_bounds__(TC_WARPS * 32)
 k_nform_d32(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
             const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
     extern __shared__ __align__(16) uint8_t smem[];
+    pdl_trigger();
     const MSeg sg = segs[blockIdx.x];
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* ring = smem + warp * (TC_STAGES_D32 * TC_STAGE_N32);
@@ -592,6 +596,8 @@ k_ttform_mr(const MSeg* __restrict__ segs32, int n32, const MSeg* __restrict__ s
             const uint8_t* __restrict__ A, const double* __restrict__ vin, OutMap om, float* __restrict__ part,
             double alpha, int add) {
     extern __shared__ __align__(16) uint8_t smem[];
+    pdl_trigger();
+    pdl_wait();
     if (int(blockIdx.x) < n32) ttform_d32(segs32[blockIdx.x], smem, cols, A, vin, om, part, alpha, add);
     else ttform_tc<F16>(segs16[blockIdx.x - n32], smem, cols, A, vin, om, part, alpha, add);
 }

@@ -194,11 +194,13 @@ __device__ __forceinline__ bool wide_wait(uint64_t* bar, uint32_t parity, int* e
 }
 
 // ------------------------------------------------------------- x -> xs
-// largest |x| of each vector: xmax[r] (as the bits of a non-negative double,
-// which order like unsigned integers), zeroed before the launch
+// Largest |x| of each vector, one maximum per block: xmax[r * WIDE_XBLOCKS + b]
+constexpr int WIDE_XBLOCKS = 32;
 __global__ void __launch_bounds__(256)
-k_wide_xmax(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, unsigned long long* xmax) {
+k_wide_xmax(const double* __restrict__ X, int64_t ldx, int64_t n, double* __restrict__ xmax) {
+    pdl_trigger();
     const int r = blockIdx.y;
+    pdl_wait();
     double m = 0.0;
 #pragma unroll 8
     for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n; i += int64_t(gridDim.x) * 256)
@@ -209,13 +211,14 @@ k_wide_xmax(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, unsign
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < 8; ++w) m = fmax(m, red[w]);
-        if (r < nr && m > 0.0) atomicMax(xmax + r, static_cast<unsigned long long>(__double_as_longlong(m)));
+        xmax[r * WIDE_XBLOCKS + int(blockIdx.x)] = m;
     }
 }
 
-// g_r = 13 - ilogb(max |x_r|) (0 for a zero vector)
-__device__ __forceinline__ int wide_xg(const unsigned long long* xmax, int r) {
-    const double m = __longlong_as_double(static_cast<long long>(xmax[r]));
+// g_r = 13 - ilogb(max |x_r|) (0 for a zero vector) of nb blocks' maxima
+__device__ __forceinline__ int wide_xg(const double* xmax, int nb, int r) {
+    double m = 0.0;
+    for (int b = 0; b < nb; ++b) m = fmax(m, xmax[r * WIDE_XBLOCKS + b]);
     return m > 0.0 ? 13 - ilogb(m) : 0;
 }
 
@@ -224,13 +227,15 @@ __device__ __forceinline__ int wide_xg(const unsigned long long* xmax, int r) {
 // vectors r >= nr are zero.  Also writes g[] (block 0).
 template <int FMT>
 __global__ void __launch_bounds__(256)
-k_wide_xsplit(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, const unsigned long long* xmax,
+k_wide_xsplit(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, const double* __restrict__ xmax, int nb,
               uint32_t* __restrict__ xs, int* __restrict__ g) {
     __shared__ double tile[WIDE_RHS][TILE + 1];
     __shared__ double sc[WIDE_RHS];
+    pdl_trigger();
     const int64_t i0 = int64_t(blockIdx.x) * TILE;
+    pdl_wait();
     if (threadIdx.x < WIDE_RHS) {
-        const int gr = threadIdx.x < nr ? wide_xg(xmax, threadIdx.x) : 0;
+        const int gr = threadIdx.x < nr ? wide_xg(xmax, nb, threadIdx.x) : 0;
         sc[threadIdx.x] = ldexp(1.0, gr);
         if (blockIdx.x == 0) g[threadIdx.x] = gr;
     }
@@ -267,10 +272,12 @@ template <int FMT>
 __global__ void __launch_bounds__(256)
 k_ttfinish_wide(const TGroup* __restrict__ groups, int ngroups, const float* __restrict__ part,
                 uint32_t* __restrict__ ts, const int8_t* __restrict__ texp) {
+    pdl_trigger();
     const int gid = int(blockIdx.x) * 8 + int(threadIdx.x >> 5);
     if (gid >= ngroups) return;
     const int lane = threadIdx.x & 31;
     const TGroup gr = groups[gid];
+    pdl_wait();
     const size_t step = size_t(gr.nc) * 32;
     for (uint32_t j = 0; j < gr.nc; ++j) {
         const float2* p = reinterpret_cast<const float2*>(part) + (size_t(gr.slot0) + j) * 32 + lane;
@@ -314,6 +321,10 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
               WaitCfg wc) {
     using namespace tc5;
     extern __shared__ uint8_t smem_raw[];
+    // a CTA that waits for the kernel before holds no tensor memory yet: CTAs
+    // of that kernel may still have to allocate theirs
+    pdl_trigger();
+    pdl_wait();
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     WTBlk* sblk = reinterpret_cast<WTBlk*>(sm + WIDE_NS_C * WIDE_C_STAGE);
@@ -493,6 +504,10 @@ k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const
     using namespace tc5;
     using W = WideT<FMT>;
     extern __shared__ uint8_t smem_raw[];
+    // a CTA that waits for the kernel before holds no tensor memory yet: CTAs
+    // of that kernel may still have to allocate theirs
+    pdl_trigger();
+    pdl_wait();
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     uint2* wq = reinterpret_cast<uint2*>(sm + WIDE_NS_N * WIDE_N_STAGE);   // [slot][producer]

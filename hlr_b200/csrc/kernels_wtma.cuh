@@ -70,6 +70,8 @@ k_nform_wtma(const WSeg* __restrict__ segs, const WStage* __restrict__ stages, c
              const int* __restrict__ g, OutMap om, double alpha, int* err, WaitCfg wc) {
     using namespace tc5;
     extern __shared__ uint8_t smem_raw[];
+    pdl_trigger();   // as in kernels_wide.cuh: before any tensor memory is held
+    pdl_wait();
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     int* snc = reinterpret_cast<int*>(sm + WTMA_NS_N * WIDE_N_STAGE);   // columns per slot
@@ -224,6 +226,8 @@ k_ctform_wtma(const WTUnit* __restrict__ units, int nunits, const WTBlk* __restr
     using namespace tc5;
     constexpr int MMA_WARP = 8, PROD_WARP = 9;
     extern __shared__ uint8_t smem_raw[];
+    pdl_trigger();   // as in kernels_wide.cuh: before any tensor memory is held
+    pdl_wait();
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     // two buffers of a unit's column table (output entry, factor, static
