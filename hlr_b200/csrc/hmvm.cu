@@ -67,6 +67,7 @@ struct DevNPass {
     const MSeg* mseg_cp = nullptr;    // 64-vector N-form with cp.async: the other tiles
     int nmseg_cp = 0;
     int nseg2 = 0;
+    int warps = 8;                    // of the FP64 one-vector kernel at the default setting (nform_default)
     int f16 = FMT_F16;                // the store's 16-bit format
     int wide = FMT_F32;               // the store's wide format (FP32, or 24-bit for BFP)
     const void* chunks = nullptr;     // NChunk (FP64 plan) or QNChunk (reduced precision)
@@ -96,6 +97,7 @@ struct DevTTPass {
     const TGroup* groups1 = nullptr;  // first finish level (long outputs), into the partial array
     int ngroups1 = 0;
     int64_t npart = 0;
+    int warps = 8;                    // of the FP64 one-vector kernel at the default setting
     // group T-form (products of more than 8 vectors of an FP64 store)
     const GTSeg* gsegs = nullptr;
     const GTChunk* gchunks = nullptr;
@@ -114,6 +116,24 @@ struct DevTTPass {
         return k;
     }
 };
+
+// Warps per CTA of the FP64 one-vector kernels where the handle keeps the
+// default of 8, by the chunks (8 columns) of a tile.  N-form: with more tiles
+// than two per SM and no more than four, all tiles are resident at once, and
+// 16 warps keep more loads in flight (n = 20011 to 32768 exponential, 512 tiles
+// of 100 and more chunks: 193 -> 176, 221 -> 201, 294 -> 273 us; 1024 tiles:
+// 499 -> 517; 82 chunks, uniform-H: 54 -> 59); light tiles in many waves take 4
+// (1D log, 2048 tiles of 18 chunks: 66 -> 60 us; 512 tiles: no change).  Up to
+// two tiles per SM the order of the sums stays that of 8 warps, which the
+// one-launch products share.  Tile T-form (the results do not depend on it):
+// tiles of a few chunks leave half of 8 warps idle (H^2 leaf bases, 512 tiles
+// of 3 chunks: product 74 -> 65 us).
+int nform_default(size_t tiles, size_t chunks) {
+    if (tiles <= 2 * 148) return 8;
+    if (tiles <= 4 * 148) return chunks >= 100 * tiles ? 16 : 8;
+    return tiles >= 6 * 148 && chunks <= 24 * tiles ? 4 : 8;
+}
+int ttform_default(size_t tiles, size_t chunks) { return chunks <= 4 * tiles ? 4 : 8; }
 
 // Scratch used by one product: the coefficient vectors and the partial sums
 // of a one-vector product, and (when present) the same arrays as row-major
@@ -1223,6 +1243,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         }
         if (e == cudaSuccess) e = put(o_nc[i], enc.data(), enc.size());
         d.chunks = hp->arena + o_nc[i];
+        if (f64) d.warps = nform_default(np.segs[FMT_F64].size(), np.chunks.size());
         d.vx = np.vx; d.vt = np.vt; d.out = np.out; d.mode = np.mode; d.bytes = np.bytes; d.alg_bytes = np.alg_bytes;
         if (!np.cta_begin.empty() && e == cudaSuccess) {
             if (!f64) {
@@ -1312,6 +1333,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (e == cudaSuccess) e = put(L.ttg[i], tp.groups.data(), tp.groups.size() * sizeof(TGroup));
         if (e == cudaSuccess) e = put(L.ttg1[i], tp.groups1.data(), tp.groups1.size() * sizeof(TGroup));
         d.chunks = hp->arena + L.ttc[i];
+        if (f64) d.warps = ttform_default(tp.segs[FMT_F64].size(), tp.chunks.size());
         d.groups = reinterpret_cast<const TGroup*>(hp->arena + L.ttg[i]);
         d.ngroups = int(tp.groups.size());
         d.groups1 = reinterpret_cast<const TGroup*>(hp->arena + L.ttg1[i]);
@@ -1798,8 +1820,9 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
                     }
                 }
             };
-            if (M->ttform_warps == 4) ttform(Warps<4>{});
-            else if (M->ttform_warps == 16) ttform(Warps<16>{});
+            const int tw = M->ttform_warps == 8 ? tp.warps : M->ttform_warps;
+            if (tw == 4) ttform(Warps<4>{});
+            else if (tw == 16) ttform(Warps<16>{});
             else ttform(Warps<8>{});
             if (ws.profile) prof_end(M, s);
             if (tp.ngroups > 0) {
@@ -1848,8 +1871,9 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
                                    M->store, vx, vt, vo, alpha, add));
                 }
             };
-            if (M->nform_warps == 4) nform(Warps<4>{});
-            else if (M->nform_warps == 16) nform(Warps<16>{});
+            const int nw = M->nform_warps == 8 ? np.warps : M->nform_warps;
+            if (nw == 4) nform(Warps<4>{});
+            else if (nw == 16) nform(Warps<16>{});
             else nform(Warps<8>{});
             if (ws.profile) prof_end(M, s);
             HLRC_AFTER_LAUNCH(stage_name(M, 1, st.idx));

@@ -383,7 +383,9 @@ hlrc_status hlrc_workspace_free(hlrc_workspace ws);
  * per-warp partial sums differs, so results agree to rounding).
  *   nform_warps, ttform_warps: warps per CTA (4, 8 or 16) of the one-vector
  *     N-form and tile T-form kernels (16 for small matrices, where each
- *     output tile's chain of loads sets the time);
+ *     output tile's chain of loads sets the time).  8 is the default: FP64
+ *     passes whose tiles hold few or many columns then take 4 or 16, chosen at
+ *     upload;
  *   mr_min_nrhs: products with at least this many vectors use the
  *     8-vector tensor-core kernels, smaller ones loop the one-vector kernels
  *     (2..HLRC_MR_NEVER; HLRC_MR_NEVER always loops);
