@@ -144,6 +144,7 @@ struct Workspace {
     double* t = nullptr;
     double* t2 = nullptr;
     double* part = nullptr;
+    double* part2 = nullptr;     // partial sums of a transposed near field that runs beside the chain
     unsigned* ctr = nullptr;     // counters of one-launch products (FLOW_CTRS, zero between products)
     int mr_nt = 0;               // the multi-vector arrays hold blocks of 8 * mr_nt vectors
     double* mr_x = nullptr;      // null: no multi-vector arrays
@@ -232,6 +233,12 @@ struct hlrc_hmat_s {
     std::vector<Stage> stages[3];
     std::vector<Stage> stages_mr[3];   // multi-vector products, when they differ (H^2: no tree sweeps)
     std::vector<Stage> stages_nf[3];   // one-vector products with side stages, when present
+    // op T / C: the stage of the transposed near field when its tile T-form may
+    // run on the side stream beside the other passes (near_t_stage; -1: not),
+    // and the partial sums it needs of its own
+    int near_t[3] = {-1, -1, -1};
+    double* part2 = nullptr;
+    int64_t n_part2 = 0;
     bool nf_multi = false;             // multi-vector products take stages_nf too
     Workspace side_ws;                 // the handle's side stream and events (side stages only)
     hlrc_info info{};
@@ -240,6 +247,7 @@ struct hlrc_hmat_s {
     struct Flow {
         FlowStage st[FLOW_MAXST];
         int nst = 0, side = -1, main_items = 0, side_items = 0;
+        bool near_t = false;   // the side pass is a transposed near field: needs part2
     };
     Flow flow[3];
     unsigned* ctr = nullptr;           // counters of the handle's own workspace
@@ -373,9 +381,23 @@ struct ArenaLayout {
     std::vector<size_t> tu, ts, tg, nc, ttc, ttg, ttg1, n2;
     std::vector<std::array<size_t, 7>> ntree;   // per N-pass: the tree sweep's seven arrays
     std::vector<std::array<size_t, NFMT>> ns, tts;   // per pass, per StoreFmt
-    size_t t = 0, t2 = 0, part = 0, ctr = 0, err = 0, total = 0;
-    size_t part_elems = 0;
+    size_t t = 0, t2 = 0, part = 0, part2 = 0, ctr = 0, err = 0, total = 0;
+    size_t part_elems = 0, part2_elems = 0;
 };
+
+// The stage of op's one-vector list that is the transposed near field (its
+// last, y += alpha D^T x), when its tile T-form writes partial sums only: that
+// part reads x alone and can run beside the passes before it; -1 otherwise.
+// Plans without side stages keep everything on the caller's stream.
+int near_t_stage(const Plan& p, int op) {
+    const std::vector<Stage>& l = p.stages[op];
+    if (!has_side(p.stages_nf) || !p.stages_nf[op].empty() || l.size() < 2 || l.back().kind != 2) return -1;
+    const TTPass& t = p.ttpasses[size_t(l.back().idx)];
+    if (t.in != V_X || t.out != V_Y || t.mode != OUT_ADD_ALPHA || t.chunks.empty()) return -1;
+    for (const GChunk& c : t.chunks)
+        if (c.flags & TT_DIRECT) return -1;
+    return int(l.size()) - 1;
+}
 
 ArenaLayout arena_layout(const Plan& p) {
     ArenaLayout L;
@@ -419,6 +441,10 @@ ArenaLayout arena_layout(const Plan& p) {
     L.t = take(size_t(std::max<int64_t>(1, p.n_t)) * sizeof(double));
     L.t2 = take(size_t(std::max<int64_t>(1, p.n_t2)) * sizeof(double));
     L.part = take(part_elems * sizeof(double));
+    for (int op = 0; op < 3; ++op)
+        if (const int nt = near_t_stage(p, op); nt >= 0)
+            L.part2_elems = std::max(L.part2_elems, size_t(p.ttpasses[size_t(p.stages[op][size_t(nt)].idx)].npart));
+    L.part2 = take(L.part2_elems * sizeof(double));
     L.ctr = take(FLOW_CTRS * sizeof(unsigned));
     L.err = take(sizeof(int));
     L.part_elems = part_elems;
@@ -1025,7 +1051,9 @@ hlrc_status plan_h_leaves(const hlrc_h_desc& d, hlrc_options o, Plan& p, double 
 // launches; what is saved are the host's calls (B200, one vector, eager
 // launches, separate -> one: 1D log n = 2048 20 -> 11 us, n = 8192 28 -> 14 us,
 // n = 16384 (256 tiles) 22 -> 19 us; exponential n = 13001 117 -> 113 us; but 512
-// tiles of a uniform-H matrix 55 -> 75 us, 2048 tiles 66 -> 124 us).
+// tiles of a uniform-H matrix 55 -> 75 us, 2048 tiles 66 -> 124 us).  Op T / C with
+// the tiles of D^T x in the side queue instead of in line: exponential n = 8192
+// 110 -> 71 us, n = 4096 72 -> 52 us, 1D log n = 8192 20.7 -> 17.2 us.
 constexpr int FLOW_TILES = 296;
 void plan_flow(hlrc_hmat_s* h) {
     if (h->precision != HLRC_PREC_F64) return;
@@ -1064,7 +1092,7 @@ void plan_flow(hlrc_hmat_s* h) {
             if (side) {
                 F.side = F.nst;
             } else {
-                if (out == V_Y && F.side >= 0 && !joined) {
+                if ((out == V_Y || vt == 5) && F.side >= 0 && !joined) {
                     f.join = F.side;
                     joined = true;
                 }
@@ -1072,21 +1100,25 @@ void plan_flow(hlrc_hmat_s* h) {
             }
             ++F.nst;
         };
-        for (const Stage& st : list) {
+        for (size_t i = 0; i < list.size(); ++i) {
+            const Stage& st = list[i];
             if (st.kind == 1) {
                 const DevNPass& np = h->n[size_t(st.idx)];
                 ok = ok && np.ncta == 0;
                 push(FLOW_N, np.segs[FMT_F64], np.chunks, np.nsegs[FMT_F64], st.side, np.vx, np.vt, np.out, np.mode);
             } else if (st.kind == 2) {
                 const DevTTPass& tp = h->tt[size_t(st.idx)];
-                push(FLOW_TT, tp.segs[FMT_F64], tp.chunks, tp.nsegs[FMT_F64], st.side, tp.in, tp.in, tp.out, tp.mode);
-                push(FLOW_FINISH, tp.groups1, nullptr, tp.ngroups1, st.side, tp.in, tp.in, 4, OUT_SET);
-                push(FLOW_FINISH, tp.groups, nullptr, tp.ngroups, st.side, tp.in, tp.in, tp.out, tp.mode);
+                const bool near = int(i) == h->near_t[op];   // its tiles beside the chain, its sums in place
+                const int part = near ? 5 : 4;
+                F.near_t = F.near_t || near;
+                push(FLOW_TT, tp.segs[FMT_F64], tp.chunks, tp.nsegs[FMT_F64], near, tp.in, part, tp.out, tp.mode);
+                push(FLOW_FINISH, tp.groups1, nullptr, tp.ngroups1, false, tp.in, part, part, OUT_SET);
+                push(FLOW_FINISH, tp.groups, nullptr, tp.ngroups, false, tp.in, part, tp.out, tp.mode);
             } else {
                 const DevTPass& tp = h->t[size_t(st.idx)];
                 ok = ok && tp.cls_begin[1] == tp.cls_begin[3];   // 8-column units only
-                push(FLOW_T, tp.units, tp.slabs, tp.cls_begin[3], st.side, tp.in, tp.in, tp.out, tp.mode);
-                push(FLOW_TFINISH, tp.groups, nullptr, tp.ngroups, st.side, tp.in, tp.in, tp.out, tp.mode);
+                push(FLOW_T, tp.units, tp.slabs, tp.cls_begin[3], false, tp.in, 4, tp.out, tp.mode);
+                push(FLOW_TFINISH, tp.groups, nullptr, tp.ngroups, false, tp.in, 4, tp.out, tp.mode);
             }
         }
         if (ok && F.nst > 0) h->flow[op] = F;
@@ -1362,10 +1394,13 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
     hp->part = reinterpret_cast<double*>(hp->arena + o_part);
     hp->dev_err = reinterpret_cast<int*>(hp->arena + L.err);
     hp->ctr = reinterpret_cast<unsigned*>(hp->arena + L.ctr);
+    hp->n_part2 = int64_t(L.part2_elems);
+    hp->part2 = L.part2_elems ? reinterpret_cast<double*>(hp->arena + L.part2) : nullptr;
     for (int op = 0; op < 3; ++op) {
         hp->stages[op] = p.stages[op];
         hp->stages_mr[op] = p.stages_mr[op];
         hp->stages_nf[op] = p.stages_nf[op];
+        hp->near_t[op] = near_t_stage(p, op);
     }
     hp->nf_multi = p.nf_multi;
     if (has_side(hp->stages_nf)) {
@@ -1538,6 +1573,7 @@ Workspace handle_workspace(hlrc_hmat M) {
     Workspace w;
     w.t = M->ws_t; w.t2 = M->ws_t2; w.part = M->part;
     w.ctr = M->ctr;
+    w.part2 = M->part2;
     w.mr_nt = M->mr_nt;
     w.mr_x = M->mr_x; w.mr_t = M->mr_t; w.mr_t2 = M->mr_t2; w.mr_part = M->mr_part;
     w.w_xs = M->wws.w_xs; w.w_ts = M->wws.w_ts; w.w_part = M->wws.w_part;
@@ -1721,7 +1757,7 @@ const std::vector<int>& stage_order(hlrc_hmat M, const std::vector<Stage>& stl, 
 // shapes other than the default (its CTAs have 8 warps, which gives the sums
 // of the default shapes).
 bool flow_ok(hlrc_hmat M, const Workspace& ws, int op, cudaStream_t s) {
-    return M->flow[op].nst > 0 && ws.ctr && !ws.profile && M->nform_warps == 8 && M->ttform_warps == 8 &&
+    return M->flow[op].nst > 0 && ws.ctr && (ws.part2 || !M->flow[op].near_t) && !ws.profile && M->nform_warps == 8 && M->ttform_warps == 8 &&
            !debug_sync() && !capturing(s);
 }
 hlrc_status run_flow(hlrc_hmat M, const Workspace& ws, double alpha, int op, const double* x, double* y,
@@ -1739,6 +1775,7 @@ hlrc_status run_flow(hlrc_hmat M, const Workspace& ws, double alpha, int op, con
     a.v[V_T] = ws.t;
     a.v[V_T2] = ws.t2;
     a.v[4] = ws.part;
+    a.v[5] = ws.part2;
     a.alpha = alpha;
     a.ctr = ws.ctr;
     a.err = M->dev_err;
@@ -1763,6 +1800,73 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
     auto L = [&](cudaError_t e) { if (le == cudaSuccess) le = e; };
     SideFork side{M, ws, s0};
     const std::vector<Stage>& stl = M->stages_nf[op].empty() ? M->stages[op] : M->stages_nf[op];
+    // the two halves of a tile T-form pass on stream s, partial sums in `part`
+    auto tt_form = [&](int idx, cudaStream_t s, double* part) {
+        const DevTTPass& tp = M->tt[size_t(idx)];
+        const double* vin = bind(ws, tp.in, x, y);
+        double* vout = bind(ws, tp.out, x, y);
+        const int add = tp.mode != OUT_SET;
+        const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
+        if (ws.profile) prof_begin(M, stage_name(M, 2, idx), tp.alg_bytes, s);
+        auto ttform = [&](auto wc) {
+            constexpr int TW = decltype(wc)::value;
+            if (f64plan && tp.nsegs[FMT_F64] > 0)
+                L(launch_k(ov, k_ttform_f64<TW>, unsigned(tp.nsegs[FMT_F64]), TW * 32, 0, s, tp.segs[FMT_F64],
+                           static_cast<const TTChunk*>(tp.chunks), reinterpret_cast<const double*>(M->store), vin,
+                           vout, part, alpha, add));
+            // reduced precision: each tile's run of columns, streamed in full
+            // 4 KB iterations; FP32 and 16-bit runs in one grid
+            if (!f64plan) {
+                if (tp.nmseg[FMT_I24] + tp.nmseg[FMT_I16] > 0) {   // block floating point
+                    const int n24 = tp.nmseg[FMT_I24];
+                    L(launch_k(ov, k_ttform_qs<TW, FMT_I24, FMT_I16>, unsigned(n24 + tp.nmseg[FMT_I16]), TW * 32, 0,
+                               s, tp.mseg[FMT_I24], n24, tp.mseg[FMT_I16], tp.mcol, M->store, vin, vout, part,
+                               alpha, add));
+                } else {
+                    const int n32 = tp.nmseg[FMT_F32];
+                    if (tp.nmseg[FMT_BF16] > 0)
+                        L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_BF16>, unsigned(n32 + tp.nmseg[FMT_BF16]),
+                                   TW * 32, 0, s, tp.mseg[FMT_F32], n32, tp.mseg[FMT_BF16], tp.mcol, M->store, vin,
+                                   vout, part, alpha, add));
+                    else if (n32 + tp.nmseg[FMT_F16] > 0)
+                        L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_F16>, unsigned(n32 + tp.nmseg[FMT_F16]),
+                                   TW * 32, 0, s, tp.mseg[FMT_F32], n32, tp.mseg[FMT_F16], tp.mcol, M->store, vin,
+                                   vout, part, alpha, add));
+                }
+            }
+        };
+        const int tw = M->ttform_warps == 8 ? tp.warps : M->ttform_warps;
+        if (tw == 4) ttform(Warps<4>{});
+        else if (tw == 16) ttform(Warps<16>{});
+        else ttform(Warps<8>{});
+        if (ws.profile) prof_end(M, s);
+    };
+    auto tt_finish = [&](int idx, cudaStream_t s, double* part) {
+        const DevTTPass& tp = M->tt[size_t(idx)];
+        double* vout = bind(ws, tp.out, x, y);
+        const int add = tp.mode != OUT_SET;
+        const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;
+        if (tp.ngroups > 0) {
+            if (ws.profile) prof_begin(M, "ttfinish", tp.npart * 8, s);
+            if (tp.ngroups1 > 0)   // first level: runs of slots into the scratch part of the partials
+                L(launch_k(ov, k_ttfinish_f64, unsigned((tp.ngroups1 + 7) / 8), 256, 0, s, tp.groups1, tp.ngroups1,
+                           static_cast<const double*>(part), part, 1.0, 0));
+            L(launch_k(ov, k_ttfinish_f64, unsigned((tp.ngroups + 7) / 8), 256, 0, s, tp.groups, tp.ngroups,
+                       static_cast<const double*>(part), vout, alpha, add));
+            if (ws.profile) prof_end(M, s);
+        }
+    };
+    // The transposed near field's tile T-form starts on the side stream; its
+    // finish adds to y in its place.  Same sums in the same order (B200, one
+    // vector, adjoint, in line -> beside: uniform-H sphere of 32768 triangles
+    // 87 -> 76 us, as H^2 102 -> 82 us; exponential n = 20011 FP64 208 -> 186, BFP
+    // 116 -> 107, n = 50021 FP64 530 -> 506 us; 1D log n = 50000 44.7 -> 39.0 us).
+    const int beside = ws.part2 && ws.side && !ws.profile ? M->near_t[op] : -1;
+    if (beside >= 0) {
+        L(cudaEventRecord(ws.ev_fork, s0));
+        L(cudaStreamWaitEvent(ws.side, ws.ev_fork, 0));
+        tt_form(stl[size_t(beside)].idx, ws.side, ws.part2);
+    }
     thread_local std::vector<int> order;
     for (const int oi : stage_order(M, stl, order)) {
         const Stage& st = stl[size_t(oi)];
@@ -1786,53 +1890,14 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
             if (ws.profile) prof_end(M, s);
             HLRC_AFTER_LAUNCH(stage_name(M, 0, st.idx));
         } else if (st.kind == 2) {
-            const DevTTPass& tp = M->tt[size_t(st.idx)];
-            if (tp.launches() == 0) continue;
-            const double* vin = bind(ws, tp.in, x, y);
-            double* vout = bind(ws, tp.out, x, y);
-            const int add = tp.mode != OUT_SET;
-            const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
-            if (ws.profile) prof_begin(M, stage_name(M, 2, st.idx), tp.alg_bytes, s);
-            auto ttform = [&](auto wc) {
-                constexpr int TW = decltype(wc)::value;
-                if (f64plan && tp.nsegs[FMT_F64] > 0)
-                    L(launch_k(ov, k_ttform_f64<TW>, unsigned(tp.nsegs[FMT_F64]), TW * 32, 0, s, tp.segs[FMT_F64],
-                               static_cast<const TTChunk*>(tp.chunks), reinterpret_cast<const double*>(M->store), vin,
-                               vout, ws.part, alpha, add));
-                // reduced precision: each tile's run of columns, streamed in full
-                // 4 KB iterations; FP32 and 16-bit runs in one grid
-                if (!f64plan) {
-                    if (tp.nmseg[FMT_I24] + tp.nmseg[FMT_I16] > 0) {   // block floating point
-                        const int n24 = tp.nmseg[FMT_I24];
-                        L(launch_k(ov, k_ttform_qs<TW, FMT_I24, FMT_I16>, unsigned(n24 + tp.nmseg[FMT_I16]), TW * 32, 0,
-                                   s, tp.mseg[FMT_I24], n24, tp.mseg[FMT_I16], tp.mcol, M->store, vin, vout, ws.part,
-                                   alpha, add));
-                    } else {
-                        const int n32 = tp.nmseg[FMT_F32];
-                        if (tp.nmseg[FMT_BF16] > 0)
-                            L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_BF16>, unsigned(n32 + tp.nmseg[FMT_BF16]),
-                                       TW * 32, 0, s, tp.mseg[FMT_F32], n32, tp.mseg[FMT_BF16], tp.mcol, M->store, vin,
-                                       vout, ws.part, alpha, add));
-                        else if (n32 + tp.nmseg[FMT_F16] > 0)
-                            L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_F16>, unsigned(n32 + tp.nmseg[FMT_F16]),
-                                       TW * 32, 0, s, tp.mseg[FMT_F32], n32, tp.mseg[FMT_F16], tp.mcol, M->store, vin,
-                                       vout, ws.part, alpha, add));
-                    }
-                }
-            };
-            const int tw = M->ttform_warps == 8 ? tp.warps : M->ttform_warps;
-            if (tw == 4) ttform(Warps<4>{});
-            else if (tw == 16) ttform(Warps<16>{});
-            else ttform(Warps<8>{});
-            if (ws.profile) prof_end(M, s);
-            if (tp.ngroups > 0) {
-                if (ws.profile) prof_begin(M, "ttfinish", tp.npart * 8, s);
-                if (tp.ngroups1 > 0)   // first level: runs of slots into the scratch part of the partials
-                    L(launch_k(ov, k_ttfinish_f64, unsigned((tp.ngroups1 + 7) / 8), 256, 0, s, tp.groups1, tp.ngroups1,
-                               static_cast<const double*>(ws.part), ws.part, 1.0, 0));
-                L(launch_k(ov, k_ttfinish_f64, unsigned((tp.ngroups + 7) / 8), 256, 0, s, tp.groups, tp.ngroups,
-                           static_cast<const double*>(ws.part), vout, alpha, add));
-                if (ws.profile) prof_end(M, s);
+            if (M->tt[size_t(st.idx)].launches() == 0) continue;
+            if (oi == beside) {   // its tile T-form ran on the side stream
+                L(cudaEventRecord(ws.ev_join, ws.side));
+                L(cudaStreamWaitEvent(s0, ws.ev_join, 0));
+                tt_finish(st.idx, s, ws.part2);
+            } else {
+                tt_form(st.idx, s, ws.part);
+                tt_finish(st.idx, s, ws.part);
             }
             HLRC_AFTER_LAUNCH(stage_name(M, 2, st.idx));
         } else {
@@ -2746,6 +2811,7 @@ extern "C" hlrc_status hlrc_mvm_noalloc(hlrc_hmat M, double alpha, int op, const
     ws.t = base;
     ws.t2 = base + std::max<int64_t>(1, M->n_t);
     ws.part = base + std::max<int64_t>(1, M->n_t) + std::max<int64_t>(1, M->n_t2);
+    if (need + size_t(M->n_part2) <= NOALLOC_SCRATCH_DOUBLES && M->n_part2 > 0) ws.part2 = base + need;   // else in line
     ws.ctr = ctr;
     return run_single(M, ws, alpha, op, x, y, static_cast<cudaStream_t>(stream));
 }
@@ -2762,7 +2828,7 @@ extern "C" int64_t hlrc_launch_count(hlrc_hmat M) { return M ? M->launches.load(
 // its own workspace.
 struct hlrc_workspace_s {
     int device = 0;
-    int64_t n_t = 0, n_t2 = 0, n_part = 0;   // one-vector capacities (doubles)
+    int64_t n_t = 0, n_t2 = 0, n_part = 0, n_part2 = 0;   // one-vector capacities (doubles)
     size_t mr_nx = 0, mr_nt = 0, mr_nt2 = 0, mr_np = 0;   // multi-vector capacities (0: none)
     int mr_tiles = 0;                                     // and the 8-vector tiles they were made for
     size_t w_xs = 0, w_ts = 0, w_part = 0;                // 64-vector capacities in bytes (0: none)
@@ -2786,7 +2852,7 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     size_t off = 0;
     auto take = [&](size_t elems) { const size_t o_ = off; off = align_up(off + elems * sizeof(double), 256); return o_; };
     const size_t o_t = take(size_t(W->n_t)), o_t2 = take(size_t(W->n_t2)), o_p = take(size_t(W->n_part)),
-                 o_ctr = take(FLOW_CTRS * sizeof(unsigned) / sizeof(double) + 1);
+                 o_p2 = take(size_t(M->n_part2)), o_ctr = take(FLOW_CTRS * sizeof(unsigned) / sizeof(double) + 1);
     WideSizes zw;
     size_t o_w = 0;
     if (max_nrhs > MR_RB && M->wide) {
@@ -2822,6 +2888,8 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     W->ws.t = reinterpret_cast<double*>(W->arena + o_t);
     W->ws.t2 = reinterpret_cast<double*>(W->arena + o_t2);
     W->ws.part = reinterpret_cast<double*>(W->arena + o_p);
+    if (M->n_part2 > 0) W->ws.part2 = reinterpret_cast<double*>(W->arena + o_p2);
+    W->n_part2 = M->n_part2;
     W->ws.ctr = reinterpret_cast<unsigned*>(W->arena + o_ctr);
     if (const cudaError_t me = cudaMemset(W->ws.ctr, 0, FLOW_CTRS * sizeof(unsigned)); me != cudaSuccess) {
         cudaFree(W->arena);
@@ -2868,6 +2936,7 @@ extern "C" hlrc_status hlrc_mvm_ws(hlrc_hmat M, hlrc_workspace W, double alpha, 
     if (!g.ok) return fail(HLRC_ERR_CUDA, "cannot select device %d", M->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Workspace ws = W->ws;
+    if (W->n_part2 < M->n_part2) ws.part2 = nullptr;   // made for another handle: the near field in line
     if (ws.mr_x) {   // the multi-vector arrays serve only handles they fit, in blocks that fit
         ws.mr_nt = std::min(W->mr_tiles, mr_tiles(M, DW_MAXNT * MR_RB));
         auto fits = [&](int nt) {

@@ -7,11 +7,12 @@
 // on the device: four hand-overs of about 2 us (ticket, descriptor and data
 // loads, completion count).  Here resident CTAs take work items (an output tile, an input tile, a few
 // finish groups) from two queues: the passes of the chain in order, and the
-// near field D x, which depends on nothing but x.  An item of pass s waits
+// near field D x (op T / C: the tile T-form of D^T x), which depends on nothing
+// but x.  An item of pass s waits
 // until every item of the pass before it is done; it loads its descriptors
 // and its first matrix columns before that wait.  Part of the CTAs start on
-// the near field; the pass that adds to y after it drains that queue first
-// and then waits for it.
+// the near field; the pass that adds to y after it (op T / C: its finish) drains
+// that queue first and then waits for it.
 //
 // Progress.  A queue is a counter: tickets are taken in pass order, so the
 // items an item waits for are held by CTAs that already run, whatever part of
@@ -48,7 +49,8 @@ struct FlowStage {
     int32_t first;         // first ticket of the pass in its queue
     int32_t dep;           // the pass that has to be done first (-1: none)
     int32_t join;          // the near-field pass to wait for as well (-1: none)
-    int8_t in, vt, out, add;   // VecName of inputs and output; 0 set, 1 add alpha * s, 2 add s
+    int8_t in, vt, out, add;   // VecName of inputs and output (4, 5: partial sums; vt: those of T-forms and finishes);
+                               // add: 0 set, 1 add alpha * s, 2 add s
 };
 static_assert(sizeof(FlowStage) == 48, "FlowStage is 48 bytes");
 
@@ -58,7 +60,7 @@ struct FlowArgs {
     int main_items, side_items;
     int main_ctas;                   // CTAs that start on the chain
     const double* A;
-    double* v[5];                    // by VecName; [4] the partial sums
+    double* v[6];                    // by VecName; [4] the partial sums, [5] those of a side pass
     double alpha;
     unsigned* ctr;
     int* err;
@@ -246,7 +248,7 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
                           ready);
         } else if (p.kind == FLOW_TT) {
             const TTSeg sg = static_cast<const TTSeg*>(p.items)[item];
-            flow_ttform<W>(sg, static_cast<const TTChunk*>(p.data), a.A, in, out, a.v[4], alpha, p.add != 0, ready);
+            flow_ttform<W>(sg, static_cast<const TTChunk*>(p.data), a.A, in, out, a.v[p.vt], alpha, p.add != 0, ready);
         } else {
             const int e = min(p.n, (item + 1) * p.per);
             int i = item * p.per + warp;
@@ -256,13 +258,13 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
             const bool go = ready();
             while (go && i < e) {
                 if (p.kind == FLOW_FINISH) {
-                    ttfinish_group<true>(g, a.v[4], out, alpha, p.add != 0, lane);
+                    ttfinish_group<true>(g, a.v[p.vt], out, alpha, p.add != 0, lane);
                 } else if (p.kind == FLOW_TFINISH) {
-                    tfinish_group<true>(g, a.v[4], out, alpha, p.add != 0, lane);
+                    tfinish_group<true>(g, a.v[p.vt], out, alpha, p.add != 0, lane);
                 } else {
                     TUnit u;
                     memcpy(&u, &g, sizeof(u));
-                    tform_unit<TCOLS, true>(u, static_cast<const TSlab*>(p.data), a.A, in, out, a.v[4], alpha, p.add != 0,
+                    tform_unit<TCOLS, true>(u, static_cast<const TSlab*>(p.data), a.A, in, out, a.v[p.vt], alpha, p.add != 0,
                                         lane);
                 }
                 i += W;

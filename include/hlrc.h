@@ -207,7 +207,9 @@ typedef struct hlrc_options {
      * default: 2 for one-vector products, 1 for multi-vector ones (their
      * passes are compute-heavy: nothing to overlap).  With 2, D x is added
      * first, then the low-rank part, per row tile; the 64-vector product of
-     * 16-bit stores always takes the fused pass.                          */
+     * 16-bit stores always takes the fused pass.  With 0 or 2, one-vector
+     * products of op T / C run the tiles of D^T x beside the other passes in
+     * the same way; y is summed as without.                                */
     int32_t near_field;
     int32_t reserved[3];
 } hlrc_options;
