@@ -68,6 +68,7 @@ struct DevNPass {
     int nmseg_cp = 0;
     int nseg2 = 0;
     int warps = 8;                    // of the FP64 one-vector kernel at the default setting (nform_default)
+    int split = 1;                    // CTAs per tile at the default setting (tile_split)
     int f16 = FMT_F16;                // the store's 16-bit format
     int wide = FMT_F32;               // the store's wide format (FP32, or 24-bit for BFP)
     const void* chunks = nullptr;     // NChunk (FP64 plan) or QNChunk (reduced precision)
@@ -98,6 +99,7 @@ struct DevTTPass {
     int ngroups1 = 0;
     int64_t npart = 0;
     int warps = 8;                    // of the FP64 one-vector kernel at the default setting
+    int split = 1;                    // CTAs per tile at the default setting (tile_split)
     // group T-form (products of more than 8 vectors of an FP64 store)
     const GTSeg* gsegs = nullptr;
     const GTChunk* gchunks = nullptr;
@@ -116,6 +118,22 @@ struct DevTTPass {
         return k;
     }
 };
+
+// CTAs per tile of the one-vector kernels at the default of 8 warps: a power of
+// two that keeps all CTAs resident (four per SM) and leaves each 64 KB, two
+// chunks a warp.  With fewer tiles than that a tile's chain of loads sets the time
+// and SMs idle: n = 4096 exponential (64 tiles of about 0.5 MB) 45 -> 23 us, n = 8192
+// (128 tiles) 80 -> 53, adjoint 71 -> 57; mixed store 47 -> 34, BFP 41 -> 33 us.
+// Measured beside it: 32 KB (mixed n = 8192 34 -> 37 us), 8 CTAs per tile (no change),
+// two CTAs for 297 to 592 tiles (uniform-H sphere of 512 tiles 53 -> 57 us).
+constexpr size_t SPLIT_CTAS = 4 * 148;
+constexpr int64_t SPLIT_BYTES = 64 << 10;
+constexpr int SPLIT_MAX = 4;
+int tile_split(size_t tiles, int64_t bytes) {
+    int s = 1;
+    while (2 * s <= SPLIT_MAX && 2 * s * tiles <= SPLIT_CTAS && bytes >= int64_t(2 * s * tiles) * SPLIT_BYTES) s *= 2;
+    return s;
+}
 
 // Warps per CTA of the FP64 one-vector kernels where the handle keeps the
 // default of 8, by the chunks (8 columns) of a tile.  N-form: with more tiles
@@ -1050,11 +1068,16 @@ hlrc_status plan_h_leaves(const hlrc_h_desc& d, hlrc_options o, Plan& p, double 
 // a hand-over between passes costs about 2 us on the device, as between
 // launches; what is saved are the host's calls (B200, one vector, eager
 // launches, separate -> one: 1D log n = 2048 20 -> 11 us, n = 8192 28 -> 14 us,
-// n = 16384 (256 tiles) 22 -> 19 us; exponential n = 13001 117 -> 113 us; but 512
-// tiles of a uniform-H matrix 55 -> 75 us, 2048 tiles 66 -> 124 us).  Op T / C with
-// the tiles of D^T x in the side queue instead of in line: exponential n = 8192
-// 110 -> 71 us, n = 4096 72 -> 52 us, 1D log n = 8192 20.7 -> 17.2 us.
+// n = 16384 (256 tiles) 22 -> 19 us; but 512 tiles of a uniform-H matrix
+// 55 -> 75 us, 2048 tiles 66 -> 124 us).  Op T / C with the tiles of D^T x in the
+// side queue instead of in line: 1D log n = 8192 20.7 -> 17.2 us, uniform-H sphere of
+// 8192 triangles 44 -> 37 us.  Nor do products whose chain holds much in tiles worth
+// several CTAs (tile_split): n = 4096 exponential (62 MB of it) 45 us as one launch,
+// 23 us so split; where only the near field or little of the chain does, one launch
+// wins (sphere of 2048 triangles, 15 MB in all: 16 against 24 us), and its sums are
+// those of whole tiles in separate launches too.
 constexpr int FLOW_TILES = 296;
+constexpr int64_t FLOW_SPLIT_BYTES = 16 << 20;
 void plan_flow(hlrc_hmat_s* h) {
     if (h->precision != HLRC_PREC_F64) return;
     for (int op = 0; op < 3; ++op) {
@@ -1063,6 +1086,7 @@ void plan_flow(hlrc_hmat_s* h) {
         bool ok = !list.empty();
         int prev = -1;
         bool joined = false;
+        int64_t split_bytes = 0;   // of the chain, in passes with several CTAs per tile
         auto push = [&](int kind, const void* items, const void* data, int n, bool side, int in, int vt, int out, int mode) {
             if (n <= 0) return;
             if (F.nst == FLOW_MAXST || (side && F.side >= 0)) ok = false;
@@ -1105,12 +1129,14 @@ void plan_flow(hlrc_hmat_s* h) {
             if (st.kind == 1) {
                 const DevNPass& np = h->n[size_t(st.idx)];
                 ok = ok && np.ncta == 0;
+                if (!st.side && np.split > 1) split_bytes += np.bytes;
                 push(FLOW_N, np.segs[FMT_F64], np.chunks, np.nsegs[FMT_F64], st.side, np.vx, np.vt, np.out, np.mode);
             } else if (st.kind == 2) {
                 const DevTTPass& tp = h->tt[size_t(st.idx)];
                 const bool near = int(i) == h->near_t[op];   // its tiles beside the chain, its sums in place
                 const int part = near ? 5 : 4;
                 F.near_t = F.near_t || near;
+                if (!near && tp.split > 1) split_bytes += tp.bytes;
                 push(FLOW_TT, tp.segs[FMT_F64], tp.chunks, tp.nsegs[FMT_F64], near, tp.in, part, tp.out, tp.mode);
                 push(FLOW_FINISH, tp.groups1, nullptr, tp.ngroups1, false, tp.in, part, part, OUT_SET);
                 push(FLOW_FINISH, tp.groups, nullptr, tp.ngroups, false, tp.in, part, tp.out, tp.mode);
@@ -1121,7 +1147,10 @@ void plan_flow(hlrc_hmat_s* h) {
                 push(FLOW_TFINISH, tp.groups, nullptr, tp.ngroups, false, tp.in, 4, tp.out, tp.mode);
             }
         }
-        if (ok && F.nst > 0) h->flow[op] = F;
+        if (!ok || F.nst == 0 || split_bytes > FLOW_SPLIT_BYTES) continue;
+        h->flow[op] = F;
+        for (const Stage& st : list)   // the same sums in separate launches
+            if (st.kind == 1) h->n[size_t(st.idx)].split = 1;
     }
 }
 
@@ -1276,6 +1305,9 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (e == cudaSuccess) e = put(o_nc[i], enc.data(), enc.size());
         d.chunks = hp->arena + o_nc[i];
         if (f64) d.warps = nform_default(np.segs[FMT_F64].size(), np.chunks.size());
+        size_t tiles = 0;   // a tile has one CTA for all formats
+        for (int f = 0; f < NFMT; ++f) tiles = std::max(tiles, np.segs[f].size());
+        if (np.cta_begin.empty()) d.split = tile_split(tiles, np.bytes);
         d.vx = np.vx; d.vt = np.vt; d.out = np.out; d.mode = np.mode; d.bytes = np.bytes; d.alg_bytes = np.alg_bytes;
         if (!np.cta_begin.empty() && e == cudaSuccess) {
             if (!f64) {
@@ -1366,6 +1398,9 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (e == cudaSuccess) e = put(L.ttg1[i], tp.groups1.data(), tp.groups1.size() * sizeof(TGroup));
         d.chunks = hp->arena + L.ttc[i];
         if (f64) d.warps = ttform_default(tp.segs[FMT_F64].size(), tp.chunks.size());
+        size_t tiles = 0;   // a CTA for each format of a tile
+        for (int f = 0; f < NFMT; ++f) tiles += tp.segs[f].size();
+        d.split = tile_split(tiles, tp.bytes);
         d.groups = reinterpret_cast<const TGroup*>(hp->arena + L.ttg[i]);
         d.ngroups = int(tp.groups.size());
         d.groups1 = reinterpret_cast<const TGroup*>(hp->arena + L.ttg1[i]);
@@ -1666,21 +1701,36 @@ bool capturing(cudaStream_t s) {
 // Launches k on stream s.  With `overlap` the launch carries the
 // programmatic-stream-serialization attribute: the kernel may be scheduled
 // while the preceding kernel of the stream still runs, and waits for it
-// inside (pdl_wait) before it touches the vectors.
+// inside (pdl_wait) before it touches the vectors.  cluster: CTAs of the grid's x
+// direction per cluster.
 template <typename... P, typename... A>
-cudaError_t launch_k(bool overlap, void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
+cudaError_t launch_c(bool overlap, int cluster, void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
                      A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    if (overlap) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = unsigned(cluster);
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = overlap ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, k, args...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_k(bool overlap, void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
+                     A... args) {
+    return launch_c(overlap, 1, k, grid, block, smem, s, args...);
 }
 
 // Side stages (the near field) run on the workspace's side stream, forked
@@ -1808,10 +1858,11 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
         const int add = tp.mode != OUT_SET;
         const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
         if (ws.profile) prof_begin(M, stage_name(M, 2, idx), tp.alg_bytes, s);
+        const unsigned ts = M->ttform_warps == 8 ? unsigned(tp.split) : 1u;   // CTAs per tile
         auto ttform = [&](auto wc) {
             constexpr int TW = decltype(wc)::value;
             if (f64plan && tp.nsegs[FMT_F64] > 0)
-                L(launch_k(ov, k_ttform_f64<TW>, unsigned(tp.nsegs[FMT_F64]), TW * 32, 0, s, tp.segs[FMT_F64],
+                L(launch_k(ov, k_ttform_f64<TW>, dim3(unsigned(tp.nsegs[FMT_F64]), ts), TW * 32, 0, s, tp.segs[FMT_F64],
                            static_cast<const TTChunk*>(tp.chunks), reinterpret_cast<const double*>(M->store), vin,
                            vout, part, alpha, add));
             // reduced precision: each tile's run of columns, streamed in full
@@ -1819,17 +1870,17 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
             if (!f64plan) {
                 if (tp.nmseg[FMT_I24] + tp.nmseg[FMT_I16] > 0) {   // block floating point
                     const int n24 = tp.nmseg[FMT_I24];
-                    L(launch_k(ov, k_ttform_qs<TW, FMT_I24, FMT_I16>, unsigned(n24 + tp.nmseg[FMT_I16]), TW * 32, 0,
+                    L(launch_k(ov, k_ttform_qs<TW, FMT_I24, FMT_I16>, dim3(unsigned(n24 + tp.nmseg[FMT_I16]), ts), TW * 32, 0,
                                s, tp.mseg[FMT_I24], n24, tp.mseg[FMT_I16], tp.mcol, M->store, vin, vout, part,
                                alpha, add));
                 } else {
                     const int n32 = tp.nmseg[FMT_F32];
                     if (tp.nmseg[FMT_BF16] > 0)
-                        L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_BF16>, unsigned(n32 + tp.nmseg[FMT_BF16]),
+                        L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_BF16>, dim3(unsigned(n32 + tp.nmseg[FMT_BF16]), ts),
                                    TW * 32, 0, s, tp.mseg[FMT_F32], n32, tp.mseg[FMT_BF16], tp.mcol, M->store, vin,
                                    vout, part, alpha, add));
                     else if (n32 + tp.nmseg[FMT_F16] > 0)
-                        L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_F16>, unsigned(n32 + tp.nmseg[FMT_F16]),
+                        L(launch_k(ov, k_ttform_qs<TW, FMT_F32, FMT_F16>, dim3(unsigned(n32 + tp.nmseg[FMT_F16]), ts),
                                    TW * 32, 0, s, tp.mseg[FMT_F32], n32, tp.mseg[FMT_F16], tp.mcol, M->store, vin,
                                    vout, part, alpha, add));
                 }
@@ -1909,8 +1960,8 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
             double* vo = bind(ws, np.out, x, y);
             const int add = np.mode != OUT_SET;
             const double alpha = np.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
-            auto nform = [&](auto wc) {
-                constexpr int NW = decltype(wc)::value;
+            auto nform = [&](auto wc, auto sc) {
+                constexpr int NW = decltype(wc)::value, S = decltype(sc)::value;
                 if (np.ncta > 0) {   // tree sweep (FP64 plans only)
                     L(launch_k(ov, k_ntree_f64<TREE_WARPS>, unsigned(np.ncta), TREE_WARPS * 32, np.tree_smem, s,
                                np.segs[FMT_F64], static_cast<const NChunk*>(np.chunks), np.tree,
@@ -1919,27 +1970,30 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
                     return;
                 }
                 if (f64plan && np.nsegs[FMT_F64] > 0)
-                    L(launch_k(ov, k_nform_f64<NW>, unsigned(np.nsegs[FMT_F64]), NW * 32, 0, s, np.segs[FMT_F64],
+                    L(launch_c(ov, S, k_nform_f64<NW, S>, unsigned(np.nsegs[FMT_F64]) * S, NW * 32, 0, s, np.segs[FMT_F64],
                                static_cast<const NChunk*>(np.chunks), reinterpret_cast<const double*>(M->store), vx, vt,
                                vo, alpha, add));
                 // reduced precision: one CTA per tile takes the packs of both formats
                 const QNPack* qc = static_cast<const QNPack*>(np.chunks);
                 if (!f64plan && np.nseg2 > 0) {
                     if (np.wide == FMT_I24)
-                        L(launch_k(ov, k_nform_q<NW, FMT_I24, FMT_I16>, unsigned(np.nseg2), NW * 32, 0, s, np.seg2, qc,
+                        L(launch_c(ov, S, k_nform_q<NW, FMT_I24, FMT_I16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
                                    M->store, vx, vt, vo, alpha, add));
                     else if (np.f16 == FMT_BF16)
-                        L(launch_k(ov, k_nform_q<NW, FMT_F32, FMT_BF16>, unsigned(np.nseg2), NW * 32, 0, s, np.seg2, qc,
+                        L(launch_c(ov, S, k_nform_q<NW, FMT_F32, FMT_BF16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
                                    M->store, vx, vt, vo, alpha, add));
                     else
-                        L(launch_k(ov, k_nform_q<NW, FMT_F32, FMT_F16>, unsigned(np.nseg2), NW * 32, 0, s, np.seg2, qc,
+                        L(launch_c(ov, S, k_nform_q<NW, FMT_F32, FMT_F16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
                                    M->store, vx, vt, vo, alpha, add));
                 }
             };
             const int nw = M->nform_warps == 8 ? np.warps : M->nform_warps;
-            if (nw == 4) nform(Warps<4>{});
-            else if (nw == 16) nform(Warps<16>{});
-            else nform(Warps<8>{});
+            const int ns = M->nform_warps == 8 ? np.split : 1;
+            if (ns == 4) nform(Warps<8>{}, Warps<4>{});
+            else if (ns == 2) nform(Warps<8>{}, Warps<2>{});
+            else if (nw == 4) nform(Warps<4>{}, Warps<1>{});
+            else if (nw == 16) nform(Warps<16>{}, Warps<1>{});
+            else nform(Warps<8>{}, Warps<1>{});
             if (ws.profile) prof_end(M, s);
             HLRC_AFTER_LAUNCH(stage_name(M, 1, st.idx));
         }

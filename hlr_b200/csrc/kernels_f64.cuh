@@ -64,22 +64,51 @@ __device__ __forceinline__ double ld_vec(const double* p) {
     else return __ldg(p);
 }
 
-// N-form: one CTA (W warps) per output tile; chunk c goes to warp c % W;
-// lane l owns rows 2l, 2l+1; warps are summed in index order.
-template <int W>
+// The end of an N-form tile: the sum of the W warps' rows in warp order, of the S
+// CTAs of a cluster in rank order through distributed shared memory.
+template <int W, int S>
+__device__ __forceinline__ void nform_finish(double (&red)[W][TILE], int rows, double* out, double alpha, int add) {
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x < rows) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) s += red[w][threadIdx.x];
+    }
+    if constexpr (S > 1) {
+        cg::cluster_group cl = cg::this_cluster();
+        const int rank = int(blockIdx.x) % S;
+        if (threadIdx.x < rows && rank > 0) red[0][threadIdx.x] = s;   // read above by this thread only
+        cl.sync();
+        if (threadIdx.x < rows && rank == 0) {
+#pragma unroll
+            for (int r = 1; r < S; ++r) s += *cl.map_shared_rank(&red[0][threadIdx.x], r);
+        }
+        cl.sync();   // rank 0 has read the others' rows
+        if (rank > 0) return;
+    }
+    if (threadIdx.x < rows) {
+        double* o = out + threadIdx.x;
+        if (add) *o += alpha * s;
+        else *o = s;
+    }
+}
+
+// N-form: one CTA (W warps), or a cluster of S CTAs, per output tile; chunk c
+// goes to warp c % (S W); lane l owns rows 2l, 2l+1.
+template <int W, int S = 1>
 __global__ void __launch_bounds__(W * 32)
 k_nform_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
             const double* __restrict__ vx, const double* __restrict__ vt, double* __restrict__ out, double alpha,
             int add) {
     __shared__ double red[W][TILE];
     pdl_trigger();
-    const NSeg sg = segs[blockIdx.x];
+    const NSeg sg = segs[blockIdx.x / S];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = 2 * lane;
     const bool active = r < sg.ld;
     double acc0 = 0.0, acc1 = 0.0;
     pdl_wait();
-    for (uint32_t c = sg.cb + warp; c < sg.ce; c += W) {
+    for (uint32_t c = sg.cb + (blockIdx.x % S) * W + warp; c < sg.ce; c += S * W) {
         const NChunk ch = chunks[c];
         const double* v = (ch.v_off & VEC_T) ? vt + (ch.v_off & ~VEC_T) : vx + ch.v_off;
         if (active) {
@@ -105,15 +134,7 @@ k_nform_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, co
     }
     red[warp][r] = acc0;
     red[warp][r + 1] = acc1;
-    __syncthreads();
-    if (threadIdx.x < sg.rows) {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) s += red[w][threadIdx.x];
-        double* o = out + sg.out + threadIdx.x;
-        if (add) *o += alpha * s;
-        else *o = s;
-    }
+    nform_finish<W, S>(red, sg.rows, out + sg.out, alpha, add);
 }
 
 // Tree entries of a sweep pass (device copies of the planner's arrays) and
@@ -408,9 +429,10 @@ k_tform_f64(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict
     tform_unit<NC, false>(u, slabs, A, vin, out, part, alpha, add, threadIdx.x & 31);
 }
 
-// Tile T-form: one CTA (W warps) per input tile; x restricted to the tile
+// Tile T-form: gridDim.y CTAs (W warps) per input tile; x restricted to the tile
 // stays in registers (lane l holds rows 2l, 2l+1); chunk c goes to warp
-// c % W and is reduced on its own (8 columns -> one transpose-reduction).
+// c % (W gridDim.y) and is reduced on its own (8 columns -> one
+// transpose-reduction).
 template <int W>
 __global__ void __launch_bounds__(W * 32)
 k_ttform_f64(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks, const double* __restrict__ A,
@@ -424,12 +446,13 @@ k_ttform_f64(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks,
     pdl_wait();
     const double v0 = (r < sg.rows) ? __ldg(vin + sg.v_off + r) : 0.0;
     const double v1 = (r + 1 < sg.rows) ? __ldg(vin + sg.v_off + r + 1) : 0.0;
-    // software pipeline: the loads of chunk c + W are issued before chunk c
+    // software pipeline: the loads of chunk c + step are issued before chunk c
     // is reduced and written; descriptors are fetched two iterations ahead
-    uint32_t c = sg.cb + warp;
+    const uint32_t step = W * gridDim.y;
+    uint32_t c = sg.cb + W * blockIdx.y + warp;
     if (c >= sg.ce) return;
     TTChunk cur = chunks[c], nxt{0, 0, 0, 0};
-    if (c + W < sg.ce) nxt = chunks[c + W];
+    if (c + step < sg.ce) nxt = chunks[c + step];
     double2 m[TCOLS];
     auto issue = [&](const TTChunk& q) {
         const double* a = A + q.a_off + r;
@@ -438,15 +461,15 @@ k_ttform_f64(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks,
             m[j] = (active && j < q.nc) ? ld_stream(a + size_t(j) * sg.ld) : make_double2(0.0, 0.0);
     };
     issue(cur);
-    for (; c < sg.ce; c += W) {
+    for (; c < sg.ce; c += step) {
         double p[TCOLS];
 #pragma unroll
         for (int j = 0; j < TCOLS; ++j) p[j] = fma(m[j].y, v1, m[j].x * v0);
         const TTChunk ch = cur;
-        if (c + W < sg.ce) {
+        if (c + step < sg.ce) {
             cur = nxt;
             issue(cur);
-            if (c + 2 * W < sg.ce) nxt = chunks[c + 2 * W];
+            if (c + 2 * step < sg.ce) nxt = chunks[c + 2 * step];
         }
         TransposeReduce<TCOLS, 16>::run(p, lane);
         constexpr int SH = 5 - Log2<TCOLS>::v;

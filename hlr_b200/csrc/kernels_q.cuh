@@ -254,19 +254,20 @@ __device__ __forceinline__ void npacks_q(uint32_t cb, uint32_t ce, int ld, const
     }
 }
 
-// N-form of a reduced-precision store: a CTA takes one output tile, both its
+// N-form of a reduced-precision store: a CTA, or a cluster of S, takes one output tile, both its
 // packs of the wide format WIDE (FP32, or 24-bit for block floating point)
 // and its packs of the 16-bit format F16 (either may be empty), sums them in
 // FP64 and updates y once.
-template <int W, int WIDE, int F16>
+template <int W, int WIDE, int F16, int S = 1>
 __global__ void __launch_bounds__(W * 32, W >= 16 ? 1 : 3)
 k_nform_q(const NSeg2* __restrict__ segs, const QNPack* __restrict__ packs, const uint8_t* __restrict__ A,
           const double* __restrict__ vx, const double* __restrict__ vt, double* __restrict__ out, double alpha,
           int add) {
     __shared__ double red[W][TILE];
     pdl_trigger();
-    const NSeg2 sg = segs[blockIdx.x];
+    const NSeg2 sg = segs[blockIdx.x / S];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slot = int(blockIdx.x % S) * W + warp;
     pdl_wait();
     if constexpr (WIDE == FMT_I24) {
         // the wide packs flushed before the 16-bit ones start: fewer live
@@ -275,13 +276,13 @@ k_nform_q(const NSeg2* __restrict__ segs, const QNPack* __restrict__ packs, cons
             double a32[QFmt<WIDE>::R];
 #pragma unroll
             for (int r = 0; r < QFmt<WIDE>::R; ++r) a32[r] = 0.0;
-            npacks_q<W, WIDE>(sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, warp, lane, a32);
+            npacks_q<S * W, WIDE>(sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, slot, lane, a32);
             nflush_q<WIDE>(a32, lane, red[warp]);
         }
         double a16[QFmt<F16>::R];
 #pragma unroll
         for (int r = 0; r < QFmt<F16>::R; ++r) a16[r] = 0.0;
-        npacks_q<W, F16>(sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, warp, lane, a16);
+        npacks_q<S * W, F16>(sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, slot, lane, a16);
         __syncwarp();
         nflush_add_q<F16>(a16, lane, red[warp]);
     } else {
@@ -290,21 +291,13 @@ k_nform_q(const NSeg2* __restrict__ segs, const QNPack* __restrict__ packs, cons
         for (int r = 0; r < QFmt<WIDE>::R; ++r) a32[r] = 0.0;
 #pragma unroll
         for (int r = 0; r < QFmt<F16>::R; ++r) a16[r] = 0.0;
-        npacks_q<W, WIDE>(sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, warp, lane, a32);
-        npacks_q<W, F16>(sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, warp, lane, a16);
+        npacks_q<S * W, WIDE>(sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, slot, lane, a32);
+        npacks_q<S * W, F16>(sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, slot, lane, a16);
         nflush_q<WIDE>(a32, lane, red[warp]);
         __syncwarp();
         nflush_add_q<F16>(a16, lane, red[warp]);
     }
-    __syncthreads();
-    if (threadIdx.x < sg.rows) {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) s += red[w][threadIdx.x];
-        double* o = out + sg.out + threadIdx.x;
-        if (add) *o += alpha * s;
-        else *o = s;
-    }
+    nform_finish<W, S>(red, sg.rows, out + sg.out, alpha, add);
 }
 
 // -------------------------------------------------------------- tile T-form
@@ -392,19 +385,20 @@ __device__ __forceinline__ void ttform_qs(const MSeg& sg, const MCol* __restrict
                            : make_uint2(0u, 0u);
         }
     };
-    int c0 = warp * BC;
+    const int step = W * BC * int(gridDim.y);
+    int c0 = (W * int(blockIdx.y) + warp) * BC;
     if (c0 >= ncols) return;
     uint4 m[8];
     load(c0, m);
     MCol mc = (writer && c0 + jown < ncols) ? ld_mcol(ctab + c0 + jown) : MCol{0u, 0.f};
-    for (; c0 < ncols; c0 += W * BC) {
+    for (; c0 < ncols; c0 += step) {
         float p[8];
         ttdots_q<FMT>(m, ml, xr, p);
         const MCol done = mc;
         const int cd = c0;
-        if (c0 + W * BC < ncols) {
-            load(c0 + W * BC, m);
-            mc = (writer && c0 + W * BC + jown < ncols) ? ld_mcol(ctab + c0 + W * BC + jown) : MCol{0u, 0.f};
+        if (c0 + step < ncols) {
+            load(c0 + step, m);
+            mc = (writer && c0 + step + jown < ncols) ? ld_mcol(ctab + c0 + step + jown) : MCol{0u, 0.f};
         }
         TransposeReduce<8, F::G / 2, float>::run(p, lane);
         if (writer && cd + jown < ncols) {
@@ -420,7 +414,7 @@ __device__ __forceinline__ void ttform_qs(const MSeg& sg, const MCol* __restrict
     }
 }
 
-// All stream segments of one tile T-form pass in one grid: the first n32
+// All stream segments of one tile T-form pass in one grid, gridDim.y CTAs each: the first n32
 // CTAs take the runs of the wide format WIDE (FP32, or 24-bit for block
 // floating point), the others the runs of the 16-bit format F16.
 // The outputs of the two formats are disjoint, so their CTAs may run side

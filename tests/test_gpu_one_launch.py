@@ -52,7 +52,8 @@ def test_one_launch_matches_separate_passes(name, near_field):
             for alpha in (0.5, -1.75, 3.0):        # a chain of products on one workspace
                 hlr.mul_vec(alpha, op, M, x, y)
             torch.cuda.synchronize()
-            assert separate or M.launch_count() - n0 == 3
+            # heavy tiles keep separate launches, several CTAs a tile
+            assert separate or name == "h_exp" or M.launch_count() - n0 == 3
             M.last_profile()
             ys.append(y.cpu().numpy() - y0)
         M.set_profiling(False)
