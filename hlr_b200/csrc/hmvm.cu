@@ -69,6 +69,7 @@ struct DevNPass {
     int nseg2 = 0;
     int warps = 8;                    // of the FP64 one-vector kernel at the default setting (nform_default)
     int split = 1;                    // CTAs per tile at the default setting (tile_split)
+    int msplit = 1;                   // the same of the 8- to 32-vector kernels
     int f16 = FMT_F16;                // the store's 16-bit format
     int wide = FMT_F32;               // the store's wide format (FP32, or 24-bit for BFP)
     const void* chunks = nullptr;     // NChunk (FP64 plan) or QNChunk (reduced precision)
@@ -100,6 +101,7 @@ struct DevTTPass {
     int64_t npart = 0;
     int warps = 8;                    // of the FP64 one-vector kernel at the default setting
     int split = 1;                    // CTAs per tile at the default setting (tile_split)
+    int msplit = 1;                   // the same of the 8- to 32-vector kernels
     // group T-form (products of more than 8 vectors of an FP64 store)
     const GTSeg* gsegs = nullptr;
     const GTChunk* gchunks = nullptr;
@@ -129,9 +131,17 @@ struct DevTTPass {
 constexpr size_t SPLIT_CTAS = 4 * 148;
 constexpr int64_t SPLIT_BYTES = 64 << 10;
 constexpr int SPLIT_MAX = 4;
-int tile_split(size_t tiles, int64_t bytes) {
+// The same of the 8- to 32-vector kernels; FP64 passes, whose CTAs add more rows at
+// the end, are split down to 128 KB (uniform-H sphere of 8192 triangles, 128 tiles, 32
+// vectors: whole 77 us, 64 KB 90 us, 128 KB 68 us), the others to 64 KB (n = 8192 FP16
+// adjoint, 8 vectors: 92, 71, 99 us).  n = 8192 exponential FP64, 8 / 16 / 32 vectors:
+// 116 / 192 / 223 -> 76 / 110 / 160 us; mixed and BFP, 8 vectors: 96 -> 78, 141 -> 104 us;
+// n = 13001 (256 tiles), 24 vectors: 350 -> 224 us.  Half as many CTAs leave the last at
+// 349 us, twice as many make 512 tiles slower (uniform-H sphere, 32 vectors: 168 -> 215).
+int64_t msplit_bytes(bool f64) { return f64 ? 2 * SPLIT_BYTES : SPLIT_BYTES; }
+int tile_split(size_t tiles, int64_t bytes, int64_t least) {
     int s = 1;
-    while (2 * s <= SPLIT_MAX && 2 * s * tiles <= SPLIT_CTAS && bytes >= int64_t(2 * s * tiles) * SPLIT_BYTES) s *= 2;
+    while (2 * s <= SPLIT_MAX && 2 * s * tiles <= SPLIT_CTAS && bytes >= int64_t(2 * s * tiles) * least) s *= 2;
     return s;
 }
 
@@ -807,14 +817,18 @@ hlrc_status enable_tc_smem(int dev) {
                                    tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT)));
     HLRC_CUDA(cudaFuncSetAttribute(k_ttform_mr<FMT_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT)));
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_tc<FMT_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16)));
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_tc<FMT_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16)));
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_d32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32)));
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_bfp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bq_smem_n(true)));
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_bfp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bq_smem_n(false)));
+    const int n16 = tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), n32 = tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32);
+    auto smem = [](auto k, int bytes) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+    HLRC_CUDA(smem(k_nform_tc<FMT_F16, false>, n16));
+    HLRC_CUDA(smem(k_nform_tc<FMT_F16, true>, n16));
+    HLRC_CUDA(smem(k_nform_tc<FMT_BF16, false>, n16));
+    HLRC_CUDA(smem(k_nform_tc<FMT_BF16, true>, n16));
+    HLRC_CUDA(smem(k_nform_d32<false>, n32));
+    HLRC_CUDA(smem(k_nform_d32<true>, n32));
+    HLRC_CUDA(smem(k_nform_bfp<true, false>, bq_smem_n(true)));
+    HLRC_CUDA(smem(k_nform_bfp<true, true>, bq_smem_n(true)));
+    HLRC_CUDA(smem(k_nform_bfp<false, false>, bq_smem_n(false)));
+    HLRC_CUDA(smem(k_nform_bfp<false, true>, bq_smem_n(false)));
     HLRC_CUDA(cudaFuncSetAttribute(k_ttform_bfp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bq_smem_t(true)));
     HLRC_CUDA(cudaFuncSetAttribute(k_ttform_bfp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bq_smem_t(false)));
     done.push_back(dev);
@@ -1205,9 +1219,12 @@ hlrc_status enable_dw_smem(int dev) {
     static std::vector<int> done;
     std::lock_guard<std::mutex> lock(mu);
     if (std::find(done.begin(), done.end(), dev) != done.end()) return HLRC_OK;
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<2>()));
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<3>()));
-    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<4>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<2>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<2>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<3>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<3>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<4>()));
+    HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<4>()));
     HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<2>()));
     HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<3>()));
     HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<4>()));
@@ -1307,7 +1324,8 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (f64) d.warps = nform_default(np.segs[FMT_F64].size(), np.chunks.size());
         size_t tiles = 0;   // a tile has one CTA for all formats
         for (int f = 0; f < NFMT; ++f) tiles = std::max(tiles, np.segs[f].size());
-        if (np.cta_begin.empty()) d.split = tile_split(tiles, np.bytes);
+        if (np.cta_begin.empty()) d.split = tile_split(tiles, np.bytes, SPLIT_BYTES);
+        d.msplit = tile_split(tiles, np.bytes, msplit_bytes(f64));
         d.vx = np.vx; d.vt = np.vt; d.out = np.out; d.mode = np.mode; d.bytes = np.bytes; d.alg_bytes = np.alg_bytes;
         if (!np.cta_begin.empty() && e == cudaSuccess) {
             if (!f64) {
@@ -1400,7 +1418,8 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (f64) d.warps = ttform_default(tp.segs[FMT_F64].size(), tp.chunks.size());
         size_t tiles = 0;   // a CTA for each format of a tile
         for (int f = 0; f < NFMT; ++f) tiles += tp.segs[f].size();
-        d.split = tile_split(tiles, tp.bytes);
+        d.split = tile_split(tiles, tp.bytes, SPLIT_BYTES);
+        d.msplit = tile_split(tiles, tp.bytes, msplit_bytes(f64));
         d.groups = reinterpret_cast<const TGroup*>(hp->arena + L.ttg[i]);
         d.ngroups = int(tp.groups.size());
         d.groups1 = reinterpret_cast<const TGroup*>(hp->arena + L.ttg1[i]);
@@ -1701,10 +1720,10 @@ bool capturing(cudaStream_t s) {
 // Launches k on stream s.  With `overlap` the launch carries the
 // programmatic-stream-serialization attribute: the kernel may be scheduled
 // while the preceding kernel of the stream still runs, and waits for it
-// inside (pdl_wait) before it touches the vectors.  cluster: CTAs of the grid's x
-// direction per cluster.
+// inside (pdl_wait) before it touches the vectors.  cluster: CTAs of the grid
+// per cluster.
 template <typename... P, typename... A>
-cudaError_t launch_c(bool overlap, int cluster, void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
+cudaError_t launch_c(bool overlap, dim3 cluster, void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
                      A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -1717,10 +1736,11 @@ cudaError_t launch_c(bool overlap, int cluster, void (*k)(P...), dim3 grid, unsi
         at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[n++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (cluster > 1) {
+    if (cluster.x * cluster.y > 1) {
         at[n].id = cudaLaunchAttributeClusterDimension;
-        at[n].val.clusterDim.x = unsigned(cluster);
-        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        at[n].val.clusterDim.x = cluster.x;
+        at[n].val.clusterDim.y = cluster.y;
+        at[n].val.clusterDim.z = 1;
         ++n;
     }
     cfg.attrs = at;
@@ -1730,7 +1750,16 @@ cudaError_t launch_c(bool overlap, int cluster, void (*k)(P...), dim3 grid, unsi
 template <typename... P, typename... A>
 cudaError_t launch_k(bool overlap, void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
                      A... args) {
-    return launch_c(overlap, 1, k, grid, block, smem, s, args...);
+    return launch_c(overlap, dim3(1), k, grid, block, smem, s, args...);
+}
+
+// N-form of several vectors: n whole tiles on `one`, or a cluster of `split` CTAs
+// per tile on `many`.
+template <typename... P, typename... A>
+cudaError_t launch_n(bool overlap, void (*one)(P...), void (*many)(P...), int n, int split, unsigned block, size_t smem,
+                     cudaStream_t s, A... args) {
+    if (split == 1) return launch_c(overlap, dim3(1), one, dim3(unsigned(n)), block, smem, s, args...);
+    return launch_c(overlap, dim3(1, unsigned(split)), many, dim3(unsigned(n), unsigned(split)), block, smem, s, args...);
 }
 
 // Side stages (the near field) run on the workspace's side stream, forked
@@ -1970,20 +1999,20 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
                     return;
                 }
                 if (f64plan && np.nsegs[FMT_F64] > 0)
-                    L(launch_c(ov, S, k_nform_f64<NW, S>, unsigned(np.nsegs[FMT_F64]) * S, NW * 32, 0, s, np.segs[FMT_F64],
+                    L(launch_c(ov, dim3(S), k_nform_f64<NW, S>, unsigned(np.nsegs[FMT_F64]) * S, NW * 32, 0, s, np.segs[FMT_F64],
                                static_cast<const NChunk*>(np.chunks), reinterpret_cast<const double*>(M->store), vx, vt,
                                vo, alpha, add));
                 // reduced precision: one CTA per tile takes the packs of both formats
                 const QNPack* qc = static_cast<const QNPack*>(np.chunks);
                 if (!f64plan && np.nseg2 > 0) {
                     if (np.wide == FMT_I24)
-                        L(launch_c(ov, S, k_nform_q<NW, FMT_I24, FMT_I16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
+                        L(launch_c(ov, dim3(S), k_nform_q<NW, FMT_I24, FMT_I16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
                                    M->store, vx, vt, vo, alpha, add));
                     else if (np.f16 == FMT_BF16)
-                        L(launch_c(ov, S, k_nform_q<NW, FMT_F32, FMT_BF16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
+                        L(launch_c(ov, dim3(S), k_nform_q<NW, FMT_F32, FMT_BF16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
                                    M->store, vx, vt, vo, alpha, add));
                     else
-                        L(launch_c(ov, S, k_nform_q<NW, FMT_F32, FMT_F16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
+                        L(launch_c(ov, dim3(S), k_nform_q<NW, FMT_F32, FMT_F16, S>, unsigned(np.nseg2) * S, NW * 32, 0, s, np.seg2, qc,
                                    M->store, vx, vt, vo, alpha, add));
                 }
             };
@@ -2082,7 +2111,7 @@ hlrc_status run_dw(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, co
             if (ws.profile) prof_begin(M, stage_name(M, 2, st.idx), tp.alg_bytes, s);
             if constexpr (NT == 1) {
                 if (tp.nsegs[FMT_F64] > 0)
-                    L(launch_k(ov, k_ttform_dmma<DMMA_WARPS>, unsigned(tp.nsegs[FMT_F64]), DMMA_WARPS * 32, 0, s,
+                    L(launch_k(ov, k_ttform_dmma<DMMA_WARPS>, dim3(unsigned(tp.nsegs[FMT_F64]), unsigned(tp.msplit)), DMMA_WARPS * 32, 0, s,
                                tp.segs[FMT_F64], static_cast<const TTChunk*>(tp.chunks), A, vec(tp.in), om, ws.mr_part,
                                alpha, add));
                 nl += tp.nsegs[FMT_F64] > 0;
@@ -2121,10 +2150,12 @@ hlrc_status run_dw(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, co
             const double alpha = np.mode == OUT_ADD ? 1.0 : alpha_in;
             const NChunk* ch = static_cast<const NChunk*>(np.chunks);
             if constexpr (NT == 1)
-                L(launch_k(ov, k_nform_dmma<DMMA_WARPS>, unsigned(np.nsegs[FMT_F64]), DMMA_WARPS * 32, 0, s,
+                L(launch_n(ov, k_nform_dmma<DMMA_WARPS, false>, k_nform_dmma<DMMA_WARPS, true>,
+                           np.nsegs[FMT_F64], np.msplit, DMMA_WARPS * 32, 0, s,
                            np.segs[FMT_F64], ch, A, vec(np.vx), vec(np.vt), omap(np.out), alpha, add));
             else
-                L(launch_k(ov, k_nform_dw<NT>, unsigned(np.nsegs[FMT_F64]), DW_WARPS * 32, dw_nsmem<NT>(), s,
+                L(launch_n(ov, k_nform_dw<NT, false>, k_nform_dw<NT, true>,
+                           np.nsegs[FMT_F64], np.msplit, DW_WARPS * 32, dw_nsmem<NT>(), s,
                            np.segs[FMT_F64], ch, A, vec(np.vx), vec(np.vt), omap(np.out), alpha, add));
             ++nl;
             if (ws.profile) prof_end(M, s);
@@ -2202,13 +2233,13 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 if (M->precision == HLRC_PREC_BFP) {
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     if (tp.nmseg[FMT_I24] > 0) {
-                        L(launch_k(ov, k_ttform_bfp<true>, unsigned(tp.nmseg[FMT_I24]), TC_WARPS * 32,
+                        L(launch_k(ov, k_ttform_bfp<true>, dim3(unsigned(tp.nmseg[FMT_I24]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    bq_smem_t(true), s, tp.mseg[FMT_I24], tp.mcol, M->store, vec(tp.in), om, fpart,
                                    alpha, add));
                         ++nl;
                     }
                     if (tp.nmseg[FMT_I16] > 0) {
-                        L(launch_k(ov, k_ttform_bfp<false>, unsigned(tp.nmseg[FMT_I16]), TC_WARPS * 32,
+                        L(launch_k(ov, k_ttform_bfp<false>, dim3(unsigned(tp.nmseg[FMT_I16]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    bq_smem_t(false), s, tp.mseg[FMT_I16], tp.mcol, M->store, vec(tp.in), om, fpart,
                                    alpha, add));
                         ++nl;
@@ -2217,12 +2248,12 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                     const int n32 = tp.nmseg[FMT_F32];
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     if (tp.nmseg[FMT_BF16] > 0) {
-                        L(launch_k(ov, k_ttform_mr<FMT_BF16>, unsigned(n32 + tp.nmseg[FMT_BF16]), TC_WARPS * 32,
+                        L(launch_k(ov, k_ttform_mr<FMT_BF16>, dim3(unsigned(n32 + tp.nmseg[FMT_BF16]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s, tp.mseg[FMT_F32], n32,
                                    tp.mseg[FMT_BF16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add));
                         ++nl;
                     } else if (n32 + tp.nmseg[FMT_F16] > 0) {
-                        L(launch_k(ov, k_ttform_mr<FMT_F16>, unsigned(n32 + tp.nmseg[FMT_F16]), TC_WARPS * 32,
+                        L(launch_k(ov, k_ttform_mr<FMT_F16>, dim3(unsigned(n32 + tp.nmseg[FMT_F16]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s, tp.mseg[FMT_F32], n32,
                                    tp.mseg[FMT_F16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add));
                         ++nl;
@@ -2257,30 +2288,35 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 // the formats of one output tile run as separate grids, each
                 // adding its share to the output in a fixed launch order
                 if (np.nmseg[FMT_F32] > 0) {
-                    L(launch_k(ov, k_nform_d32, unsigned(np.nmseg[FMT_F32]), TC_WARPS * 32,
+                    L(launch_n(ov, k_nform_d32<false>, k_nform_d32<true>,
+                               np.nmseg[FMT_F32], np.msplit, TC_WARPS * 32,
                                tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32), s, np.mseg[FMT_F32], np.mcol, M->store,
                                vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_F16] > 0) {
-                    L(launch_k(ov, k_nform_tc<FMT_F16>, unsigned(np.nmseg[FMT_F16]), TC_WARPS * 32,
+                    L(launch_n(ov, k_nform_tc<FMT_F16, false>, k_nform_tc<FMT_F16, true>,
+                               np.nmseg[FMT_F16], np.msplit, TC_WARPS * 32,
                                tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s, np.mseg[FMT_F16], np.mcol, M->store,
                                vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_BF16] > 0) {
-                    L(launch_k(ov, k_nform_tc<FMT_BF16>, unsigned(np.nmseg[FMT_BF16]), TC_WARPS * 32,
+                    L(launch_n(ov, k_nform_tc<FMT_BF16, false>, k_nform_tc<FMT_BF16, true>,
+                               np.nmseg[FMT_BF16], np.msplit, TC_WARPS * 32,
                                tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s, np.mseg[FMT_BF16], np.mcol, M->store,
                                vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_I24] > 0) {
-                    L(launch_k(ov, k_nform_bfp<true>, unsigned(np.nmseg[FMT_I24]), TC_WARPS * 32, bq_smem_n(true), s,
+                    L(launch_n(ov, k_nform_bfp<true, false>, k_nform_bfp<true, true>,
+                               np.nmseg[FMT_I24], np.msplit, TC_WARPS * 32, bq_smem_n(true), s,
                                np.mseg[FMT_I24], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_I16] > 0) {
-                    L(launch_k(ov, k_nform_bfp<false>, unsigned(np.nmseg[FMT_I16]), TC_WARPS * 32, bq_smem_n(false),
+                    L(launch_n(ov, k_nform_bfp<false, false>, k_nform_bfp<false, true>,
+                               np.nmseg[FMT_I16], np.msplit, TC_WARPS * 32, bq_smem_n(false),
                                s, np.mseg[FMT_I16], np.mcol, M->store, vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }

@@ -135,7 +135,7 @@ __device__ __forceinline__ void stage_bfp(uint8_t* sa, const uint8_t* base, int 
 // A[m][k] = tile row m, stream column k (ldmatrix.trans of the staged
 // words); lane (g, t) accumulates rows 16i + g, 16i + g + 8 for right-hand
 // sides 2t, 2t+1.  Launch: bq_smem_n(I24) bytes of dynamic shared memory.
-template <bool I24>
+template <bool I24, bool SP>
 __global__ void __launch_bounds__(TC_WARPS * 32, HLRC_BQ_MINB)
 k_nform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
             const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
@@ -145,7 +145,7 @@ k_nform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const 
     constexpr int NT = I24 ? 3 : 2;                                        // FP16 terms of the vector operand
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
-    const MSeg sg = segs[blockIdx.x];
+    const MSeg sg = SP ? run_part(segs[blockIdx.x], I24 ? 3 : 2) : segs[blockIdx.x];
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -274,7 +274,7 @@ k_nform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const 
         r1[1] = acc[i][3];
     }
     __syncthreads();
-    nform_store(red, int(sg.vo), sg.rows, om, alpha, add);
+    nform_store<SP>(red, int(sg.vo), sg.rows, om, alpha, add);
 }
 
 // -------------------------------------------------------------- tile T-form
@@ -406,7 +406,7 @@ k_ttform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
     pdl_wait();
-    ttform_bfp<I24>(segs[blockIdx.x], smem, cols, A, vin, om, part, alpha, add);
+    ttform_bfp<I24>(run_part(segs[blockIdx.x], I24 ? 3 : 2), smem, cols, A, vin, om, part, alpha, add);
 }
 
 }  // namespace hlrc

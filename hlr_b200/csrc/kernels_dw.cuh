@@ -79,7 +79,7 @@ __device__ __forceinline__ void dw_cp16(uint32_t dst, const void* src, bool ok) 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-template <int NT>
+template <int NT, bool SP>
 __global__ void __launch_bounds__(DW_WARPS * 32, dw_ctas<NT>())
 k_nform_dw(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
            const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
@@ -88,7 +88,7 @@ k_nform_dw(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, con
     constexpr int VU = RB / 2;   // 16-byte units of a vector row
     extern __shared__ __align__(16) double dw_sn[];
     pdl_trigger();
-    const NSeg sg = segs[blockIdx.x];
+    const NSeg sg = SP ? seg_part(segs[blockIdx.x]) : segs[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int np = (sg.rows + 15) / 16;      // 16-row groups
@@ -181,18 +181,15 @@ k_nform_dw(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, con
             for (int e = 0; e < 2; ++e)
                 red[(warp * TILE + 16 * (i >> 1) + 2 * g + (i & 1)) * RS + dw_vec<NT>(n, t, e)] = acc[i][n][e];
     __syncthreads();
-    // outputs along the direction that is contiguous in memory
-    const bool by_row = om.rs == 1;
-    for (int i = threadIdx.x; i < TILE * RB; i += W * 32) {
-        const int row = by_row ? i % TILE : i / RB, k = by_row ? i / TILE : i % RB;
-        if (row >= sg.rows || k >= om.nr) continue;
-        double s = 0.0;
+    nform_update<RB, W * 32, SP>(
+        int(sg.out), sg.rows, om, alpha, add,
+        [&](int row, int kk) {
+            double s = 0.0;
 #pragma unroll
-        for (int w = 0; w < W; ++w) s += red[(w * TILE + row) * RS + k];
-        double* o = om.base + int64_t(sg.out + row) * om.rs + int64_t(k) * om.cs;
-        if (add) *o += alpha * s;
-        else *o = s;
-    }
+            for (int w = 0; w < W; ++w) s += red[(w * TILE + row) * RS + kk];
+            return s;
+        },
+        [&](int row, int kk) { return red + row * RS + kk; });
 }
 
 // Stores one column's results of a vector group (tiles 2 vg and, with TWO,

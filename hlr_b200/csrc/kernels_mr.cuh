@@ -154,6 +154,48 @@ k_ttfinish_flat(const TGroup* __restrict__ groups, int ngroups, int gpb, const T
 //   tile T-form: contraction = tile rows, k-step s = 2j + b maps fragment
 //     k = t to row 8j + 2t + b; the output rows are the chunk's 8 columns.
 
+// Part blockIdx.y of gridDim.y of a segment's chunks: the CTAs that share a tile.
+template <typename Seg>
+__device__ __forceinline__ Seg seg_part(Seg sg) {
+    if (gridDim.y > 1) {
+        const uint32_t n = sg.ce - sg.cb, cb = sg.cb;
+        sg.cb = cb + n * blockIdx.y / gridDim.y;
+        sg.ce = cb + n * (blockIdx.y + 1) / gridDim.y;
+    }
+    return sg;
+}
+
+// Update of an N-form tile's outputs: sum(row, k) over the warps of this CTA and,
+// with SP, over the cluster of CTAs that share the tile, in rank order (through
+// slot(row, k), a place in this CTA's shared memory that only the thread of (row, k)
+// reads).  Whole tiles have kernels of their own: with one body for both the
+// 32-vector N-form measured 2 % slower.
+template <int RB, int THREADS, bool SP, typename Sum, typename Slot>
+__device__ __forceinline__ void nform_update(int out, int rows, const OutMap& om, double alpha, int add, Sum&& sum,
+                                             Slot&& slot) {
+    const bool by_row = om.rs == 1;   // along the direction that is contiguous in memory
+    if constexpr (SP) {
+        if (blockIdx.y > 0)
+            for (int i = threadIdx.x; i < TILE * RB; i += THREADS) {
+                const int row = by_row ? i % TILE : i / RB, k = by_row ? i / TILE : i % RB;
+                if (row < rows && k < om.nr) *slot(row, k) = sum(row, k);
+            }
+        cg::this_cluster().sync();
+    }
+    if (!SP || blockIdx.y == 0)
+        for (int i = threadIdx.x; i < TILE * RB; i += THREADS) {
+            const int row = by_row ? i % TILE : i / RB, k = by_row ? i / TILE : i % RB;
+            if (row >= rows || k >= om.nr) continue;
+            double s = sum(row, k);
+            if constexpr (SP)
+                for (unsigned p = 1; p < gridDim.y; ++p) s += *cg::this_cluster().map_shared_rank(slot(row, k), p);
+            double* o = om.base + int64_t(out + row) * om.rs + int64_t(k) * om.cs;
+            if (add) *o += alpha * s;
+            else *o = s;
+        }
+    if constexpr (SP) cg::this_cluster().sync();   // the other CTAs' rows have been read
+}
+
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
         : "+d"(d[0]), "+d"(d[1])
@@ -163,13 +205,13 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 // Both kernels keep two operand sets in registers: the loads of chunk
 // c + W are in flight while chunk c is multiplied, and chunk descriptors are
 // read two chunks ahead.
-template <int W>
+template <int W, bool SP>
 __global__ void __launch_bounds__(W * 32, 2)
 k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
              const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
     __shared__ double red[W][TILE][MR_RB];
     pdl_trigger();
-    const NSeg sg = segs[blockIdx.x];
+    const NSeg sg = SP ? seg_part(segs[blockIdx.x]) : segs[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     // acc[2p + b]: tile row 16p + 2g + b, right-hand sides 2t, 2t+1
@@ -233,16 +275,15 @@ k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, c
         red[warp][row][2 * t + 1] = acc[i][1];
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < TILE * MR_RB; i += W * 32) {
-        const int row = i % TILE, k = i / TILE;
-        if (row >= sg.rows || k >= om.nr) continue;
-        double s = 0.0;
+    nform_update<MR_RB, W * 32, SP>(
+        int(sg.out), sg.rows, om, alpha, add,
+        [&](int row, int kk) {
+            double s = 0.0;
 #pragma unroll
-        for (int w = 0; w < W; ++w) s += red[w][row][k];
-        double* o = om.base + int64_t(sg.out + row) * om.rs + int64_t(k) * om.cs;
-        if (add) *o += alpha * s;
-        else *o = s;
-    }
+            for (int w = 0; w < W; ++w) s += red[w][row][kk];
+            return s;
+        },
+        [&](int row, int kk) { return &red[0][row][kk]; });
 }
 
 template <int W>
@@ -250,7 +291,7 @@ __global__ void __launch_bounds__(W * 32, 2)
 k_ttform_dmma(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks, const double* __restrict__ A,
               const double* __restrict__ vin, OutMap om, double* __restrict__ part, double alpha, int add) {
     pdl_trigger();
-    const TTSeg sg = segs[blockIdx.x];
+    const TTSeg sg = seg_part(segs[blockIdx.x]);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     pdl_wait();

@@ -242,20 +242,32 @@ __device__ __forceinline__ void tt_out(const MCol& m, int n, double val, const O
     }
 }
 
+// Part blockIdx.y of gridDim.y of a column run (columns of bytes per element,
+// whole 32-column stages): the CTAs that share a tile.
+__device__ __forceinline__ MSeg run_part(MSeg sg, int bytes) {
+    if (gridDim.y > 1) {
+        const uint32_t st = (sg.ncols + 31) / 32;
+        const uint32_t b = 32 * (st * blockIdx.y / gridDim.y), e = min(32 * (st * (blockIdx.y + 1) / gridDim.y), sg.ncols);
+        sg.a16 += b * (uint32_t(sg.ld) * bytes / 16);
+        sg.col0 += b;
+        sg.ncols = e - b;
+    }
+    return sg;
+}
+
 // Fixed-order sum of the per-warp accumulators of an N-form tile
 // (red[(w * TILE + row) * MR_RB + k]) and the update of the output rows.
-__device__ __forceinline__ void nform_store(const double* red, int out, int rows, const OutMap& om, double alpha,
-                                            int add) {
-    for (int i = threadIdx.x; i < TILE * MR_RB; i += TC_WARPS * 32) {
-        const int row = i % TILE, k = i / TILE;
-        if (row >= rows || k >= om.nr) continue;
-        double sum = 0.0;
+template <bool SP>
+__device__ __forceinline__ void nform_store(double* red, int out, int rows, const OutMap& om, double alpha, int add) {
+    nform_update<MR_RB, TC_WARPS * 32, SP>(
+        out, rows, om, alpha, add,
+        [&](int row, int k) {
+            double sum = 0.0;
 #pragma unroll
-        for (int w = 0; w < TC_WARPS; ++w) sum += red[(w * TILE + row) * MR_RB + k];
-        double* o = om.base + int64_t(out + row) * om.rs + int64_t(k) * om.cs;
-        if (add) *o += alpha * sum;
-        else *o = sum;
-    }
+            for (int w = 0; w < TC_WARPS; ++w) sum += red[(w * TILE + row) * MR_RB + k];
+            return sum;
+        },
+        [&](int row, int k) { return red + row * MR_RB + k; });
 }
 
 // ------------------------------------------------------- 16-bit chunks
@@ -352,14 +364,14 @@ __device__ __forceinline__ void ttform_tc(const MSeg& sg, uint8_t* smem, const M
 // A[m][k] = tile row m, stream column k, read with ldmatrix.trans; lane
 // (g, t) accumulates rows 16i + g, 16i + g + 8 (i < 4) for right-hand sides
 // 2t, 2t+1; fixed-order cross-warp sum at the end.
-template <int FMT>
+template <int FMT, bool SP>
 __global__ void __launch_bounds__(TC_WARPS * 32, HLRC_N16_MINB)
 k_nform_tc(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
            const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
     using O = TcOp<FMT>;
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
-    const MSeg sg = segs[blockIdx.x];
+    const MSeg sg = SP ? run_part(segs[blockIdx.x], 2) : segs[blockIdx.x];
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -446,7 +458,7 @@ k_nform_tc(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const u
         r1[1] = acc[i][3];
     }
     __syncthreads();
-    nform_store(red, int(sg.vo), sg.rows, om, alpha, add);
+    nform_store<SP>(red, int(sg.vo), sg.rows, om, alpha, add);
 }
 
 // --------------------------------------------------------- FP32 chunks
@@ -521,12 +533,13 @@ __device__ __forceinline__ void ttform_d32(const MSeg& sg, uint8_t* smem, const 
 
 // N-form: one CTA per output tile; 16-column stages; the vector entries (times
 // the column scale) are the B operand, and the MMA accumulates in FP64.
+template <bool SP>
 __global__ void __launch_bounds__(TC_WARPS * 32)
 k_nform_d32(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
             const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
-    const MSeg sg = segs[blockIdx.x];
+    const MSeg sg = SP ? run_part(segs[blockIdx.x], 4) : segs[blockIdx.x];
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -582,7 +595,7 @@ k_nform_d32(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const 
         red[(warp * TILE + row) * MR_RB + 2 * t + 1] = acc[i][1];
     }
     __syncthreads();
-    nform_store(red, int(sg.vo), sg.rows, om, alpha, add);
+    nform_store<SP>(red, int(sg.vo), sg.rows, om, alpha, add);
 }
 
 // One tile T-form pass of a reduced-precision store in one grid: the first
@@ -598,8 +611,8 @@ k_ttform_mr(const MSeg* __restrict__ segs32, int n32, const MSeg* __restrict__ s
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
     pdl_wait();
-    if (int(blockIdx.x) < n32) ttform_d32(segs32[blockIdx.x], smem, cols, A, vin, om, part, alpha, add);
-    else ttform_tc<F16>(segs16[blockIdx.x - n32], smem, cols, A, vin, om, part, alpha, add);
+    if (int(blockIdx.x) < n32) ttform_d32(run_part(segs32[blockIdx.x], 4), smem, cols, A, vin, om, part, alpha, add);
+    else ttform_tc<F16>(run_part(segs16[blockIdx.x - n32], 2), smem, cols, A, vin, om, part, alpha, add);
 }
 
 }  // namespace hlrc

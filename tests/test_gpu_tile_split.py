@@ -1,6 +1,6 @@
-"""One-vector products of matrices with few, heavy tiles: a cluster of 2 or 4
-CTAs sums each output tile of the N-form (distributed shared memory), and 2 or
-4 CTAs share the columns of each input tile of the T-form.  Sizes around the
+"""Products of matrices with few, heavy tiles: a cluster of 2 or 4 CTAs sums
+each output tile of the N-form (distributed shared memory), and 2 or 4 CTAs
+share the columns of each input tile of the T-form.  Sizes around the
 limits (148 and 296 tiles, ragged tiles, runs shorter than a CTA's share),
 every store format, against the oracle (arith/mulvec.hh:158-312 restated);
 direct launches, plain launches and graph replays give identical bits, and
@@ -60,5 +60,30 @@ def test_few_heavy_tiles(n, prec, op):
     yo = np.zeros(n)
     oracle.hmvm_seq(hm.h_desc(), 1.5, op, xh, yo)
     assert relerr(y - y0, yo) <= TOL[prec]
+    assert M.device_error() == 0
+    M.free()
+
+
+@pytest.mark.parametrize("n,prec,nrhs", [(3001, "f64", 5), (3001, "f64", 16), (6007, "f64", 23), (9001, "f64", 32),
+                                         (3001, "mixed", 8), (6007, "bfp", 3), (6007, "f32", 8), (9001, "bf16", 7),
+                                         (3001, "f16", 8), (6007, "mixed", 19)])
+@pytest.mark.parametrize("op", [0, 1])
+def test_few_heavy_tiles_several_vectors(n, prec, nrhs, op):
+    hm = built(f"exp_{n}", lambda: hlr.build(hlr.Problem.exp3d(n)))
+    M = hlr.upload(hm, precision=prec, max_nrhs=nrhs)
+    rng = np.random.default_rng(n + nrhs)
+    X, Y0 = rng.standard_normal((nrhs, n)), rng.standard_normal((nrhs, n))
+    Xd = torch.from_numpy(X).cuda().T
+    ys = []
+    for _ in range(2):
+        Yd = torch.from_numpy(Y0.copy()).cuda().T
+        hlr.mul_vec(-0.75, op, M, Xd, Yd)
+        torch.cuda.synchronize()
+        ys.append(Yd.T.cpu().numpy() - Y0)
+    assert np.array_equal(ys[0], ys[1])
+    for j in range(0, nrhs, 4):
+        yo = np.zeros(n)
+        oracle.hmvm_seq(hm.h_desc(), -0.75, op, X[j], yo)
+        assert relerr(ys[0][j], yo) <= TOL[prec], j
     assert M.device_error() == 0
     M.free()
