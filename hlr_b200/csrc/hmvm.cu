@@ -2286,23 +2286,30 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 const double alpha = np.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
                 const OutMap om = omap(np.out);
                 // the formats of one output tile run as separate grids, each
-                // adding its share to the output in a fixed launch order
+                // adding its share to the output in a fixed launch order.
+                // Whole tiles of the FP32 and 16-bit kernels are launched
+                // plainly: their one or two waves, started while the
+                // predecessor drains, crowd the SMs that empty first (FP32
+                // n = 20011 226 -> 250 us, FP16/FP32 n = 32768 adjoint
+                // 263 -> 274, batch of 4, 2 vectors 115 -> 121; the other way
+                // n = 65536 437 -> 432, BFP n = 20011 234 -> 229)
+                const bool early = ov && np.msplit > 1;
                 if (np.nmseg[FMT_F32] > 0) {
-                    L(launch_n(ov, k_nform_d32<false>, k_nform_d32<true>,
+                    L(launch_n(early, k_nform_d32<false>, k_nform_d32<true>,
                                np.nmseg[FMT_F32], np.msplit, TC_WARPS * 32,
                                tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32), s, np.mseg[FMT_F32], np.mcol, M->store,
                                vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_F16] > 0) {
-                    L(launch_n(ov, k_nform_tc<FMT_F16, false>, k_nform_tc<FMT_F16, true>,
+                    L(launch_n(early, k_nform_tc<FMT_F16, false>, k_nform_tc<FMT_F16, true>,
                                np.nmseg[FMT_F16], np.msplit, TC_WARPS * 32,
                                tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s, np.mseg[FMT_F16], np.mcol, M->store,
                                vec(np.vx), vec(np.vt), om, alpha, add));
                     ++nl;
                 }
                 if (np.nmseg[FMT_BF16] > 0) {
-                    L(launch_n(ov, k_nform_tc<FMT_BF16, false>, k_nform_tc<FMT_BF16, true>,
+                    L(launch_n(early, k_nform_tc<FMT_BF16, false>, k_nform_tc<FMT_BF16, true>,
                                np.nmseg[FMT_BF16], np.msplit, TC_WARPS * 32,
                                tc_smem_bytes(TC_STAGE_N16, TC_STAGES_N16), s, np.mseg[FMT_BF16], np.mcol, M->store,
                                vec(np.vx), vec(np.vt), om, alpha, add));
