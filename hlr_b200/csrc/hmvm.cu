@@ -388,6 +388,33 @@ struct DeviceGuard {
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// Zeroes device memory and returns when it is zero.  A memset of device memory
+// is asynchronous to the host, and on the legacy default stream it is not
+// ordered with the non-blocking streams that products may run on.  A stream of
+// its own, so that work queued on the default stream does not hold up the call.
+cudaError_t zero_now(void* p, size_t bytes) {
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(p, 0, bytes, s);
+    const cudaError_t es = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+    return e != cudaSuccess ? e : es;
+}
+
+// Returns when what this thread put on the legacy default stream so far has
+// happened: a copy from pageable memory may return while its last part is on
+// its way to the device.
+cudaError_t legacy_done() {
+    cudaEvent_t ev = nullptr;
+    cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    e = cudaEventRecord(ev, nullptr);
+    if (e == cudaSuccess) e = cudaEventSynchronize(ev);
+    cudaEventDestroy(ev);
+    return e;
+}
+
 const char* stage_name(hlrc_hmat M, int nk, int idx) {
     // names used in profiles: kind 0 = H, 1 = uniform; nk = stage kind (0 T, 1 N, 2 tile T);
     // plans with their own names (H^2) carry them per pass
@@ -1617,6 +1644,16 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
                                : (st.kind == 1 ? hp->n[size_t(st.idx)].launches() : hp->tt[size_t(st.idx)].launches());
         hp->info.launches[op] = nl;
     }
+    // products may run on any stream from here on: the tables, counters and
+    // error word are in place before the handle is given out
+    if (e = legacy_done(); e != cudaSuccess) {
+        cudaFree(hp->w_arena);
+        cudaFree(hp->w_static);
+        cudaFree(hp->mr_tables);
+        cudaFree(hp->mr_arena);
+        cleanup();
+        return fail(HLRC_ERR_CUDA, "upload: %s", cudaGetErrorString(e));
+    }
     *out = h.release();
     return HLRC_OK;
 }
@@ -2837,7 +2874,7 @@ extern "C" hlrc_status hlrc_check_device_error(hlrc_hmat M, int* code) {
     DeviceGuard g(M->device);
     if (!g.ok) return fail(HLRC_ERR_CUDA, "cannot select device %d", M->device);
     HLRC_CUDA(cudaMemcpy(code, M->dev_err, sizeof(int), cudaMemcpyDeviceToHost));
-    HLRC_CUDA(cudaMemset(M->dev_err, 0, sizeof(int)));
+    HLRC_CUDA(zero_now(M->dev_err, sizeof(int)));
     return HLRC_OK;
 }
 
@@ -2988,7 +3025,8 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     if (M->n_part2 > 0) W->ws.part2 = reinterpret_cast<double*>(W->arena + o_p2);
     W->n_part2 = M->n_part2;
     W->ws.ctr = reinterpret_cast<unsigned*>(W->arena + o_ctr);
-    if (const cudaError_t me = cudaMemset(W->ws.ctr, 0, FLOW_CTRS * sizeof(unsigned)); me != cudaSuccess) {
+    // before the call returns: products on the workspace may run on any stream
+    if (const cudaError_t me = zero_now(W->ws.ctr, FLOW_CTRS * sizeof(unsigned)); me != cudaSuccess) {
         cudaFree(W->arena);
         return fail(HLRC_ERR_CUDA, "hlrc_workspace_create: %s", cudaGetErrorString(me));
     }
