@@ -163,6 +163,16 @@ int nform_default(size_t tiles, size_t chunks) {
 }
 int ttform_default(size_t tiles, size_t chunks) { return chunks <= 4 * tiles ? 4 : 8; }
 
+// Counters of one-launch products (FLOW_CTRS words of device memory, zero at
+// first) and the number of the last product that ran on them.  The lock is held
+// from taking a number to the launch, so that numbers grow in launch order
+// whichever threads call.
+struct FlowCount {
+    unsigned long long* dev = nullptr;
+    std::mutex mu;
+    uint64_t last = 0;
+};
+
 // Scratch used by one product: the coefficient vectors and the partial sums
 // of a one-vector product, and (when present) the same arrays as row-major
 // blocks of MR_RB (FP64 stores: up to DW_MAXNT * MR_RB) vectors for the
@@ -173,7 +183,7 @@ struct Workspace {
     double* t2 = nullptr;
     double* part = nullptr;
     double* part2 = nullptr;     // partial sums of a transposed near field that runs beside the chain
-    unsigned* ctr = nullptr;     // counters of one-launch products (FLOW_CTRS, zero between products)
+    FlowCount* ctr = nullptr;    // of one-launch products (its owner is the handle, the workspace or the library)
     int mr_nt = 0;               // the multi-vector arrays hold blocks of 8 * mr_nt vectors
     double* mr_x = nullptr;      // null: no multi-vector arrays
     double* mr_t = nullptr;
@@ -278,7 +288,7 @@ struct hlrc_hmat_s {
         bool near_t = false;   // the side pass is a transposed near field: needs part2
     };
     Flow flow[3];
-    unsigned* ctr = nullptr;           // counters of the handle's own workspace
+    FlowCount ctr;                     // of the handle's own workspace
     // multi-RHS workspace (allocated at upload when max_nrhs > 1): row-major
     // blocks of MR_RB * mr_nt vectors
     char* mr_arena = nullptr;
@@ -500,7 +510,7 @@ ArenaLayout arena_layout(const Plan& p) {
         if (const int nt = near_t_stage(p, op); nt >= 0)
             L.part2_elems = std::max(L.part2_elems, size_t(p.ttpasses[size_t(p.stages[op][size_t(nt)].idx)].npart));
     L.part2 = take(L.part2_elems * sizeof(double));
-    L.ctr = take(FLOW_CTRS * sizeof(unsigned));
+    L.ctr = take(FLOW_CTRS * sizeof(unsigned long long));
     L.err = take(sizeof(int));
     L.part_elems = part_elems;
     L.total = off;
@@ -1456,7 +1466,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         hp->tt.push_back(d);
     }
     if (e == cudaSuccess) e = cudaMemset(hp->arena + L.err, 0, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(hp->arena + L.ctr, 0, FLOW_CTRS * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(hp->arena + L.ctr, 0, FLOW_CTRS * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         cleanup();
         return fail(HLRC_ERR_CUDA, "upload copy failed: %s", cudaGetErrorString(e));
@@ -1474,7 +1484,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
     hp->ws_t2 = reinterpret_cast<double*>(hp->arena + o_t2);
     hp->part = reinterpret_cast<double*>(hp->arena + o_part);
     hp->dev_err = reinterpret_cast<int*>(hp->arena + L.err);
-    hp->ctr = reinterpret_cast<unsigned*>(hp->arena + L.ctr);
+    hp->ctr.dev = reinterpret_cast<unsigned long long*>(hp->arena + L.ctr);
     hp->n_part2 = int64_t(L.part2_elems);
     hp->part2 = L.part2_elems ? reinterpret_cast<double*>(hp->arena + L.part2) : nullptr;
     for (int op = 0; op < 3; ++op) {
@@ -1663,7 +1673,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
 Workspace handle_workspace(hlrc_hmat M) {
     Workspace w;
     w.t = M->ws_t; w.t2 = M->ws_t2; w.part = M->part;
-    w.ctr = M->ctr;
+    w.ctr = &M->ctr;
     w.part2 = M->part2;
     w.mr_nt = M->mr_nt;
     w.mr_x = M->mr_x; w.mr_t = M->mr_t; w.mr_t2 = M->mr_t2; w.mr_part = M->mr_part;
@@ -1893,13 +1903,15 @@ hlrc_status run_flow(hlrc_hmat M, const Workspace& ws, double alpha, int op, con
     a.v[4] = ws.part;
     a.v[5] = ws.part2;
     a.alpha = alpha;
-    a.ctr = ws.ctr;
+    a.ctr = ws.ctr->dev;
     a.err = M->dev_err;
     a.wait_ns = M->wait_ns;
     a.skip = M->wait_skip;
     const int grid = std::min(FLOW_CTAS * M->sms, F.main_items + F.side_items);
     a.main_ctas = grid - (F.side >= 0 ? std::min(F.side_items, grid / 2) : 0);
     M->launches += 1;
+    std::lock_guard<std::mutex> lock(ws.ctr->mu);
+    a.base = ++ws.ctr->last << FLOW_CNT_BITS;
     const cudaError_t e = launch_k(M->overlap != 0, k_flow_f64, unsigned(grid), 256, 0, s, a);
     if (e != cudaSuccess) return fail(HLRC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
     return HLRC_OK;
@@ -2890,16 +2902,16 @@ extern "C" hlrc_status hlrc_check_device_error(hlrc_hmat M, int* code) {
 // per device with cudaGetSymbolAddress while that device is current.
 constexpr size_t NOALLOC_SCRATCH_DOUBLES = size_t(1) << 20;  // 8 MiB
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_SCRATCH_DOUBLES];
-static __device__ __align__(256) unsigned g_noalloc_ctr[FLOW_CTRS];   // one-launch products: zero between calls
+static __device__ __align__(256) unsigned long long g_noalloc_ctr[FLOW_CTRS];   // one-launch products
 
 namespace {
 constexpr int NOALLOC_MAX_DEVICES = 128;
 std::mutex g_noalloc_mu;
 double* g_noalloc_ptr[NOALLOC_MAX_DEVICES] = {};
-unsigned* g_noalloc_ctr_ptr[NOALLOC_MAX_DEVICES] = {};
+FlowCount g_noalloc_count[NOALLOC_MAX_DEVICES];
 
 // device address of the scratch on `dev` (which must be current)
-hlrc_status noalloc_scratch(int dev, double** out, unsigned** ctr) {
+hlrc_status noalloc_scratch(int dev, double** out, FlowCount** ctr) {
     if (dev < 0 || dev >= NOALLOC_MAX_DEVICES)
         return fail(HLRC_ERR_ARG, "hlrc_mvm_noalloc: device ordinal %d outside 0..%d", dev, NOALLOC_MAX_DEVICES - 1);
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
@@ -2911,10 +2923,10 @@ hlrc_status noalloc_scratch(int dev, double** out, unsigned** ctr) {
             return fail(HLRC_ERR_CUDA, "hlrc_mvm_noalloc: cudaGetSymbolAddress on device %d failed: %s", dev,
                         cudaGetErrorString(e));
         g_noalloc_ptr[dev] = static_cast<double*>(p);
-        g_noalloc_ctr_ptr[dev] = static_cast<unsigned*>(c);
+        g_noalloc_count[dev].dev = static_cast<unsigned long long*>(c);
     }
     *out = g_noalloc_ptr[dev];
-    *ctr = g_noalloc_ctr_ptr[dev];
+    *ctr = &g_noalloc_count[dev];
     return HLRC_OK;
 }
 }  // namespace
@@ -2935,7 +2947,7 @@ extern "C" hlrc_status hlrc_mvm_noalloc(hlrc_hmat M, double alpha, int op, const
     DeviceGuard g(M->device);
     if (!g.ok) return fail(HLRC_ERR_CUDA, "cannot select device %d", M->device);
     double* base = nullptr;
-    unsigned* ctr = nullptr;
+    FlowCount* ctr = nullptr;
     st = noalloc_scratch(M->device, &base, &ctr);
     if (st != HLRC_OK) return st;
     // every scratch entry a product reads is written earlier in the same
@@ -2968,6 +2980,7 @@ struct hlrc_workspace_s {
     size_t w_xs = 0, w_ts = 0, w_part = 0;                // 64-vector capacities in bytes (0: none)
     char* arena = nullptr;
     size_t bytes = 0;
+    FlowCount ctr;
     Workspace ws;
 };
 
@@ -2986,7 +2999,7 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     size_t off = 0;
     auto take = [&](size_t elems) { const size_t o_ = off; off = align_up(off + elems * sizeof(double), 256); return o_; };
     const size_t o_t = take(size_t(W->n_t)), o_t2 = take(size_t(W->n_t2)), o_p = take(size_t(W->n_part)),
-                 o_p2 = take(size_t(M->n_part2)), o_ctr = take(FLOW_CTRS * sizeof(unsigned) / sizeof(double) + 1);
+                 o_p2 = take(size_t(M->n_part2)), o_ctr = take(FLOW_CTRS);   // words of a double's size
     WideSizes zw;
     size_t o_w = 0;
     if (max_nrhs > MR_RB && M->wide) {
@@ -3024,9 +3037,10 @@ extern "C" hlrc_status hlrc_workspace_create(hlrc_hmat M, int max_nrhs, hlrc_wor
     W->ws.part = reinterpret_cast<double*>(W->arena + o_p);
     if (M->n_part2 > 0) W->ws.part2 = reinterpret_cast<double*>(W->arena + o_p2);
     W->n_part2 = M->n_part2;
-    W->ws.ctr = reinterpret_cast<unsigned*>(W->arena + o_ctr);
+    W->ctr.dev = reinterpret_cast<unsigned long long*>(W->arena + o_ctr);
+    W->ws.ctr = &W->ctr;
     // before the call returns: products on the workspace may run on any stream
-    if (const cudaError_t me = zero_now(W->ws.ctr, FLOW_CTRS * sizeof(unsigned)); me != cudaSuccess) {
+    if (const cudaError_t me = zero_now(W->ctr.dev, FLOW_CTRS * sizeof(unsigned long long)); me != cudaSuccess) {
         cudaFree(W->arena);
         return fail(HLRC_ERR_CUDA, "hlrc_workspace_create: %s", cudaGetErrorString(me));
     }

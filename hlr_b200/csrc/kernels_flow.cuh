@@ -17,9 +17,16 @@
 // Progress.  A queue is a counter: tickets are taken in pass order, so the
 // items an item waits for are held by CTAs that already run, whatever part of
 // the grid is resident; no co-residency is needed.  Every wait is bounded
-// (wait_ns): one that runs out sets bit 0 of the error word and an abort flag
-// on which all CTAs leave.  The last CTA to leave zeroes the counters for the
-// next product of the workspace.
+// (wait_ns): one that runs out sets bit 0 of the error word and a stop mark
+// on which all CTAs leave.
+//
+// Counters.  Each counter holds the number of the product that uses it above
+// FLOW_CNT_BITS bits of count.  A product's number is larger than those before
+// it on the same counters, and every CTA first raises the counters to it
+// (atomicMax), so whatever an earlier product left there, one that gave up or
+// products that wrongly overlapped on one workspace, reads as zero.  A ticket
+// of another number means such an overlap: the CTA reports it (bit 0) and
+// leaves, as it does for a ticket out of range.
 //
 // Vectors written in the launch are read through L2 (__ldcg): L1 is not
 // coherent with other SMs' writes.  The sums are those of the separate
@@ -34,7 +41,9 @@
 namespace hlrc {
 
 constexpr int FLOW_MAXST = 12;        // passes of a product
-constexpr int FLOW_CTRS = 8 + FLOW_MAXST;   // tickets (main, side), leavers, abort flag; items done per pass
+constexpr int FLOW_CTRS = 3 + FLOW_MAXST;   // tickets (main, side), stop mark; items done per pass
+constexpr int FLOW_CNT_BITS = 20;     // count of a counter (5.6 years of products of 10 us for the number above it)
+constexpr unsigned long long FLOW_CNT_MASK = (1ull << FLOW_CNT_BITS) - 1;
 constexpr int FLOW_CTAS = 2;          // CTAs per SM: 128 registers (three: 80, spills, 33 us against 25 us at n = 8192)
 
 enum : int32_t { FLOW_N = 0, FLOW_TT = 1, FLOW_FINISH = 2, FLOW_T = 3, FLOW_TFINISH = 4 };
@@ -62,7 +71,8 @@ struct FlowArgs {
     const double* A;
     double* v[6];                    // by VecName; [4] the partial sums, [5] those of a side pass
     double alpha;
-    unsigned* ctr;
+    unsigned long long* ctr;
+    unsigned long long base;         // the product's number << FLOW_CNT_BITS
     int* err;
     uint64_t wait_ns;
     int skip;                        // test hook: the first item of the chain is never counted as done
@@ -180,9 +190,9 @@ __device__ __forceinline__ void flow_ttform(const TTSeg& sg, const TTChunk* __re
     }
 }
 
-__device__ __forceinline__ unsigned flow_load(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned long long flow_load(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -195,14 +205,24 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_wait();
-    unsigned* done = a.ctr + 8;
+    unsigned long long* const stop = a.ctr + 2;
+    unsigned long long* const done = a.ctr + 3;
+    if (threadIdx.x < FLOW_CTRS && threadIdx.x != 2) atomicMax(a.ctr + threadIdx.x, a.base);
+    __syncthreads();
     int flip = 0, flip_ok = 0;   // a slot is written again only two barriers later
     bool ok = true;          // no wait ran out (the same in every thread)
     uint32_t seen = 0;       // passes known to be done
-    // the next ticket of queue q (0 chain, 1 near field)
+    // the next ticket of queue q (0 chain, 1 near field); -1: not one of this product
     auto take = [&](int q) {
         flip ^= 1;
-        if (threadIdx.x == 0) s_item[flip] = int(atomicAdd(a.ctr + q, 1u));
+        if (threadIdx.x == 0) {
+            const unsigned long long v = atomicAdd(a.ctr + q, 1ull), num = v & ~FLOW_CNT_MASK;
+            if (num != a.base) {   // another product runs on these counters: its ticket is lost as well
+                atomicOr(a.err, 1);
+                atomicExch(stop, num);
+            }
+            s_item[flip] = num == a.base ? int(v & FLOW_CNT_MASK) : -1;
+        }
         __syncthreads();
         return s_item[flip];
     };
@@ -211,16 +231,20 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
         if (d < 0 || (seen >> d & 1u) || !ok) return;
         flip_ok ^= 1;
         if (threadIdx.x == 0) {
-            const unsigned want = unsigned(a.st[d].nitems);
+            const unsigned long long want = a.base + unsigned(a.st[d].nitems);
             bool good = true;
             if (flow_load(done + d) < want) {
                 const uint64_t t0 = tree_clock();
                 for (uint32_t i = 1; flow_load(done + d) < want; ++i) {
                     if ((i & 15u) != 0u) continue;
-                    if (flow_load(a.ctr + 3) != 0u) { good = false; break; }
+                    if (flow_load(stop) == a.base) {
+                        atomicOr(a.err, 1);   // marked by this product, or by another that took its ticket
+                        good = false;
+                        break;
+                    }
                     if (tree_clock() - t0 > a.wait_ns) {
                         atomicOr(a.err, 1);
-                        atomicExch(a.ctr + 3, 1u);
+                        atomicExch(stop, a.base);
                         good = false;
                         break;
                     }
@@ -273,7 +297,7 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
         }
         __syncthreads();
         if (threadIdx.x == 0 && ok && !(a.skip && s != a.side && p.first + item == 0)) {
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(done + s) : "memory");
+            asm volatile("red.release.gpu.global.add.u64 [%0], 1;\n" ::"l"(done + s) : "memory");
         }
     };
     // one item per round: from the near field's queue while `side` (at the
@@ -286,6 +310,7 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
         int s = a.side, item;
         if (side) {
             item = take(1);
+            if (item < 0) break;
             if (item >= a.side_items) {
                 side = false;
                 drained = true;
@@ -294,6 +319,7 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
         } else {
             item = held >= 0 ? held : take(0);
             held = -1;
+            if (item < 0) break;
             if (item >= a.main_items) {   // no chain left; nor a near field that no pass waits for
                 if (drained) break;
                 side = true;
@@ -309,15 +335,6 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
             item -= a.st[s].first;
         }
         run(s, item);
-    }
-    // leave; the last one zeroes the counters
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(a.ctr + 2, 1u) == gridDim.x - 1) {
-            __threadfence();
-            for (int i = 0; i < FLOW_CTRS; ++i) a.ctr[i] = 0u;
-        }
     }
 }
 

@@ -348,8 +348,11 @@ hlrc_status hlrc_mvm_host(hlrc_hmat M, double alpha, int op, const double* x,
  *    handles on the same device — race; order them on one stream.
  *  - Uniform-H and H^2 handles are accepted (op N and C).
  *  - A near field planned as its own pass (hlrc_options.near_field) runs
- *    first on `stream`, not beside the other passes: the same kernels in
- *    the same order on y, so the same result as hlrc_mvm.               */
+ *    first on `stream`, not on a stream beside the other passes; a small FP64
+ *    product runs as one launch, as with hlrc_mvm.  y is summed in the same
+ *    order either way, so the result is that of hlrc_mvm.  Products that
+ *    wrongly overlap spoil only their own results: the counters of a launch
+ *    do not depend on what an earlier one left in them.                  */
 hlrc_status hlrc_mvm_noalloc(hlrc_hmat M, double alpha, int op,
                              const double* x, double* y, void* stream);
 
@@ -450,7 +453,8 @@ hlrc_status hlrc_fp64_peak(int device, double* tflops);
  * that wait with a bound set it when a wait runs out; the products launched
  * since then are incomplete.  0 means no error; bit 0 (value 1): a copy wait
  * of an H^2 tree sweep, or a wait between the passes of a product that runs
- * as one launch, ran out; bit 1 (value 2): a stage hand-over of the
+ * as one launch, ran out (or such a product found another running on its
+ * workspace); bit 1 (value 2): a stage hand-over of the
  * 64-vector kernels ran out.                                                 */
 hlrc_status hlrc_check_device_error(hlrc_hmat M, int* code);
 
