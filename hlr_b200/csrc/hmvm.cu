@@ -2517,72 +2517,82 @@ bool pageable(const void* p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
-// The ring holds min(HOST_SLOTS, what `bytes` need) slots or more.
-hlrc_status host_ring(hlrc_hmat M, size_t bytes) {
+// Makes the ring hold min(HOST_SLOTS, what `bytes` need) slots or more; false
+// where the pinned memory or its events are not to be had (the call then copies
+// directly).
+bool host_ring(hlrc_hmat M, size_t bytes) {
     const int want = int(std::min<size_t>(HOST_SLOTS, (bytes + HOST_SLOT - 1) / HOST_SLOT));
-    for (cudaEvent_t& e : M->pin_ev)
-        if (!e) HLRC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    if (want <= M->pin_slots) return HLRC_OK;
-    if (M->pin) cudaFreeHost(M->pin);
-    M->pin = nullptr;
-    M->pin_slots = 0;
-    HLRC_CUDA(cudaMallocHost(&M->pin, size_t(want) * HOST_SLOT));
-    M->pin_slots = want;
-    return HLRC_OK;
+    cudaError_t e = cudaSuccess;
+    for (cudaEvent_t& ev : M->pin_ev)
+        if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess && want > M->pin_slots) {
+        if (M->pin) cudaFreeHost(M->pin);
+        M->pin = nullptr;
+        M->pin_slots = 0;
+        e = cudaMallocHost(&M->pin, size_t(want) * HOST_SLOT);
+        if (e == cudaSuccess) M->pin_slots = want;
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
 }
 
-// Visits nrhs columns of n doubles, slot by slot: f(element offset in a
-// packed array, column, first row, elements).
+// The columns of nrhs vectors of n doubles (ld apart) as one packed sequence:
+// f(pointer into the vectors, elements) for each run of column entries in
+// [at, at + m).  Short columns share a slot (n = 1000, 16 vectors: one slot and
+// one copy each way; a slot per column took 323 us, a copy of pitched columns
+// each way 120 us).
 template <typename F>
-hlrc_status host_pieces(int64_t n, int nrhs, F&& f) {
-    constexpr int64_t per = int64_t(HOST_SLOT / sizeof(double));
-    for (int r = 0; r < nrhs; ++r)
-        for (int64_t i = 0; i < n; i += per)
-            if (const hlrc_status st = f(int64_t(r) * n + i, r, i, std::min(per, n - i)); st != HLRC_OK) return st;
-    return HLRC_OK;
+void host_runs(double* v, int64_t n, int64_t ld, int64_t at, int64_t m, F&& f) {
+    for (int64_t r = at / n, i = at % n; m > 0; ++r, i = 0) {
+        const int64_t c = std::min(m, n - i);
+        f(v + r * ld + i, c);
+        m -= c;
+    }
 }
+
+constexpr int64_t HOST_PER = int64_t(HOST_SLOT / sizeof(double));   // elements of a slot
 
 // dev (packed) = v, through the ring, on the legacy default stream
 hlrc_status host_put(hlrc_hmat M, double* dev, const double* v, int64_t n, int nrhs, int64_t ld) {
-    int k = 0;
-    return host_pieces(n, nrhs, [&](int64_t at, int r, int64_t i, int64_t m) -> hlrc_status {
-        const int slot = k % M->pin_slots;
+    const int64_t total = n * nrhs;
+    for (int64_t at = 0, k = 0; at < total; at += HOST_PER, ++k) {
+        const int slot = int(k % M->pin_slots);
         char* p = M->pin + size_t(slot) * HOST_SLOT;
+        const int64_t m = std::min(HOST_PER, total - at);
         HLRC_CUDA(cudaEventSynchronize(M->pin_ev[slot]));   // also a copy that a failed call left behind
-        std::memcpy(p, v + int64_t(r) * ld + i, size_t(m) * sizeof(double));
+        char* d = p;
+        host_runs(const_cast<double*>(v), n, ld, at, m, [&](const double* c, int64_t len) {
+            std::memcpy(d, c, size_t(len) * sizeof(double));
+            d += size_t(len) * sizeof(double);
+        });
         HLRC_CUDA(cudaMemcpyAsync(dev + at, p, size_t(m) * sizeof(double), cudaMemcpyHostToDevice, nullptr));
         HLRC_CUDA(cudaEventRecord(M->pin_ev[slot], nullptr));
-        ++k;
-        return HLRC_OK;
-    });
+    }
+    return HLRC_OK;
 }
 
 // v += dev (packed), through the ring; returns when v is complete
 hlrc_status host_add(hlrc_hmat M, const double* dev, double* v, int64_t n, int nrhs, int64_t ld) {
-    struct Piece { double* v; int64_t m; };
-    std::vector<Piece> q;   // pieces in flight, by slot
-    q.resize(size_t(M->pin_slots));
-    auto take = [&](int slot) -> hlrc_status {
-        HLRC_CUDA(cudaEventSynchronize(M->pin_ev[slot]));
-        const double* p = reinterpret_cast<const double*>(M->pin + size_t(slot) * HOST_SLOT);
-        const Piece c = q[size_t(slot)];
-        for (int64_t i = 0; i < c.m; ++i) c.v[i] += p[i];
-        return HLRC_OK;
-    };
-    int k = 0;
-    hlrc_status st = host_pieces(n, nrhs, [&](int64_t at, int r, int64_t i, int64_t m) -> hlrc_status {
-        const int slot = k % M->pin_slots;
-        if (k >= M->pin_slots)
-            if (const hlrc_status ts = take(slot); ts != HLRC_OK) return ts;
-        HLRC_CUDA(cudaMemcpyAsync(M->pin + size_t(slot) * HOST_SLOT, dev + at, size_t(m) * sizeof(double),
-                                  cudaMemcpyDeviceToHost, nullptr));
-        HLRC_CUDA(cudaEventRecord(M->pin_ev[slot], nullptr));
-        q[size_t(slot)] = Piece{v + int64_t(r) * ld + i, m};
-        ++k;
-        return HLRC_OK;
-    });
-    for (int j = std::max(0, k - M->pin_slots); j < k && st == HLRC_OK; ++j) st = take(j % M->pin_slots);
-    return st;
+    const int64_t total = n * nrhs, pieces = (total + HOST_PER - 1) / HOST_PER;
+    for (int64_t k = 0; k < pieces + M->pin_slots; ++k) {   // piece k starts when piece k - pin_slots is added
+        if (const int64_t j = k - M->pin_slots; j >= 0 && j < pieces) {
+            const int slot = int(j % M->pin_slots);
+            HLRC_CUDA(cudaEventSynchronize(M->pin_ev[slot]));
+            const double* p = reinterpret_cast<const double*>(M->pin + size_t(slot) * HOST_SLOT);
+            host_runs(v, n, ld, j * HOST_PER, std::min(HOST_PER, total - j * HOST_PER), [&](double* c, int64_t len) {
+                for (int64_t i = 0; i < len; ++i) c[i] += p[i];
+                p += len;
+            });
+        }
+        if (k < pieces) {
+            const int slot = int(k % M->pin_slots);
+            const int64_t at = k * HOST_PER, m = std::min(HOST_PER, total - at);
+            HLRC_CUDA(cudaMemcpyAsync(M->pin + size_t(slot) * HOST_SLOT, dev + at, size_t(m) * sizeof(double),
+                                      cudaMemcpyDeviceToHost, nullptr));
+            HLRC_CUDA(cudaEventRecord(M->pin_ev[slot], nullptr));
+        }
+    }
+    return HLRC_OK;
 }
 
 hlrc_status check_mvm_args(hlrc_hmat M, int op, const double* x, double* y, int nrhs, int64_t ldx, int64_t ldy) {
@@ -2764,9 +2774,9 @@ extern "C" hlrc_status hlrc_mvm_host(hlrc_hmat M, double alpha, int op, const do
     // pageable y: the product goes into zeroed device memory and the host adds
     // it to y, which saves y's way down; vectors the driver knows (pinned,
     // managed) are copied directly
-    const bool add_y = pageable(y), ring_x = pageable(x);
-    if (add_y || ring_x)
-        if (st = host_ring(M, std::max(ring_x ? ex : 0, add_y ? ey : 0) * sizeof(double)); st != HLRC_OK) return st;
+    bool add_y = pageable(y), ring_x = pageable(x);
+    if ((add_y || ring_x) && !host_ring(M, std::max(ring_x ? ex : 0, add_y ? ey : 0) * sizeof(double)))
+        add_y = ring_x = false;
     if (ring_x) {
         if (st = host_put(M, M->hx, x, nx, nrhs, lx); st != HLRC_OK) return st;
     } else {

@@ -315,8 +315,12 @@ hlrc_status hlrc_mvm(hlrc_hmat M, double alpha, int op, const double* x,
                      double* y, int nrhs, int64_t ldx, int64_t ldy,
                      void* stream);
 
-/* Same with x, y in host memory: copies x and y to the device, runs the
- * product, copies y back, synchronises.  Matches the reference's call on
+/* Same with x, y in host memory; returns when y is complete.  Pageable
+ * vectors pass through a ring of pinned memory that the handle keeps (up to
+ * 2 MiB, allocated by the first such call): x is copied to the device, the
+ * product alone comes back, and the host adds it to y.  Pinned or managed
+ * vectors are copied directly, y both ways.  A call that fails after its
+ * product may leave y partly updated.  Matches the reference's call on
  * host-resident scalar_vectors.  Uses the handle's staging buffers and
  * workspace under a per-handle lock, so concurrent host calls on one handle
  * are correct but run one after the other.                                   */
