@@ -390,10 +390,15 @@ struct DeviceGuard {
     }
 };
 
-#define HLRC_CUDA(call)                                                                          \
-    do {                                                                                         \
-        cudaError_t e_ = (call);                                                                 \
-        if (e_ != cudaSuccess) return fail(HLRC_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
+// A failing call's error is reported here and cleared, so that the launches of a
+// later product are not taken to have failed.
+#define HLRC_CUDA(call)                                                                \
+    do {                                                                               \
+        cudaError_t e_ = (call);                                                       \
+        if (e_ != cudaSuccess) {                                                       \
+            cudaGetLastError();                                                        \
+            return fail(HLRC_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_));       \
+        }                                                                              \
     } while (0)
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -2761,12 +2766,14 @@ extern "C" hlrc_status hlrc_mvm_host(hlrc_hmat M, double alpha, int op, const do
     if (ex > M->hx_elems) {
         cudaFree(M->hx);
         M->hx = nullptr;
+        M->hx_elems = 0;   // should the allocation fail
         HLRC_CUDA(cudaMalloc(&M->hx, std::max<size_t>(ex, 1) * sizeof(double)));
         M->hx_elems = ex;
     }
     if (ey > M->hy_elems) {
         cudaFree(M->hy);
         M->hy = nullptr;
+        M->hy_elems = 0;   // should the allocation fail
         HLRC_CUDA(cudaMalloc(&M->hy, std::max<size_t>(ey, 1) * sizeof(double)));
         M->hy_elems = ey;
     }

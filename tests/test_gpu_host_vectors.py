@@ -4,11 +4,14 @@ pinned slots of 128 KiB, filled in packed order whatever the column length;
 pinned ones are copied directly.  Short columns that share a slot, columns that
 end inside a slot, one column longer than the ring, a ring that grows between
 calls, a leading dimension with padding, and every mix of pageable and pinned."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import hlr_b200 as hlr
 import oracle
+from hlr_b200 import _capi
 
 from conftest import built, relerr
 
@@ -69,5 +72,21 @@ def test_ring_grows_and_mixed_calls():
     for k, px, py in ((1, False, False), (1, True, True), (4, False, False), (2, True, False), (64, False, False),
                       (3, False, True), (1, False, False)):
         _check(M, hm, k, pad=1, px=px, py=py)
+    assert M.device_error() == 0
+    M.free()
+
+
+def test_after_a_call_too_large_for_the_device():
+    """A call whose staging buffers do not fit is refused before it touches its
+    vectors; the next call works."""
+    hm = built("log_300", lambda: hlr.build(hlr.Problem.log1d(300)))
+    M = hlr.upload(hm, max_nrhs=2)
+    _check(M, hm, 2)
+    x, y = np.ones((4, 300)), np.ones((4, 300))
+    st = _capi.lib().hlrc_mvm_host(M.handle, 1.0, 0, C.c_void_p(x.ctypes.data), C.c_void_p(y.ctypes.data),
+                                   100_000_000, 300, 300)          # 240 GB
+    assert st != 0 and np.array_equal(y, np.ones((4, 300)))
+    _check(M, hm, 1)
+    _check(M, hm, 2, pad=1)
     assert M.device_error() == 0
     M.free()
