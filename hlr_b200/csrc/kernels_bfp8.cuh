@@ -138,7 +138,7 @@ __device__ __forceinline__ void stage_bfp(uint8_t* sa, const uint8_t* base, int 
 template <bool I24, bool SP>
 __global__ void __launch_bounds__(TC_WARPS * 32, HLRC_BQ_MINB)
 k_nform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
-            const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
+            const double* vx, const double* vt, OutMap om, double alpha, int add) {
     using O = TcOp<FMT_F16>;
     constexpr int STAGE = I24 ? BQ_STAGE_N24 : BQ_STAGE_N16;
     constexpr int VOFF = I24 ? BQ_PLANE + 32 * BQ_LO_STRIDE : BQ_PLANE;   // vector part of a stage
@@ -146,7 +146,7 @@ k_nform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const 
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
     const MSeg sg = SP ? run_part(segs[blockIdx.x], I24 ? 3 : 2) : segs[blockIdx.x];
-    pdl_wait();
+    pdl_wait(vx, vt);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* ring = smem + warp * (BQ_STAGES * STAGE + (I24 ? BQ_PLANE : 0));
@@ -285,7 +285,7 @@ k_nform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const 
 // its output or FP32 partial slot through the column table.
 template <bool I24>
 __device__ __forceinline__ void ttform_bfp(const MSeg& sg, uint8_t* smem, const MCol* __restrict__ cols,
-                                           const uint8_t* __restrict__ A, const double* __restrict__ vin,
+                                           const uint8_t* __restrict__ A, const double* vin,
                                            const OutMap& om, float* __restrict__ part, double alpha, int add) {
     using O = TcOp<FMT_F16>;
     constexpr int NT = I24 ? 3 : 2;
@@ -303,7 +303,7 @@ __device__ __forceinline__ void ttform_bfp(const MSeg& sg, uint8_t* smem, const 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int row = 16 * kt + 2 * t + (j & 1) + 8 * (j >> 1);
-            const double v = row < sg.rows ? __ldg(vin + size_t(sg.vo + row) * MR_RB + g) : 0.0;
+            const double v = row < sg.rows ? __ldca(vin + size_t(sg.vo + row) * MR_RB + g) : 0.0;
             xv[kt][j] = v;
             E = max(E, dexp(v));
         }
@@ -402,10 +402,10 @@ __device__ __forceinline__ void ttform_bfp(const MSeg& sg, uint8_t* smem, const 
 template <bool I24>
 __global__ void __launch_bounds__(TC_WARPS * 32, HLRC_BQ_MINB)
 k_ttform_bfp(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
-             const double* __restrict__ vin, OutMap om, float* __restrict__ part, double alpha, int add) {
+             const double* vin, OutMap om, float* __restrict__ part, double alpha, int add) {
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(vin);
     ttform_bfp<I24>(run_part(segs[blockIdx.x], I24 ? 3 : 2), smem, cols, A, vin, om, part, alpha, add);
 }
 

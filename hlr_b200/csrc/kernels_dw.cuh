@@ -37,15 +37,15 @@ template <int NT> __device__ __forceinline__ int dw_vec(int n, int t, int e) {
 // columns of X and the writes along the rows of xr
 template <int NT>
 __global__ void __launch_bounds__(256)
-k_dw_rows(const double* __restrict__ X, int64_t ldx, int64_t n, int r0, int nr, double* __restrict__ xr) {
+k_dw_rows(const double* X, int64_t ldx, int64_t n, int r0, int nr, double* __restrict__ xr) {
     constexpr int RB = 8 * NT;
     __shared__ double s[RB][33];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(X);
     const int64_t i0 = int64_t(blockIdx.x) * 32;
     const int lane = threadIdx.x & 31;
     for (int r = threadIdx.x >> 5; r < RB; r += 8)
-        s[r][lane] = r < nr && i0 + lane < n ? X[i0 + lane + int64_t(r0 + r) * ldx] : 0.0;
+        s[r][lane] = r < nr && i0 + lane < n ? __ldca(X + i0 + lane + int64_t(r0 + r) * ldx) : 0.0;
     __syncthreads();
     for (int q = threadIdx.x; q < 32 * RB; q += 256)
         if (i0 + q / RB < n) xr[i0 * RB + q] = s[q % RB][q / RB];
@@ -82,7 +82,7 @@ __device__ __forceinline__ void dw_cp16(uint32_t dst, const void* src, bool ok) 
 template <int NT, bool SP>
 __global__ void __launch_bounds__(DW_WARPS * 32, dw_ctas<NT>())
 k_nform_dw(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
-           const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
+           const double* vx, const double* vt, OutMap om, double alpha, int add) {
     constexpr int RB = 8 * NT, NP = NT / 2, W = DW_WARPS, RS = RB + 1, D = dw_depth<NT>(), BS = dw_bs<NT>();
     constexpr bool ODD = NT % 2 == 1;
     constexpr int VU = RB / 2;   // 16-byte units of a vector row
@@ -160,7 +160,7 @@ k_nform_dw(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, con
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    pdl_wait();
+    pdl_wait(vx, vt);
 #pragma unroll
     for (int d = 0; d < D - 1; ++d) issue_next(d);
     for (int d = 0; c < sg.ce; c += W) {
@@ -222,8 +222,8 @@ template <int NT> constexpr int dw_gsmem() { return GT_TILES * TILE * dw_xs<NT>(
 template <int NT>
 __global__ void __launch_bounds__(DW_GWARPS * 32, 2)
 k_gtform_dw(const GTSeg* __restrict__ segs, const GTChunk* __restrict__ chunks, const GTTile* __restrict__ tiles,
-            const double* __restrict__ A, const double* __restrict__ vin, OutMap om, double* __restrict__ part,
-            double alpha, int add) {
+            const double* __restrict__ A, const double* vin, OutMap om, double* __restrict__ part, double alpha,
+            int add) {
     constexpr int RB = 8 * NT, NP = NT / 2, XS = dw_xs<NT>(), W = DW_GWARPS;
     constexpr bool ODD = NT % 2 == 1;
     constexpr int CH = NT <= 2 ? 2 : 1;   // accumulator sets (even / odd rows): enough independent MMA chains
@@ -232,7 +232,7 @@ k_gtform_dw(const GTSeg* __restrict__ segs, const GTChunk* __restrict__ chunks, 
     const GTSeg sg = segs[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    pdl_wait();
+    pdl_wait(vin);
     for (uint32_t s = 0; s < sg.ntiles; ++s) {
         const GTTile tl = tiles[sg.tile0 + s];
         const double2* src = reinterpret_cast<const double2*>(vin + size_t(tl.v_off) * RB);
@@ -240,7 +240,7 @@ k_gtform_dw(const GTSeg* __restrict__ segs, const GTChunk* __restrict__ chunks, 
         for (int i = threadIdx.x; i < TILE * (RB / 2); i += W * 32) {
             const int row = i / (RB / 2), u = i % (RB / 2);
             *reinterpret_cast<double2*>(dw_sx + (s * TILE + row) * XS + 2 * u) =
-                row < tl.rows ? __ldg(src + i) : make_double2(0.0, 0.0);
+                row < tl.rows ? __ldca(src + i) : make_double2(0.0, 0.0);
         }
     }
     int ld[GT_TILES];
@@ -381,7 +381,7 @@ k_gtform_dw(const GTSeg* __restrict__ segs, const GTChunk* __restrict__ chunks, 
 template <int NT>
 __global__ void __launch_bounds__(256)
 k_tform_dw(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict__ slabs, const double* __restrict__ A,
-           const double* __restrict__ vin, OutMap om, double* __restrict__ part, double alpha, int add) {
+           const double* vin, OutMap om, double* __restrict__ part, double alpha, int add) {
     constexpr int RB = 8 * NT, NG = (NT + 1) / 2;
     pdl_trigger();
     const int wid = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -390,7 +390,7 @@ k_tform_dw(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict_
     const int g = lane >> 2, t = lane & 3;
     const int vg = wid % NG;
     const TUnit u = units[wid / NG];
-    pdl_wait();
+    pdl_wait(vin);
     auto body = [&](auto two) {
         constexpr bool TWO = decltype(two)::value;
         double d[2][2] = {}, f[2][2] = {};
@@ -409,9 +409,9 @@ k_tform_dw(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict_
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const bool ok = row + b < cur.rows;
-                    if constexpr (TWO) v[b] = ok ? __ldg(reinterpret_cast<const double2*>(x + size_t(row + b) * RB))
+                    if constexpr (TWO) v[b] = ok ? __ldca(reinterpret_cast<const double2*>(x + size_t(row + b) * RB))
                                                  : make_double2(0.0, 0.0);
-                    else v[b] = make_double2(ok ? __ldg(x + size_t(row + b) * RB) : 0.0, 0.0);
+                    else v[b] = make_double2(ok ? __ldca(x + size_t(row + b) * RB) : 0.0, 0.0);
                 }
                 dmma(d[0], m.x, v[0].x);
                 dmma(f[0], m.y, v[1].x);
@@ -437,7 +437,7 @@ k_tform_dw(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict_
 // column and vector, 8 columns per group.
 template <int NT>
 __global__ void __launch_bounds__(256)
-k_tfinish_dw(const TGroup* __restrict__ groups, int ngroups, const double* __restrict__ part, OutMap om, double alpha,
+k_tfinish_dw(const TGroup* __restrict__ groups, int ngroups, const double* part, OutMap om, double alpha,
              int add) {
     constexpr int RB = 8 * NT;
     pdl_trigger();
@@ -447,9 +447,9 @@ k_tfinish_dw(const TGroup* __restrict__ groups, int ngroups, const double* __res
     const TGroup g = groups[gi];
     const int c = int(idx / RB) % TCOLS, k = int(idx % RB);
     if (c >= int(g.nc) || k >= om.nr) return;
-    pdl_wait();
+    pdl_wait(part);
     double s = 0.0;
-    for (uint32_t i = 0; i < g.nslots; ++i) s += part[(size_t(g.slot0 + i) * 32 + c) * RB + k];
+    for (uint32_t i = 0; i < g.nslots; ++i) s += __ldca(part + (size_t(g.slot0 + i) * 32 + c) * RB + k);
     double* o = om.base + int64_t(g.out + c) * om.rs + int64_t(k) * om.cs;
     if (add) *o += alpha * s;
     else *o = s;

@@ -24,8 +24,34 @@ __device__ __forceinline__ double2 ld_stream(const double* p) {
 // its static descriptors before pdl_wait, and after pdl_wait (which returns
 // once the preceding kernel has completed and its writes are visible) reads
 // and writes the vectors.  Without the launch attribute both are no-ops.
+//
+// What the wait orders has to be read through pointers that come out of it
+// (pdl_wait(p, ...), past()): the compiler may move a load from a kernel's own
+// read-only pointer argument, and a load by a cache-hint intrinsic, to before an
+// asm statement that does not mention the pointer, "memory" or not.  It did: with
+// other arithmetic after them the x entries of k_ttform_dmma were loaded before
+// the wait, and the second pass of a 17-vector product took the first pass's x.
+// Such loads are ordinary ones (__ldca, __ldcg, __ldcs), never __ldg, whose
+// memory may not change while the kernel runs.
+template <typename T>
+__device__ __forceinline__ T* past(T* p) {
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+template <typename... T>
+__device__ __forceinline__ void pdl_wait(T*&... p) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    ((p = past(p)), ...);
+}
+// o's value for an update through an output pointer argument (*o = ld_out(o) + ...),
+// in its place among the waits; from L2, as another CTA of a launch of several
+// passes may have written it
+__device__ __forceinline__ double ld_out(const double* o) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];\n" : "=d"(v) : "l"(o) : "memory");
+    return v;
+}
 
 // Butterfly transpose-reduction of N per-lane column partials (N = 2^g,
 // g <= 5): at each step a lane keeps one half of its values and trades the
@@ -57,11 +83,11 @@ template <> struct Log2<16> { static constexpr int v = 4; };
 template <> struct Log2<32> { static constexpr int v = 5; };
 
 // A vector entry: through L2 when another CTA of the same launch may have
-// written it (CG), else through the read-only path.
+// written it (CG).  p comes from a pointer past the wait that orders it.
 template <bool CG>
 __device__ __forceinline__ double ld_vec(const double* p) {
     if constexpr (CG) return __ldcg(p);
-    else return __ldg(p);
+    else return __ldca(p);
 }
 
 // The end of an N-form tile: the sum of the W warps' rows in warp order, of the S
@@ -88,7 +114,7 @@ __device__ __forceinline__ void nform_finish(double (&red)[W][TILE], int rows, d
     }
     if (threadIdx.x < rows) {
         double* o = out + threadIdx.x;
-        if (add) *o += alpha * s;
+        if (add) *o = ld_out(o) + alpha * s;
         else *o = s;
     }
 }
@@ -98,8 +124,7 @@ __device__ __forceinline__ void nform_finish(double (&red)[W][TILE], int rows, d
 template <int W, int S = 1>
 __global__ void __launch_bounds__(W * 32)
 k_nform_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
-            const double* __restrict__ vx, const double* __restrict__ vt, double* __restrict__ out, double alpha,
-            int add) {
+            const double* vx, const double* vt, double* __restrict__ out, double alpha, int add) {
     __shared__ double red[W][TILE];
     pdl_trigger();
     const NSeg sg = segs[blockIdx.x / S];
@@ -107,7 +132,7 @@ k_nform_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, co
     const int r = 2 * lane;
     const bool active = r < sg.ld;
     double acc0 = 0.0, acc1 = 0.0;
-    pdl_wait();
+    pdl_wait(vx, vt);
     for (uint32_t c = sg.cb + (blockIdx.x % S) * W + warp; c < sg.ce; c += S * W) {
         const NChunk ch = chunks[c];
         const double* v = (ch.v_off & VEC_T) ? vt + (ch.v_off & ~VEC_T) : vx + ch.v_off;
@@ -119,7 +144,7 @@ k_nform_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, co
             for (int j = 0; j < NCHUNK; ++j) {
                 if (j < ch.nc) {
                     m[j] = ld_stream(a + size_t(j) * sg.ld);
-                    vv[j] = __ldg(v + j);
+                    vv[j] = __ldca(v + j);
                 } else {
                     m[j] = make_double2(0.0, 0.0);
                     vv[j] = 0.0;
@@ -281,7 +306,8 @@ k_ntree_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, Tr
         for (int i = 0; i < nlev; ++i) tree_bar_arrive(&bars[i]);
     // the matrix copies above read static data; the vectors below are
     // written by the preceding kernel
-    pdl_wait();
+    const double* oin = out;
+    pdl_wait(vx, vt, oin);
     for (int e = t.cta_ext[sub] + tid; e < t.cta_ext[sub + 1]; e += W * 32) {
         const TreeExt x = t.ext[e];
         mirror[x.mirror] = __ldcg((x.v_off & VEC_T) ? vt + (x.v_off & ~VEC_T) : vx + x.v_off);
@@ -289,7 +315,7 @@ k_ntree_f64(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, Tr
     if (add)
         for (int gi = 0; gi < nlev; ++gi) {
             for (int q = srun[2 * gi] + warp; q < srun[2 * gi + 1]; q += W)
-                for (int i = lane; i < sseg[q].rows; i += 32) mirror[sseg_m[q] + i] = __ldcg(out + sseg[q].out + i);
+                for (int i = lane; i < sseg[q].rows; i += 32) mirror[sseg_m[q] + i] = __ldcg(oin + sseg[q].out + i);
         }
     cl.sync();   // every CTA of the cluster runs before any writes into its mirror
     const int hw = 2 * warp + (lane >> 4), l16 = lane & 15;
@@ -408,7 +434,7 @@ __device__ __forceinline__ void tform_unit(const TUnit& u, const TSlab* __restri
     if ((lane & ((1 << SH) - 1)) == 0 && c < u.nc) {
         if (u.flags & TU_DIRECT) {
             double* o = out + u.out + c;
-            if (add) *o = (CG ? __ldcg(o) : *o) + alpha * p[0];
+            if (add) *o = ld_out(o) + alpha * p[0];
             else *o = p[0];
         } else {
             part[size_t(u.out) * 32 + c] = p[0];
@@ -419,13 +445,13 @@ __device__ __forceinline__ void tform_unit(const TUnit& u, const TSlab* __restri
 template <int NC>
 __global__ void __launch_bounds__(256)
 k_tform_f64(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict__ slabs,
-            const double* __restrict__ A, const double* __restrict__ vin, double* __restrict__ out,
+            const double* __restrict__ A, const double* vin, double* __restrict__ out,
             double* __restrict__ part, double alpha, int add) {
     pdl_trigger();
     const int wid = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (wid >= nunits) return;
     const TUnit u = units[wid];
-    pdl_wait();
+    pdl_wait(vin);
     tform_unit<NC, false>(u, slabs, A, vin, out, part, alpha, add, threadIdx.x & 31);
 }
 
@@ -436,16 +462,16 @@ k_tform_f64(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict
 template <int W>
 __global__ void __launch_bounds__(W * 32)
 k_ttform_f64(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks, const double* __restrict__ A,
-             const double* __restrict__ vin, double* __restrict__ out, double* __restrict__ part, double alpha,
+             const double* vin, double* __restrict__ out, double* __restrict__ part, double alpha,
              int add) {
     pdl_trigger();
     const TTSeg sg = segs[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = 2 * lane;
     const bool active = r < sg.ld;
-    pdl_wait();
-    const double v0 = (r < sg.rows) ? __ldg(vin + sg.v_off + r) : 0.0;
-    const double v1 = (r + 1 < sg.rows) ? __ldg(vin + sg.v_off + r + 1) : 0.0;
+    pdl_wait(vin);
+    const double v0 = (r < sg.rows) ? __ldca(vin + sg.v_off + r) : 0.0;
+    const double v1 = (r + 1 < sg.rows) ? __ldca(vin + sg.v_off + r + 1) : 0.0;
     // software pipeline: the loads of chunk c + step are issued before chunk c
     // is reduced and written; descriptors are fetched two iterations ahead
     const uint32_t step = W * gridDim.y;
@@ -477,7 +503,7 @@ k_ttform_f64(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks,
         if ((lane & ((1 << SH) - 1)) == 0 && col < ch.nc) {
             if (ch.flags & TT_DIRECT) {
                 double* o = out + ch.out + col;
-                if (add) *o += alpha * p[0];
+                if (add) *o = ld_out(o) + alpha * p[0];
                 else *o = p[0];
             } else {
                 part[ch.out + col] = p[0];
@@ -491,7 +517,7 @@ k_ttform_f64(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks,
 template <bool CG>
 __device__ __forceinline__ void ttfinish_group(const TGroup& g, const double* part, double* out, double alpha, int add,
                                                int lane) {
-    auto ld = [](const double* p) { return CG ? __ldcg(p) : *p; };
+    auto ld = [](const double* p) { return ld_vec<CG>(p); };
     for (uint32_t j = lane; j < g.nc; j += 32) {
         // four interleaved partial sums keep four loads in flight; they are
         // combined in a fixed order, so the result is deterministic
@@ -520,19 +546,19 @@ __device__ __forceinline__ void ttfinish_group(const TGroup& g, const double* pa
         for (; i < g.nslots; ++i) s0 += ld(p + size_t(i) * g.nc);
         const double s = (s0 + s1) + (s2 + s3);
         double* o = out + g.out + j;
-        if (add) *o = ld(o) + alpha * s;
+        if (add) *o = ld_out(o) + alpha * s;
         else *o = s;
     }
 }
 
 __global__ void __launch_bounds__(256)
-k_ttfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* __restrict__ part,
+k_ttfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* part,
                double* __restrict__ out, double alpha, int add) {
     pdl_trigger();
     const int gid = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gid >= ngroups) return;
     const TGroup g = groups[gid];
-    pdl_wait();
+    pdl_wait(part);
     ttfinish_group<false>(g, part, out, alpha, add, threadIdx.x & 31);
 }
 
@@ -541,22 +567,22 @@ template <bool CG>
 __device__ __forceinline__ void tfinish_group(const TGroup& g, const double* part, double* out, double alpha, int add,
                                               int lane) {
     if (lane >= int(g.nc)) return;
-    auto ld = [](const double* p) { return CG ? __ldcg(p) : *p; };
+    auto ld = [](const double* p) { return ld_vec<CG>(p); };
     double s = 0.0;
     for (uint32_t i = 0; i < g.nslots; ++i) s += ld(part + size_t(g.slot0 + i) * 32 + lane);
     double* o = out + g.out + lane;
-    if (add) *o = ld(o) + alpha * s;
+    if (add) *o = ld_out(o) + alpha * s;
     else *o = s;
 }
 
 __global__ void __launch_bounds__(256)
-k_tfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* __restrict__ part,
+k_tfinish_f64(const TGroup* __restrict__ groups, int ngroups, const double* part,
               double* __restrict__ out, double alpha, int add) {
     pdl_trigger();
     const int gid = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gid >= ngroups) return;
     const TGroup g = groups[gid];
-    pdl_wait();
+    pdl_wait(part);
     tfinish_group<false>(g, part, out, alpha, add, threadIdx.x & 31);
 }
 

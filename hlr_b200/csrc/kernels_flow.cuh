@@ -117,6 +117,8 @@ __device__ __forceinline__ void flow_nform(const NSeg& sg, const NChunk* __restr
         load(ch);
     }
     if (!ready()) return;
+    vx = past(vx);
+    vt = past(vt);
     if (c < sg.ce) {
         add_chunk(ch);
         for (c += W; c < sg.ce; c += W) {
@@ -133,7 +135,7 @@ __device__ __forceinline__ void flow_nform(const NSeg& sg, const NChunk* __restr
 #pragma unroll
         for (int w = 0; w < W; ++w) s += red[w][threadIdx.x];
         double* o = out + sg.out + threadIdx.x;
-        if (add) *o = __ldcg(o) + alpha * s;
+        if (add) *o = ld_out(o) + alpha * s;
         else *o = s;
     }
 }
@@ -163,6 +165,7 @@ __device__ __forceinline__ void flow_ttform(const TTSeg& sg, const TTChunk* __re
     issue(cur);
     if (!ready()) return;
     if (c >= sg.ce) return;
+    vin = past(vin);
     const double v0 = (r < sg.rows) ? __ldcg(vin + sg.v_off + r) : 0.0;
     const double v1 = (r + 1 < sg.rows) ? __ldcg(vin + sg.v_off + r + 1) : 0.0;
     for (; c < sg.ce; c += W) {
@@ -181,7 +184,7 @@ __device__ __forceinline__ void flow_ttform(const TTSeg& sg, const TTChunk* __re
         if ((lane & ((1 << SH) - 1)) == 0 && col < ch.nc) {
             if (ch.flags & TT_DIRECT) {
                 double* o = out + ch.out + col;
-                if (add) *o = __ldcg(o) + alpha * p[0];
+                if (add) *o = ld_out(o) + alpha * p[0];
                 else *o = p[0];
             } else {
                 part[ch.out + col] = p[0];
@@ -280,15 +283,17 @@ k_flow_f64(const __grid_constant__ FlowArgs a) {
             static_assert(sizeof(TGroup) == sizeof(TUnit), "one descriptor size");
             if (i < e) g = static_cast<const TGroup*>(p.items)[i];
             const bool go = ready();
+            in = past(in);
+            double* const part = past(a.v[p.vt]);
             while (go && i < e) {
                 if (p.kind == FLOW_FINISH) {
-                    ttfinish_group<true>(g, a.v[p.vt], out, alpha, p.add != 0, lane);
+                    ttfinish_group<true>(g, part, out, alpha, p.add != 0, lane);
                 } else if (p.kind == FLOW_TFINISH) {
-                    tfinish_group<true>(g, a.v[p.vt], out, alpha, p.add != 0, lane);
+                    tfinish_group<true>(g, part, out, alpha, p.add != 0, lane);
                 } else {
                     TUnit u;
                     memcpy(&u, &g, sizeof(u));
-                    tform_unit<TCOLS, true>(u, static_cast<const TSlab*>(p.data), a.A, in, out, a.v[p.vt], alpha, p.add != 0,
+                    tform_unit<TCOLS, true>(u, static_cast<const TSlab*>(p.data), a.A, in, out, part, alpha, p.add != 0,
                                         lane);
                 }
                 i += W;

@@ -23,15 +23,15 @@ namespace hlrc {
 constexpr int MR_RB = 8;   // right-hand sides per block (kernels, finish, workspaces)
 
 // xr[i * RB + r] = X[i + (r0 + r) * ldx] for r < nr, 0 for nr <= r < RB
-__global__ void k_rows_from_cols(const double* __restrict__ X, int64_t ldx, int64_t n, int r0, int nr,
+__global__ void k_rows_from_cols(const double* X, int64_t ldx, int64_t n, int r0, int nr,
                                  double* __restrict__ xr) {
     pdl_trigger();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= n * MR_RB) return;
-    pdl_wait();
+    pdl_wait(X);
     const int64_t i = idx / MR_RB;
     const int r = int(idx % MR_RB);
-    xr[idx] = r < nr ? X[i + int64_t(r0 + r) * ldx] : 0.0;
+    xr[idx] = r < nr ? __ldca(X + i + int64_t(r0 + r) * ldx) : 0.0;
 }
 
 struct OutMap {            // output element (i, r) lives at base[i * rs + r * cs]
@@ -96,7 +96,7 @@ k_ttfinish_flat(const TGroup* __restrict__ groups, int ngroups, int gpb, const T
         pre[ng] = acc;
     }
     __syncthreads();
-    pdl_wait();
+    pdl_wait(part);
     const uint32_t total = pre[ng];
     int lo = 0;   // the group holding item `it` (pre[lo] <= it < pre[lo + 1]); items only move forward
     for (uint32_t it = threadIdx.x; it < total; it += blockDim.x) {
@@ -208,7 +208,7 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 template <int W, bool SP>
 __global__ void __launch_bounds__(W * 32, 2)
 k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
-             const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
+             const double* vx, const double* vt, OutMap om, double alpha, int add) {
     __shared__ double red[W][TILE][MR_RB];
     pdl_trigger();
     const NSeg sg = SP ? seg_part(segs[blockIdx.x]) : segs[blockIdx.x];
@@ -227,7 +227,7 @@ k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, c
         for (int kt = 0; kt < 2; ++kt) {
             const int col = 4 * kt + t;
             const bool okc = col < q.nc;
-            b[kt] = okc ? __ldg(v + size_t(col) * MR_RB + g) : 0.0;
+            b[kt] = okc ? __ldca(v + size_t(col) * MR_RB + g) : 0.0;
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
                 const int row = 16 * p + 2 * g;
@@ -245,7 +245,7 @@ k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, c
             }
     };
     uint32_t c = sg.cb + warp;
-    pdl_wait();
+    pdl_wait(vx, vt);   // before any vector is read: issue() takes these pointers
     if (c < sg.ce) {
         const NChunk none{0, 0, 0, 0};
         double2 mA[2][4], mB[2][4];
@@ -289,12 +289,12 @@ k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, c
 template <int W>
 __global__ void __launch_bounds__(W * 32, 2)
 k_ttform_dmma(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks, const double* __restrict__ A,
-              const double* __restrict__ vin, OutMap om, double* __restrict__ part, double alpha, int add) {
+              const double* vin, OutMap om, double* __restrict__ part, double alpha, int add) {
     pdl_trigger();
     const TTSeg sg = seg_part(segs[blockIdx.x]);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    pdl_wait();
+    pdl_wait(vin);
     // x of the lane: rows 8j + 2t + b (j < 8, b < 2), right-hand side g
     double xv[16];
 #pragma unroll
@@ -302,7 +302,7 @@ k_ttform_dmma(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const int row = 8 * j + 2 * t + b;
-            xv[2 * j + b] = row < sg.rows ? __ldg(vin + size_t(sg.v_off + row) * MR_RB + g) : 0.0;
+            xv[2 * j + b] = row < sg.rows ? __ldca(vin + size_t(sg.v_off + row) * MR_RB + g) : 0.0;
         }
     // operands of one chunk: column g, rows 8j + 2t, +1
     auto issue = [&](const TTChunk& q, double2 (&m)[8]) {

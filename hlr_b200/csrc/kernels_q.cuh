@@ -172,7 +172,7 @@ __device__ __forceinline__ void npack_q(const QNPack& pk, const uint8_t* A, cons
     const uint32_t vo = second ? pk.p[1].v_off : pk.p[0].v_off;
     const float sc = second ? pk.p[1].scale : pk.p[0].scale;
     const double* v = (vo & VEC_T) ? vt + (vo & ~VEC_T) : vx + vo;
-    const float vl = lane < ntot ? float(__ldg(v + (second ? lane - n0 : lane)) * double(sc)) : 0.f;
+    const float vl = lane < ntot ? float(__ldca(v + (second ? lane - n0 : lane)) * double(sc)) : 0.f;
     uint4 m[8];
     uint2 ml[FMT == FMT_I24 ? 8 : 1];
     load_pack<FMT>(A, pk.p[0].a16, pk.p[1].a16, n0, ntot, ld, lane, m, ml);
@@ -242,8 +242,7 @@ __device__ __forceinline__ void nflush_add_q(double* acc, int lane, double* red_
 // of a tile, with the next descriptor read ahead
 template <int W, int FMT>
 __device__ __forceinline__ void npacks_q(uint32_t cb, uint32_t ce, int ld, const QNPack* __restrict__ packs,
-                                         const uint8_t* __restrict__ A, const double* __restrict__ vx,
-                                         const double* __restrict__ vt, int warp, int lane, double* acc) {
+                                         const uint8_t* __restrict__ A, const double* vx, const double* vt, int warp, int lane, double* acc) {
     uint32_t c = cb + warp;
     QNPack nxt{};
     if (c < ce) nxt = ld_pack(packs + c);
@@ -261,14 +260,13 @@ __device__ __forceinline__ void npacks_q(uint32_t cb, uint32_t ce, int ld, const
 template <int W, int WIDE, int F16, int S = 1>
 __global__ void __launch_bounds__(W * 32, W >= 16 ? 1 : 3)
 k_nform_q(const NSeg2* __restrict__ segs, const QNPack* __restrict__ packs, const uint8_t* __restrict__ A,
-          const double* __restrict__ vx, const double* __restrict__ vt, double* __restrict__ out, double alpha,
-          int add) {
+          const double* vx, const double* vt, double* __restrict__ out, double alpha, int add) {
     __shared__ double red[W][TILE];
     pdl_trigger();
     const NSeg2 sg = segs[blockIdx.x / S];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = int(blockIdx.x % S) * W + warp;
-    pdl_wait();
+    pdl_wait(vx, vt);
     if constexpr (WIDE == FMT_I24) {
         // the wide packs flushed before the 16-bit ones start: fewer live
         // registers next to the 24-bit loads
@@ -349,7 +347,7 @@ __device__ __forceinline__ MCol ld_mcol(const MCol* p) {
 // per-column table.
 template <int W, int FMT>
 __device__ __forceinline__ void ttform_qs(const MSeg& sg, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
-                                          const double* __restrict__ vin, double* __restrict__ out,
+                                          const double* vin, double* __restrict__ out,
                                           double* __restrict__ part, double alpha, int add) {
     using F = QFmt<FMT>;
     constexpr int BC = 8 * F::C;   // columns per warp iteration
@@ -360,7 +358,7 @@ __device__ __forceinline__ void ttform_qs(const MSeg& sg, const MCol* __restrict
 #pragma unroll
     for (int r = 0; r < F::R; ++r) {
         const int row = l * F::R + r;
-        xr[r] = row < sg.rows ? float(__ldg(vin + sg.vo + row)) : 0.f;
+        xr[r] = row < sg.rows ? float(__ldca(vin + sg.vo + row)) : 0.f;
     }
     const int ncols = int(sg.ncols);
     const size_t colb = size_t(sg.ld) * fmt_bytes(FMT);
@@ -405,7 +403,7 @@ __device__ __forceinline__ void ttform_qs(const MSeg& sg, const MCol* __restrict
             const double val = double(done.scale) * double(p[0]);
             if (done.idx & MC_DIRECT) {
                 double* o = out + (done.idx & ~MC_DIRECT);
-                if (add) *o += alpha * val;
+                if (add) *o = ld_out(o) + alpha * val;
                 else *o = val;
             } else {
                 part[done.idx] = val;
@@ -422,10 +420,10 @@ __device__ __forceinline__ void ttform_qs(const MSeg& sg, const MCol* __restrict
 template <int W, int WIDE, int F16>
 __global__ void __launch_bounds__(W * 32, 24 / W)
 k_ttform_qs(const MSeg* __restrict__ segs32, int n32, const MSeg* __restrict__ segs16, const MCol* __restrict__ cols,
-            const uint8_t* __restrict__ A, const double* __restrict__ vin, double* __restrict__ out,
-            double* __restrict__ part, double alpha, int add) {
+            const uint8_t* __restrict__ A, const double* vin, double* __restrict__ out, double* __restrict__ part,
+            double alpha, int add) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(vin);
     if (int(blockIdx.x) < n32) ttform_qs<W, WIDE>(segs32[blockIdx.x], cols, A, vin, out, part, alpha, add);
     else ttform_qs<W, F16>(segs16[blockIdx.x - n32], cols, A, vin, out, part, alpha, add);
 }

@@ -279,7 +279,7 @@ __device__ __forceinline__ void nform_store(double* red, int out, int rows, cons
 // B[k][n] = x row k, right-hand side n.
 template <int FMT>
 __device__ __forceinline__ void ttform_tc(const MSeg& sg, uint8_t* smem, const MCol* __restrict__ cols,
-                                          const uint8_t* __restrict__ A, const double* __restrict__ vin,
+                                          const uint8_t* __restrict__ A, const double* vin,
                                           const OutMap& om, float* __restrict__ part, double alpha, int add) {
     using O = TcOp<FMT>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -293,7 +293,7 @@ __device__ __forceinline__ void ttform_tc(const MSeg& sg, uint8_t* smem, const M
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int row = 16 * kt + 2 * t + (j & 1) + 8 * (j >> 1);
-            const double v = row < sg.rows ? __ldg(vin + size_t(sg.vo + row) * MR_RB + g) : 0.0;
+            const double v = row < sg.rows ? __ldca(vin + size_t(sg.vo + row) * MR_RB + g) : 0.0;
             xv[kt][j] = v;
             E = max(E, dexp(v));
         }
@@ -367,12 +367,12 @@ __device__ __forceinline__ void ttform_tc(const MSeg& sg, uint8_t* smem, const M
 template <int FMT, bool SP>
 __global__ void __launch_bounds__(TC_WARPS * 32, HLRC_N16_MINB)
 k_nform_tc(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
-           const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
+           const double* vx, const double* vt, OutMap om, double alpha, int add) {
     using O = TcOp<FMT>;
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
     const MSeg sg = SP ? run_part(segs[blockIdx.x], 2) : segs[blockIdx.x];
-    pdl_wait();
+    pdl_wait(vx, vt);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* ring = smem + warp * (TC_STAGES_N16 * TC_STAGE_N16);
@@ -474,7 +474,7 @@ k_nform_tc(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const u
 
 // Tile T-form: one CTA per input tile; x in FP64 registers; 16-column stages.
 __device__ __forceinline__ void ttform_d32(const MSeg& sg, uint8_t* smem, const MCol* __restrict__ cols,
-                                           const uint8_t* __restrict__ A, const double* __restrict__ vin,
+                                           const uint8_t* __restrict__ A, const double* vin,
                                            const OutMap& om, float* __restrict__ part, double alpha, int add) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -486,7 +486,7 @@ __device__ __forceinline__ void ttform_d32(const MSeg& sg, uint8_t* smem, const 
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const int row = 8 * jj + 2 * t + b;
-            xv[2 * jj + b] = row < sg.rows ? __ldg(vin + size_t(sg.vo + row) * MR_RB + g) : 0.0;
+            xv[2 * jj + b] = row < sg.rows ? __ldca(vin + size_t(sg.vo + row) * MR_RB + g) : 0.0;
         }
     const int colb = sg.ld * 4, ncols = int(sg.ncols);
     const uint8_t* base = A + size_t(sg.a16) * 16;
@@ -536,11 +536,11 @@ __device__ __forceinline__ void ttform_d32(const MSeg& sg, uint8_t* smem, const 
 template <bool SP>
 __global__ void __launch_bounds__(TC_WARPS * 32)
 k_nform_d32(const MSeg* __restrict__ segs, const MCol* __restrict__ cols, const uint8_t* __restrict__ A,
-            const double* __restrict__ vx, const double* __restrict__ vt, OutMap om, double alpha, int add) {
+            const double* vx, const double* vt, OutMap om, double alpha, int add) {
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
     const MSeg sg = SP ? run_part(segs[blockIdx.x], 4) : segs[blockIdx.x];
-    pdl_wait();
+    pdl_wait(vx, vt);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* ring = smem + warp * (TC_STAGES_D32 * TC_STAGE_N32);
@@ -606,11 +606,11 @@ constexpr int TC_STAGE_TT = TC_STAGE_T16 > TC_STAGE_T32 ? TC_STAGE_T16 : TC_STAG
 template <int F16>
 __global__ void __launch_bounds__(TC_WARPS * 32, HLRC_TT_MINB)
 k_ttform_mr(const MSeg* __restrict__ segs32, int n32, const MSeg* __restrict__ segs16, const MCol* __restrict__ cols,
-            const uint8_t* __restrict__ A, const double* __restrict__ vin, OutMap om, float* __restrict__ part,
+            const uint8_t* __restrict__ A, const double* vin, OutMap om, float* __restrict__ part,
             double alpha, int add) {
     extern __shared__ __align__(16) uint8_t smem[];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(vin);
     if (int(blockIdx.x) < n32) ttform_d32(run_part(segs32[blockIdx.x], 4), smem, cols, A, vin, om, part, alpha, add);
     else ttform_tc<F16>(run_part(segs16[blockIdx.x - n32], 2), smem, cols, A, vin, om, part, alpha, add);
 }

@@ -197,14 +197,14 @@ __device__ __forceinline__ bool wide_wait(uint64_t* bar, uint32_t parity, int* e
 // Largest |x| of each vector, one maximum per block: xmax[r * WIDE_XBLOCKS + b]
 constexpr int WIDE_XBLOCKS = 32;
 __global__ void __launch_bounds__(256)
-k_wide_xmax(const double* __restrict__ X, int64_t ldx, int64_t n, double* __restrict__ xmax) {
+k_wide_xmax(const double* X, int64_t ldx, int64_t n, double* __restrict__ xmax) {
     pdl_trigger();
     const int r = blockIdx.y;
-    pdl_wait();
+    pdl_wait(X);
     double m = 0.0;
 #pragma unroll 8
     for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n; i += int64_t(gridDim.x) * 256)
-        m = fmax(m, fabs(X[i + int64_t(r) * ldx]));
+        m = fmax(m, fabs(__ldca(X + i + int64_t(r) * ldx)));
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
     __shared__ double red[8];
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
@@ -218,7 +218,7 @@ k_wide_xmax(const double* __restrict__ X, int64_t ldx, int64_t n, double* __rest
 // g_r = 13 - ilogb(max |x_r|) (0 for a zero vector) of nb blocks' maxima
 __device__ __forceinline__ int wide_xg(const double* xmax, int nb, int r) {
     double m = 0.0;
-    for (int b = 0; b < nb; ++b) m = fmax(m, xmax[r * WIDE_XBLOCKS + b]);
+    for (int b = 0; b < nb; ++b) m = fmax(m, __ldca(xmax + r * WIDE_XBLOCKS + b));
     return m > 0.0 ? 13 - ilogb(m) : 0;
 }
 
@@ -227,13 +227,13 @@ __device__ __forceinline__ int wide_xg(const double* xmax, int nb, int r) {
 // vectors r >= nr are zero.  Also writes g[] (block 0).
 template <int FMT>
 __global__ void __launch_bounds__(256)
-k_wide_xsplit(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, const double* __restrict__ xmax, int nb,
+k_wide_xsplit(const double* X, int64_t ldx, int64_t n, int nr, const double* xmax, int nb,
               uint32_t* __restrict__ xs, int* __restrict__ g) {
     __shared__ double tile[WIDE_RHS][TILE + 1];
     __shared__ double sc[WIDE_RHS];
     pdl_trigger();
     const int64_t i0 = int64_t(blockIdx.x) * TILE;
-    pdl_wait();
+    pdl_wait(X, xmax);
     if (threadIdx.x < WIDE_RHS) {
         const int gr = threadIdx.x < nr ? wide_xg(xmax, nb, threadIdx.x) : 0;
         sc[threadIdx.x] = ldexp(1.0, gr);
@@ -241,7 +241,7 @@ k_wide_xsplit(const double* __restrict__ X, int64_t ldx, int64_t n, int nr, cons
     }
     for (int k = threadIdx.x; k < WIDE_RHS * TILE; k += 256) {
         const int r = k / TILE, i = k % TILE;
-        tile[r][i] = (r < nr && i0 + i < n) ? X[i0 + i + int64_t(r) * ldx] : 0.0;
+        tile[r][i] = (r < nr && i0 + i < n) ? __ldca(X + i0 + i + int64_t(r) * ldx) : 0.0;
     }
     __syncthreads();
     // thread: entry i, vectors 2p, 2p + 1 (p < 32) -> one 8-byte unit of the row
@@ -270,14 +270,14 @@ __device__ __forceinline__ void wide_store_row(double v0, double v1, int e, uint
 // columns one after the other; lane l takes vectors 2l, 2l + 1.
 template <int FMT>
 __global__ void __launch_bounds__(256)
-k_ttfinish_wide(const TGroup* __restrict__ groups, int ngroups, const float* __restrict__ part,
+k_ttfinish_wide(const TGroup* __restrict__ groups, int ngroups, const float* part,
                 uint32_t* __restrict__ ts, const int8_t* __restrict__ texp) {
     pdl_trigger();
     const int gid = int(blockIdx.x) * 8 + int(threadIdx.x >> 5);
     if (gid >= ngroups) return;
     const int lane = threadIdx.x & 31;
     const TGroup gr = groups[gid];
-    pdl_wait();
+    pdl_wait(part);
     const size_t step = size_t(gr.nc) * 32;
     for (uint32_t j = 0; j < gr.nc; ++j) {
         const float2* p = reinterpret_cast<const float2*>(part) + (size_t(gr.slot0) + j) * 32 + lane;
@@ -316,7 +316,7 @@ k_ttfinish_wide(const TGroup* __restrict__ groups, int ngroups, const float* __r
 template <int FMT>
 __global__ void __launch_bounds__(WIDE_THREADS, 4)
 k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, const uint32_t* __restrict__ slabs,
-              const WTTile* __restrict__ tiles, const uint8_t* __restrict__ A, const uint32_t* __restrict__ xs,
+              const WTTile* __restrict__ tiles, const uint8_t* __restrict__ A, const uint32_t* xs,
               uint32_t* __restrict__ ts, const int8_t* __restrict__ texp, float* __restrict__ part, int* err,
               WaitCfg wc) {
     using namespace tc5;
@@ -324,7 +324,7 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
     // a CTA that waits for the kernel before holds no tensor memory yet: CTAs
     // of that kernel may still have to allocate theirs
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(xs);
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     WTBlk* sblk = reinterpret_cast<WTBlk*>(sm + WIDE_NS_C * WIDE_C_STAGE);
@@ -499,15 +499,15 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
 template <int FMT>
 __global__ void __launch_bounds__(WIDE_THREADS, 2)
 k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const uint8_t* __restrict__ A,
-             const uint32_t* __restrict__ xs, const uint32_t* __restrict__ ts, const int* __restrict__ g, OutMap om,
-             double alpha, int add, int* err, WaitCfg wc) {
+             const uint32_t* xs, const uint32_t* ts, const int* g, OutMap om, double alpha, int add, int* err,
+             WaitCfg wc) {
     using namespace tc5;
     using W = WideT<FMT>;
     extern __shared__ uint8_t smem_raw[];
     // a CTA that waits for the kernel before holds no tensor memory yet: CTAs
     // of that kernel may still have to allocate theirs
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(xs, ts, g);
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     uint2* wq = reinterpret_cast<uint2*>(sm + WIDE_NS_N * WIDE_N_STAGE);   // [slot][producer]
@@ -687,7 +687,7 @@ k_nform_wide(const MSeg* __restrict__ segs, const WCol* __restrict__ wcol, const
         }
         ok = __all_sync(0xffffffffu, ok) && !wide_aborted(err);
         if (ok && r < om.nr) {
-            const int rg = g[r];
+            const int rg = __ldca(g + r);
             double* y = om.base + int64_t(r) * om.cs;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {

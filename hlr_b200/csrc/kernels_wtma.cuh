@@ -67,11 +67,11 @@ template <int FMT>
 __global__ void __launch_bounds__(WTMA_THREADS, 4)
 k_nform_wtma(const WSeg* __restrict__ segs, const WStage* __restrict__ stages, const __grid_constant__ CUtensorMap tm_a,
              const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_t,
-             const int* __restrict__ g, OutMap om, double alpha, int* err, WaitCfg wc) {
+             const int* g, OutMap om, double alpha, int* err, WaitCfg wc) {
     using namespace tc5;
     extern __shared__ uint8_t smem_raw[];
     pdl_trigger();   // as in kernels_wide.cuh: before any tensor memory is held
-    pdl_wait();
+    pdl_wait(g);
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     int* snc = reinterpret_cast<int*>(sm + WTMA_NS_N * WIDE_N_STAGE);   // columns per slot
@@ -193,7 +193,7 @@ k_nform_wtma(const WSeg* __restrict__ segs, const WStage* __restrict__ stages, c
         const bool ok = __all_sync(0xffffffffu, wide_wait(tfull, 0u, err, wc.limit_ns)) && !wide_aborted(err);
         if (ok) {
             tc_fence_after();
-            const double fr = r < om.nr ? alpha * ldexp(1.0, sg.E - g[r]) : 0.0;
+            const double fr = r < om.nr ? alpha * ldexp(1.0, sg.E - __ldca(g + r)) : 0.0;
             double* o = om.base + int64_t(sg.out) * om.rs + int64_t(r) * om.cs;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
