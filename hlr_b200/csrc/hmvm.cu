@@ -1267,9 +1267,13 @@ hlrc_status enable_dw_smem(int dev) {
     HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<3>()));
     HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<4>()));
     HLRC_CUDA(cudaFuncSetAttribute(k_nform_dw<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_nsmem<4>()));
-    HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<2>()));
-    HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<3>()));
-    HLRC_CUDA(cudaFuncSetAttribute(k_gtform_dw<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_gsmem<4>()));
+    auto gsmem = [](auto k, int bytes) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+    HLRC_CUDA(gsmem(k_gtform_dw<2, false>, dw_gsmem<2>()));
+    HLRC_CUDA(gsmem(k_gtform_dw<2, true>, dw_gsmem<2>()));
+    HLRC_CUDA(gsmem(k_gtform_dw<3, false>, dw_gsmem<3>()));
+    HLRC_CUDA(gsmem(k_gtform_dw<3, true>, dw_gsmem<3>()));
+    HLRC_CUDA(gsmem(k_gtform_dw<4, false>, dw_gsmem<4>()));
+    HLRC_CUDA(gsmem(k_gtform_dw<4, true>, dw_gsmem<4>()));
     done.push_back(dev);
     return HLRC_OK;
 }
@@ -2132,6 +2136,7 @@ hlrc_status run_dw(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, co
         return OutMap{vec(name), RB, 1, RB};
     };
     const double* A = reinterpret_cast<const double*>(M->store);
+    const bool fine = M->kind != 0 && op != HLRC_OP_N;   // kernels_mr.cuh
     const std::vector<Stage>& stl = mr_stages(M, op);
     thread_local std::vector<int> order;
     for (const int oi : stage_order(M, stl, order)) {
@@ -2165,7 +2170,7 @@ hlrc_status run_dw(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, co
             if (ws.profile) prof_begin(M, stage_name(M, 2, st.idx), tp.alg_bytes, s);
             if constexpr (NT == 1) {
                 if (tp.nsegs[FMT_F64] > 0)
-                    L(launch_k(ov, k_ttform_dmma<DMMA_WARPS>, dim3(unsigned(tp.nsegs[FMT_F64]), unsigned(tp.msplit)), DMMA_WARPS * 32, 0, s,
+                    L(launch_k(ov, fine ? k_ttform_dmma<DMMA_WARPS, true> : k_ttform_dmma<DMMA_WARPS, false>, dim3(unsigned(tp.nsegs[FMT_F64]), unsigned(tp.msplit)), DMMA_WARPS * 32, 0, s,
                                tp.segs[FMT_F64], static_cast<const TTChunk*>(tp.chunks), A, vec(tp.in), om, ws.mr_part,
                                alpha, add));
                 nl += tp.nsegs[FMT_F64] > 0;
@@ -2174,7 +2179,7 @@ hlrc_status run_dw(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, co
                 // CTAs cost the 16-vector adjoint product of an n = 50021 matrix
                 // 50 us of 875
                 if (tp.ngsegs > 0)
-                    L(launch_k(false, k_gtform_dw<NT>, unsigned(tp.ngsegs), DW_GWARPS * 32, dw_gsmem<NT>(), s, tp.gsegs,
+                    L(launch_k(false, fine ? k_gtform_dw<NT, true> : k_gtform_dw<NT, false>, unsigned(tp.ngsegs), DW_GWARPS * 32, dw_gsmem<NT>(), s, tp.gsegs,
                                tp.gchunks, tp.gtiles, A, vec(tp.in), om, ws.mr_part, alpha, add));
                 nl += tp.ngsegs > 0;
             }

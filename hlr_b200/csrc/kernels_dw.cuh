@@ -5,12 +5,22 @@
 // and are bound by HBM; with 32 vectors the same matrix elements feed 32
 // multiply-adds, 8 flop per byte, which is where HBM and the FP64 tensor pipe
 // take about the same time.  Measured, one pass against blocks of 8 (B200):
-// n = 50021 exponential, 16 vectors, adjoint 1.64 -> 0.88 ms, 32 vectors,
-// op N 2.94 -> 1.31 ms; uniform-H sphere of 32768 triangles, 32 vectors
-// 388 -> 165 us.  What bounds the passes: the FP64 tensor pipe and its operand
-// latency at 24 and 32 vectors (19 of 37 TFLOP/s), HBM with the coefficient
-// traffic at 16 (3.6 to 4.2 TB/s of matrix, 0.25 bytes of coefficients more per
-// matrix byte).
+// n = 50021 exponential, 16 vectors, adjoint 1.63 -> 0.95 ms; n = 20011, 32 vectors,
+// op N 1.09 -> 0.52 ms; uniform-H sphere of 32768 triangles, 32 vectors
+// 380 -> 179 us.  What bounds the passes: the FP64 tensor pipe and its operand
+// latency at 24 and 32 vectors, HBM with the coefficient traffic at 16 (0.25
+// bytes of coefficients more per matrix byte).
+//
+// Sums.  An MMA rounds its sum four times; a warp that keeps one sum per output
+// over all its chunks rounds at the size of that sum for each of its matrix
+// columns, and there are half as many warps to an output as in the 8-vector
+// kernels.  So 8 columns (16 with NT = 4) or 8 rows are summed from zero and the
+// result added to the output's sum.  Error of the product against long double,
+// with one sum -> summed apart, and of the 8-vector kernels (1e-16, relative
+// 2-norm): n = 20011 exponential, op N, 32 vectors 10.4 -> 3.3 (7.2), adjoint
+// 5.2 -> 2.3 (3.5); 1D log n = 100003 4.7 -> 2.2 (3.1); uniform-H sphere of 32768
+// triangles 5.4 -> 2.5 (4.0).  It costs 2 adds per 2 MMAs (4 with NT = 4): op N of
+// n = 20011, 16 / 24 / 32 vectors 352 / 409 / 472 -> 355 / 452 / 524 us.
 //
 // Vector blocks are row-major with RB = 8 NT doubles per entry.  A 16-byte
 // load of a vector row serves two tiles: tile 2p + b takes vector
@@ -64,12 +74,19 @@ k_dw_rows(const double* X, int64_t ldx, int64_t n, int r0, int nr, double* __res
 constexpr int DW_WARPS = 4;
 constexpr int DW_AS = TILE * 8 + 32;                                          // matrix column stride, bytes
 template <int NT> constexpr int dw_bs() { return 64 * NT + (NT % 2 ? (NT == 3 ? 96 : 32) : 32); }   // vector column
-template <int NT> constexpr int dw_stage() { return 8 * (DW_AS + dw_bs<NT>()); }
-// Ring depth and CTAs per SM: three CTAs where the accumulators allow it;
-// with 32 vectors two CTAs with deeper rings (three: 826 -> 791 us on 862
-// tiles, but 91 -> 101 us on 512 tiles, whose last wave is then thinner).
-template <int NT> constexpr int dw_depth() { return NT == 3 ? 2 : 3; }
+template <int NT> constexpr int dw_chunk() { return 8 * (DW_AS + dw_bs<NT>()); }
+// Chunks whose products are summed apart before they are added to a tile's sums
+// (a ring slot's), ring depth, CTAs per SM, and whether the vector operands are
+// read again for every 16 rows instead of held in registers.  32 vectors: two
+// chunks halve the adds; op N of n = 20011 exponential / 1D log n = 100003 / uniform-H
+// sphere of 32768 triangles 565 / 290 / 190 us with one, 524 / 282 / 179 with two.
+// 24 vectors: 448 / 208 / 145 us as here, 479 / 244 / 159 with two chunks (and
+// two CTAs, for the registers).
+template <int NT> constexpr int dw_fold() { return NT == 4 ? 2 : 1; }
+template <int NT> constexpr int dw_stage() { return dw_fold<NT>() * dw_chunk<NT>(); }
+template <int NT> constexpr int dw_depth() { return NT == 2 ? 3 : 2; }
 template <int NT> constexpr int dw_ctas() { return NT == 4 ? 2 : 3; }
+template <int NT> constexpr bool dw_vp() { return NT > 2; }
 template <int NT> constexpr int dw_nsmem() {
     constexpr int ring = DW_WARPS * dw_depth<NT>() * dw_stage<NT>(), red = DW_WARPS * TILE * (8 * NT + 1) * 8;
     return ring > red ? ring : red;
@@ -84,6 +101,9 @@ __global__ void __launch_bounds__(DW_WARPS * 32, dw_ctas<NT>())
 k_nform_dw(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, const double* __restrict__ A,
            const double* vx, const double* vt, OutMap om, double alpha, int add) {
     constexpr int RB = 8 * NT, NP = NT / 2, W = DW_WARPS, RS = RB + 1, D = dw_depth<NT>(), BS = dw_bs<NT>();
+    constexpr int F = dw_fold<NT>();
+    constexpr bool VP = dw_vp<NT>();
+    static_assert(D * F <= 4, "the ring's column counts fit 32 bits");
     constexpr bool ODD = NT % 2 == 1;
     constexpr int VU = RB / 2;   // 16-byte units of a vector row
     extern __shared__ __align__(16) double dw_sn[];
@@ -102,72 +122,99 @@ k_nform_dw(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, con
     const NChunk none{0, 0, 0, 0};
     auto desc = [&](uint32_t i) { return i < sg.ce ? chunks[i] : none; };   // nc == 0 past the end
     const bool unit = 2 * lane < sg.ld;      // this lane's 16 bytes of a matrix column exist
-    // copies chunk q into ring slot d: its columns, then its vector rows; the
-    // columns up to the next multiple of 4 are zero-filled
-    auto issue = [&](const NChunk& q, int d) {
+    // copies chunk q to `at`: its columns, then its vector rows; the columns up to
+    // the next multiple of 4 are zero-filled
+    auto issue = [&](const NChunk& q, uint32_t at) {
         const double* v = (q.v_off & VEC_T) ? vt + size_t(q.v_off & ~VEC_T) * RB : vx + size_t(q.v_off) * RB;
         const double* a = A + q.a_off + 2 * lane;
-        const uint32_t sa = ring_s + uint32_t(d) * dw_stage<NT>(), sb = sa + 8 * DW_AS;
+        const uint32_t sb = at + 8 * DW_AS;
         const int up = (q.nc + 3) & ~3;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (j < up && unit) dw_cp16(sa + j * DW_AS + lane * 16, j < q.nc ? a + size_t(j) * sg.ld : A, j < q.nc);
+            if (j < up && unit) dw_cp16(at + j * DW_AS + lane * 16, j < q.nc ? a + size_t(j) * sg.ld : A, j < q.nc);
 #pragma unroll
         for (int k = 0; k < 8 * VU / 32; ++k) {
             const int u = 32 * k + lane, j = u / VU;
             if (j < up) dw_cp16(sb + j * BS + (u % VU) * 16, j < q.nc ? v + 2 * u : A, j < q.nc);
         }
     };
-    auto compute = [&](int nc, int d) {
+    // the F chunks of slot d, ncs: their columns, 8 bits each.  A k-step takes four
+    // columns; FULL (one chunk a slot): it has two of them
+    auto compute = [&](uint32_t ncs, int d) {
         const uint8_t* sa = ring + d * dw_stage<NT>() + t * DW_AS + g * 16;
         const uint8_t* sb = ring + d * dw_stage<NT>() + 8 * DW_AS + t * BS;
+        auto step = [&](int k) { return (int(ncs >> (8 * (k >> 1))) & 0xff) > 4 * (k & 1); };   // is there a k-step k?
+        auto body = [&](auto full) {
+            constexpr bool FULL = decltype(full)::value;
+            double v[VP ? 1 : 2 * F][NT];
+            auto load = [&](int k, double (&o)[NT]) {   // the vector operand of k-step k
+                const uint8_t* q = sb + (k >> 1) * dw_chunk<NT>() + 4 * (k & 1) * BS;
 #pragma unroll
-        for (int kt = 0; kt < 2; ++kt) {
-            if (nc <= 4 * kt) break;
-            double2 v[NP > 0 ? NP : 1];
-            double vo = 0.0;
+                for (int h = 0; h < NP; ++h) {
+                    const double2 w = *reinterpret_cast<const double2*>(q + 128 * h + 16 * g);
+                    o[2 * h] = w.x;
+                    o[2 * h + 1] = w.y;
+                }
+                if constexpr (ODD) o[NT - 1] = *reinterpret_cast<const double*>(q + 128 * NP + 8 * g);
+            };
+            if constexpr (!VP) {
 #pragma unroll
-            for (int h = 0; h < NP; ++h) v[h] = *reinterpret_cast<const double2*>(sb + 4 * kt * BS + 128 * h + 16 * g);
-            if constexpr (ODD) vo = *reinterpret_cast<const double*>(sb + 4 * kt * BS + 128 * NP + 8 * g);
+                for (int k = 0; k < 2 * F; ++k)
+                    if (FULL || step(k)) load(k, v[k]);
+            }
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
                 if (p >= np) break;
-                const double2 m = *reinterpret_cast<const double2*>(sa + 4 * kt * DW_AS + 128 * p);
+                double s[2][NT][2];
 #pragma unroll
-                for (int h = 0; h < NP; ++h) {
-                    dmma(acc[2 * p][2 * h], m.x, v[h].x);
-                    dmma(acc[2 * p + 1][2 * h], m.y, v[h].x);
-                    dmma(acc[2 * p][2 * h + 1], m.x, v[h].y);
-                    dmma(acc[2 * p + 1][2 * h + 1], m.y, v[h].y);
+                for (int k = 0; k < 2 * F; ++k) {
+                    if (k > 0 && !FULL && !step(k)) continue;
+                    const double2 m = *reinterpret_cast<const double2*>(sa + (k >> 1) * dw_chunk<NT>() +
+                                                                        4 * (k & 1) * DW_AS + 128 * p);
+                    if constexpr (VP) load(k, v[0]);
+#pragma unroll
+                    for (int n = 0; n < NT; ++n)
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            if (k == 0) dmma0(s[b][n], b ? m.y : m.x, v[0][n]);
+                            else dmma(s[b][n], b ? m.y : m.x, v[VP ? 0 : k][n]);
+                        }
                 }
-                if constexpr (ODD) {
-                    dmma(acc[2 * p][NT - 1], m.x, vo);
-                    dmma(acc[2 * p + 1][NT - 1], m.y, vo);
-                }
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+                        acc[2 * p + b][n][0] += s[b][n][0], acc[2 * p + b][n][1] += s[b][n][1];
             }
-        }
+        };
+        if (F == 1 && step(1)) body(std::true_type{});
+        else body(std::false_type{});
     };
     uint32_t c = sg.cb + warp;
-    uint32_t ncs = 0;   // columns of the chunks in the ring, 8 bits per slot
+    uint32_t ncs = 0;   // columns of the chunks in the ring, 8 bits per chunk
     NChunk q = desc(c);
     uint32_t ci = c;    // the chunk q describes, the next one to issue
     auto issue_next = [&](int d) {
-        if (ci < sg.ce) {
-            ncs = (ncs & ~(0xffu << (8 * d))) | (uint32_t(q.nc) << (8 * d));
-            issue(q, d);
-            ci += W;
-            q = desc(ci);
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            const int at = 8 * (d * F + f);
+            ncs = (ncs & ~(0xffu << at)) | (uint32_t(q.nc) << at);
+            if (ci < sg.ce) {
+                issue(q, ring_s + uint32_t(d * dw_stage<NT>() + f * dw_chunk<NT>()));
+                ci += W;
+                q = desc(ci);
+            }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
     pdl_wait(vx, vt);
 #pragma unroll
     for (int d = 0; d < D - 1; ++d) issue_next(d);
-    for (int d = 0; c < sg.ce; c += W) {
+    for (int d = 0; c < sg.ce; c += F * W) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 2) : "memory");
         __syncwarp();    // the slot's copies of all lanes landed, and every lane is done with the slot before it
         issue_next(d == 0 ? D - 1 : d - 1);
-        compute((ncs >> (8 * d)) & 0xff, d);
+        compute(ncs >> (8 * F * d), d);
         d = d == D - 1 ? 0 : d + 1;
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -219,14 +266,14 @@ constexpr int DW_GWARPS = 8;
 template <int NT> constexpr int dw_xs() { return 8 * NT + 2; }
 template <int NT> constexpr int dw_gsmem() { return GT_TILES * TILE * dw_xs<NT>() * 8; }
 
-template <int NT>
+template <int NT, bool FINE>
 __global__ void __launch_bounds__(DW_GWARPS * 32, 2)
 k_gtform_dw(const GTSeg* __restrict__ segs, const GTChunk* __restrict__ chunks, const GTTile* __restrict__ tiles,
             const double* __restrict__ A, const double* vin, OutMap om, double* __restrict__ part, double alpha,
             int add) {
     constexpr int RB = 8 * NT, NP = NT / 2, XS = dw_xs<NT>(), W = DW_GWARPS;
     constexpr bool ODD = NT % 2 == 1;
-    constexpr int CH = NT <= 2 ? 2 : 1;   // accumulator sets (even / odd rows): enough independent MMA chains
+    constexpr int CH = NT <= 2 && !FINE ? 2 : 1;   // sets of sums, for alternate groups of 8 rows
     extern __shared__ __align__(16) double dw_sx[];   // [tile][row][XS]
     pdl_trigger();
     const GTSeg sg = segs[blockIdx.x];
@@ -296,21 +343,36 @@ k_gtform_dw(const GTSeg* __restrict__ segs, const GTChunk* __restrict__ chunks, 
 #pragma unroll
         for (int k = 1; k < GT_TILES; ++k)
             if (s == k) l = ld[k];
+        double f[NT][2];   // FINE: the sums of this slab
 #pragma unroll
         for (int j = 0; j < 8; ++j) {   // rows past the tile: zero x and zero matrix entries
             if (8 * j >= l) break;
+            const double *x0 = x + 8 * j * XS, *x1 = x0 + XS;
+            double e[NT][2];
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const double a = b ? m[j].y : m[j].x;
-                const double* xr = x + (8 * j + b) * XS;
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const double2 v = *reinterpret_cast<const double2*>(xr + 16 * p + 2 * g);
-                    dmma(d[b % CH][2 * p], a, v.x);
-                    dmma(d[b % CH][2 * p + 1], a, v.y);
-                }
-                if constexpr (ODD) dmma(d[b % CH][NT - 1], a, xr[16 * NP + g]);
+            for (int p = 0; p < NP; ++p) {
+                const double2 v = *reinterpret_cast<const double2*>(x0 + 16 * p + 2 * g);
+                dmma0(e[2 * p], m[j].x, v.x);
+                dmma0(e[2 * p + 1], m[j].x, v.y);
             }
+            if constexpr (ODD) dmma0(e[NT - 1], m[j].x, x0[16 * NP + g]);
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                const double2 v = *reinterpret_cast<const double2*>(x1 + 16 * p + 2 * g);
+                dmma(e[2 * p], m[j].y, v.x);
+                dmma(e[2 * p + 1], m[j].y, v.y);
+            }
+            if constexpr (ODD) dmma(e[NT - 1], m[j].y, x1[16 * NP + g]);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                if constexpr (!FINE) d[j % CH][n][0] += e[n][0], d[j % CH][n][1] += e[n][1];
+                else if (j == 0) f[n][0] = e[n][0], f[n][1] = e[n][1];
+                else f[n][0] += e[n][0], f[n][1] += e[n][1];
+            }
+        }
+        if constexpr (FINE) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) d[0][n][0] += f[n][0], d[0][n][1] += f[n][1];
         }
     };
     auto store = [&](const GTChunk& q) {
@@ -413,12 +475,8 @@ k_tform_dw(const TUnit* __restrict__ units, int nunits, const TSlab* __restrict_
                                                  : make_double2(0.0, 0.0);
                     else v[b] = make_double2(ok ? __ldca(x + size_t(row + b) * RB) : 0.0, 0.0);
                 }
-                dmma(d[0], m.x, v[0].x);
-                dmma(f[0], m.y, v[1].x);
-                if constexpr (TWO) {
-                    dmma(d[1], m.x, v[0].y);
-                    dmma(f[1], m.y, v[1].y);
-                }
+                dmma8(j & 1 ? f[0] : d[0], m.x, v[0].x, m.y, v[1].x);
+                if constexpr (TWO) dmma8(j & 1 ? f[1] : d[1], m.x, v[0].y, m.y, v[1].y);
             }
         }
 #pragma unroll

@@ -202,6 +202,31 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
         : "d"(a), "d"(b));
 }
 
+// d = a b
+__device__ __forceinline__ void dmma0(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};\n"
+        : "=d"(d[0]), "=d"(d[1])
+        : "d"(a), "d"(b), "d"(0.0));
+}
+// acc += a0 b0 + a1 b1 (two k-steps), the eight products summed apart and added
+// once: a chain of n terms in steps of eight rounds n / 8 times at the size of
+// the sum instead of n times.
+__device__ __forceinline__ void dmma8(double (&acc)[2], double a0, double b0, double a1, double b1) {
+    double d[2];
+    dmma0(d, a0, b0);
+    dmma(d, a1, b1);
+    acc[0] += d[0];
+    acc[1] += d[1];
+}
+
+// FINE (here and in k_gtform_dw): shorter chains of a column's sum, for the adjoint
+// products of uniform-H and H^2 matrices, which go one vector at a time through
+// the sums over lanes of the one-vector kernels where there is no block to
+// share a pass.  Error of the 8-vector adjoint of a uniform-H sphere of 32768
+// triangles against long double: 3.6e-16 with one chain, 2.3e-16 with four,
+// one vector at a time 2.1e-16; 32 vectors: 2.7e-16, 2.2e-16 FINE.  Elsewhere the
+// chains cost more than they give: n = 20011 exponential, 8 vectors, adjoint 288 us,
+// FINE 294; 32 vectors 548 us (the T-form 220), FINE 305 of T-form.
 // Both kernels keep two operand sets in registers: the loads of chunk
 // c + W are in flight while chunk c is multiplied, and chunk descriptors are
 // read two chunks ahead.
@@ -286,7 +311,7 @@ k_nform_dmma(const NSeg* __restrict__ segs, const NChunk* __restrict__ chunks, c
         [&](int row, int kk) { return &red[0][row][kk]; });
 }
 
-template <int W>
+template <int W, bool FINE>
 __global__ void __launch_bounds__(W * 32, 2)
 k_ttform_dmma(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks, const double* __restrict__ A,
               const double* vin, OutMap om, double* __restrict__ part, double alpha, int add) {
@@ -315,12 +340,16 @@ k_ttform_dmma(const TTSeg* __restrict__ segs, const TTChunk* __restrict__ chunks
         }
     };
     auto finish = [&](const TTChunk& q, const double2 (&m)[8]) {
-        double d[2] = {0.0, 0.0};
+        constexpr int CH = FINE ? 4 : 1;   // chains of 64 / CH rows
+        double f[CH][2];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            dmma(d, m[j].x, xv[2 * j]);
-            dmma(d, m[j].y, xv[2 * j + 1]);
+            if (j < CH) dmma0(f[j % CH], m[j].x, xv[2 * j]);
+            else dmma(f[j % CH], m[j].x, xv[2 * j]);
+            dmma(f[j % CH], m[j].y, xv[2 * j + 1]);
         }
+        double d[2] = {f[0][0], f[0][1]};
+        if constexpr (FINE) d[0] = (d[0] + f[1][0]) + (f[2][0] + f[3][0]), d[1] = (d[1] + f[1][1]) + (f[2][1] + f[3][1]);
         // d[e]: chunk column g, right-hand side 2t + e
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
