@@ -480,6 +480,10 @@ struct PlanKnobs {
     // 2 H^2), unless the caller asks for it fused
     bool side_dense(int /*kind*/) const { return near_field != 1; }
     bool blocks = false;           // build the group T-forms (FP64, max_nrhs > 8)
+    // elements that the chunks of one group segment lie apart at most: their 32-bit
+    // offsets count pairs from the segment's base, GT_NONE excluded (64 GiB; tiles of
+    // a wide dense block can lie further apart)
+    uint64_t group_span = 2 * uint64_t(GT_NONE);
 };
 thread_local PlanKnobs g_knobs;
 struct KnobScope {
@@ -561,6 +565,9 @@ struct TTBuilder {
             const GRef& r = gref[o.first + q];
             same = r.id == id && r.j == uint32_t(cols[q].col0 - lo) && P.gchunks[o.first + q].nc == cols[q].nc &&
                    goff[o.first + q][at] == ~uint64_t(0);
+            const uint64_t b = uint64_t(cols[q].byte_off) / sizeof(double);
+            for (const uint64_t a : goff[o.first + q])   // and lies within the reach of its offsets
+                same = same && (a == ~uint64_t(0) || (a < b ? b - a : a - b) < g_knobs.group_span);
         }
         if (!same) {
             o.group = group;
@@ -606,10 +613,15 @@ struct TTBuilder {
         for (size_t c = 0; c < gref.size();) {
             size_t e = c;
             int64_t b = 0;
-            uint64_t base = ~uint64_t(0);
+            uint64_t base = ~uint64_t(0), top = 0;
             for (; e < gref.size() && gref[e].group == gref[c].group && (e == c || b < target); ++e) {
+                uint64_t lo = base, hi = top;
+                for (const uint64_t o : goff[e])
+                    if (o != ~uint64_t(0)) lo = std::min(lo, o), hi = std::max(hi, o);
+                if (e > c && hi - lo >= g_knobs.group_span) break;
+                base = lo;
+                top = hi;
                 b += by[e];
-                for (size_t a = 0; a < GT_TILES; ++a) base = std::min(base, goff[e][a]);
             }
             const size_t t0 = size_t(gref[c].group) * GT_TILES;
             segs.push_back({b, GTSeg{base, uint32_t(c), uint32_t(e), uint32_t(t0),
@@ -618,7 +630,7 @@ struct TTBuilder {
                 for (size_t a = 0; a < GT_TILES; ++a) {
                     const uint64_t o = goff[k][a];
                     if (o == ~uint64_t(0)) continue;
-                    P.gchunks[k].a[a] = uint32_t(std::min<uint64_t>((o - base) / 2, GT_NONE));
+                    P.gchunks[k].a[a] = uint32_t((o - base) / 2);
                 }
             c = e;
         }
