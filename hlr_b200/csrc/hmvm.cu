@@ -1512,10 +1512,26 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
 
     fill_info(p, L, hp->info);
     plan_flow(hp);
+    // Without room for the group T-forms' tables, products of more than 8 vectors
+    // go in blocks of 8.
+    const int64_t no_groups = hp->info.device_bytes;
+    auto drop_groups = [&]() {
+        cudaFree(hp->mr_tables);
+        hp->mr_tables = nullptr;
+        hp->blocks = false;
+        hp->info.device_bytes = no_groups;
+        for (DevTTPass& d : hp->tt) {
+            d.gsegs = nullptr;
+            d.ngsegs = d.nggroups = d.nggroups1 = 0;
+        }
+    };
     if (p.blocks) {
         hlrc_status st = enable_dw_smem(dev);
         if (st == HLRC_OK) st = upload_groups(p, hp);
-        if (st != HLRC_OK) {
+        if (st == HLRC_ERR_OOM) {
+            drop_groups();
+            clear_error();
+        } else if (st != HLRC_OK) {
             cudaFree(hp->mr_tables);
             cleanup();
             return st;
@@ -1525,14 +1541,16 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
     // floating point (BFP) stores loop the one-vector kernels instead
     if (o.max_nrhs > 1 && has_multi_kernels(hp)) {
         // where the arrays of the widest blocks do not fit, narrower ones do
-        // the same product in more passes
+        // the same product in more passes, the narrowest without the tables
         MrSizes z;
-        for (int nt = mr_tiles(hp, o.max_nrhs); nt >= 1; --nt) {
+        for (int nt = mr_tiles(hp, o.max_nrhs);;) {
             z = mr_sizes(hp, nt);
             hp->mr_nt = nt;
             e = cudaMalloc(&hp->mr_arena, z.bytes);
-            if (e != cudaErrorMemoryAllocation) break;
-            if (nt > 1) cudaGetLastError();
+            if (e != cudaErrorMemoryAllocation || (nt == 1 && !hp->blocks)) break;
+            cudaGetLastError();
+            if (nt > 1) --nt;
+            else drop_groups();
         }
         if (e != cudaSuccess) {
             cudaGetLastError();
