@@ -262,22 +262,25 @@ class DeviceMatrix:
         nform_warps, ttform_warps (4, 8 or 16), mr_min_nrhs, wide_min_nrhs,
         overlap (programmatic dependent launch of the one-vector kernels) and
         side_at (how many other passes launch before the near field's side
-        pass is forked)."""
+        pass is forked).  8 warps are a choice per pass unless exact_warps,
+        listed where it is set, is 1."""
         t = _capi.hlrc_tuning()
         check(lib().hlrc_get_tuning(self._h, C.byref(t)), "hlrc_get_tuning")
-        return {"nform_warps": t.nform_warps, "ttform_warps": t.ttform_warps, "mr_min_nrhs": t.mr_min_nrhs,
-                "wide_min_nrhs": t.wide_min_nrhs, "overlap": t.overlap, "side_at": t.side_at}
+        d = {"nform_warps": t.nform_warps, "ttform_warps": t.ttform_warps, "mr_min_nrhs": t.mr_min_nrhs,
+             "wide_min_nrhs": t.wide_min_nrhs, "overlap": t.overlap, "side_at": t.side_at}
+        return dict(d, exact_warps=1) if t.exact_warps else d
 
     def set_tuning(self, **kw) -> None:
         """Changes some launch shapes (hlrc_set_tuning); the others keep their
         values.  Invalid values raise HLRCError (HLRC_ERR_ARG)."""
         cur = self.tuning
-        unknown = set(kw) - set(cur)
+        unknown = set(kw) - set(cur) - {"exact_warps"}
         if unknown:
             raise ValueError(f"unknown tuning keys {sorted(unknown)}")
         cur.update(kw)
         t = _capi.hlrc_tuning(int(cur["nform_warps"]), int(cur["ttform_warps"]), int(cur["mr_min_nrhs"]),
-                              int(cur["wide_min_nrhs"]), int(cur["overlap"]), int(cur["side_at"]))
+                              int(cur["wide_min_nrhs"]), int(cur["overlap"]), int(cur["side_at"]),
+                              int(cur.get("exact_warps", 0)))
         check(lib().hlrc_set_tuning(self._h, C.byref(t)), "hlrc_set_tuning")
 
     def launch_count(self) -> int:

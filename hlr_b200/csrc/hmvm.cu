@@ -337,6 +337,8 @@ struct hlrc_hmat_s {
     int wide_min_nrhs = MR_RB + 1;   // fewest vectors that take the 64-vector kernels (when the handle has them)
     int overlap = 1;          // one-vector kernels launched with programmatic dependent launch
     int side_at = 0;          // side stages forked after this many other stages
+    int exact_warps = 0;      // 8 warps as they are, not chosen per pass
+    bool per_pass(int warps) const { return warps == 8 && !exact_warps; }
     // profiling
     bool profiling = false;
     std::vector<ProfileRec> prof;
@@ -1963,7 +1965,7 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
         const int add = tp.mode != OUT_SET;
         const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
         if (ws.profile) prof_begin(M, stage_name(M, 2, idx), tp.alg_bytes, s);
-        const unsigned ts = M->ttform_warps == 8 ? unsigned(tp.split) : 1u;   // CTAs per tile
+        const unsigned ts = M->per_pass(M->ttform_warps) ? unsigned(tp.split) : 1u;   // CTAs per tile
         auto ttform = [&](auto wc) {
             constexpr int TW = decltype(wc)::value;
             if (f64plan && tp.nsegs[FMT_F64] > 0)
@@ -1991,7 +1993,7 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
                 }
             }
         };
-        const int tw = M->ttform_warps == 8 ? tp.warps : M->ttform_warps;
+        const int tw = M->per_pass(M->ttform_warps) ? tp.warps : M->ttform_warps;
         if (tw == 4) ttform(Warps<4>{});
         else if (tw == 16) ttform(Warps<16>{});
         else ttform(Warps<8>{});
@@ -2092,8 +2094,8 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
                                    M->store, vx, vt, vo, alpha, add));
                 }
             };
-            const int nw = M->nform_warps == 8 ? np.warps : M->nform_warps;
-            const int ns = M->nform_warps == 8 ? np.split : 1;
+            const int nw = M->per_pass(M->nform_warps) ? np.warps : M->nform_warps;
+            const int ns = M->per_pass(M->nform_warps) ? np.split : 1;
             if (ns == 4) nform(Warps<8>{}, Warps<4>{});
             else if (ns == 2) nform(Warps<8>{}, Warps<2>{});
             else if (nw == 4) nform(Warps<4>{}, Warps<1>{});
@@ -2848,6 +2850,7 @@ extern "C" hlrc_status hlrc_get_tuning(hlrc_hmat M, hlrc_tuning* t) {
     t->wide_min_nrhs = M->wide_min_nrhs;
     t->overlap = M->overlap;
     t->side_at = M->side_at;
+    t->exact_warps = M->exact_warps;
     return HLRC_OK;
 }
 
@@ -2874,6 +2877,7 @@ extern "C" hlrc_status hlrc_set_tuning(hlrc_hmat M, const hlrc_tuning* t) {
     M->wide_min_nrhs = t->wide_min_nrhs;
     M->overlap = t->overlap;
     M->side_at = t->side_at;
+    M->exact_warps = t->exact_warps == 1;
     return HLRC_OK;
 }
 

@@ -5,7 +5,7 @@ candidate settings of ``hlrc_tuning`` on the current device and keeps the
 fastest:
 
 * one vector: warps per CTA (4, 8 or 16) of the N-form and of the tile
-  T-form kernels, nine combinations;
+  T-form kernels, nine combinations (8, the default, is a choice per pass);
 * several vectors: the 8-vector tensor-core kernels against a loop of
   one-vector products (``mr_min_nrhs`` 2 or ``HLRC_MR_NEVER``); with more
   than 8 vectors also the one-pass 64-vector kernels of 16-bit stores

@@ -392,9 +392,11 @@ hlrc_status hlrc_workspace_free(hlrc_workspace ws);
  * per-warp partial sums differs, so results agree to rounding).
  *   nform_warps, ttform_warps: warps per CTA (4, 8 or 16) of the one-vector
  *     N-form and tile T-form kernels (16 for small matrices, where each
- *     output tile's chain of loads sets the time).  8 is the default: FP64
- *     passes whose tiles hold few or many columns then take 4 or 16, chosen at
- *     upload;
+ *     output tile's chain of loads sets the time).  8 is the default and a
+ *     choice per pass, made at upload: FP64 passes whose tiles hold few or
+ *     many columns take 4 or 16, and passes of few, heavy tiles several CTAs
+ *     a tile; with exact_warps = 1 it is 8 warps, one CTA a tile.  4 and 16
+ *     are taken as they are, one CTA a tile;
  *   mr_min_nrhs: products with at least this many vectors use the
  *     8-vector tensor-core kernels, smaller ones loop the one-vector kernels
  *     (2..HLRC_MR_NEVER; HLRC_MR_NEVER always loops);
@@ -420,7 +422,8 @@ typedef struct hlrc_tuning {
      * launched (0 = at the start; 0..16, clamped to the pass that adds the
      * low-rank part to y).  Results do not depend on it.                   */
     int32_t side_at;
-    int32_t reserved[2];
+    int32_t exact_warps;   /* 1: 8 warps are 8 warps; 0 (default): chosen per pass */
+    int32_t reserved[1];
 } hlrc_tuning;
 
 hlrc_status hlrc_get_tuning(hlrc_hmat M, hlrc_tuning* t);
