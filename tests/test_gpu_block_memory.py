@@ -2,7 +2,8 @@
 the block kernels, or only with narrower blocks, still works: its products go in
 blocks of fewer vectors.  The device is filled up to what the same matrix needs
 for 8 vectors and a little more."""
-import numpy as np
+import ctypes as C
+
 import pytest
 
 import hlr_b200 as hlr
@@ -16,15 +17,17 @@ pytestmark = pytest.mark.gpu
 MB = 1 << 20
 
 
-def _fill(leave):
-    """Tensors that leave about `leave` bytes of the device free (not below)."""
+def _fill(cudart, leave):
+    """Allocations (of the runtime itself: torch rounds its own up) that leave `leave`
+    bytes of the device free, or up to 2 MB more."""
     hold = []
     for step in (1 << 33, 1 << 30, 1 << 26, 2 * MB):
         while torch.cuda.mem_get_info()[0] - leave >= step:
-            try:
-                hold.append(torch.empty(step, dtype=torch.uint8, device="cuda"))
-            except torch.OutOfMemoryError:
+            p = C.c_void_p()
+            if cudart.cudaMalloc(C.byref(p), C.c_size_t(step)) != 0:
+                cudart.cudaGetLastError()
                 break
+            hold.append(p)
     return hold
 
 
@@ -57,11 +60,14 @@ def test_upload_beside_a_full_device():
     assert tables > 8 * MB                   # so that they do not fit in the margin below
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
-    hold = _fill(need[8] + 4 * MB)
-    M = hlr.upload(hm, max_nrhs=24)
+    cudart = C.CDLL("/usr/local/cuda/lib64/libcudart.so")
+    hold = _fill(cudart, need[8] + 4 * MB)
+    try:
+        M = hlr.upload(hm, max_nrhs=24)
+    finally:
+        for p in hold:
+            cudart.cudaFree(p)
     assert M.info["device_bytes"] < info[24]["device_bytes"] - tables // 2
-    del hold
-    torch.cuda.empty_cache()
     for y, r in zip(product(M), ref):
         assert float((y - r).norm() / r.norm()) <= 1e-13
     assert M.device_error() == 0
