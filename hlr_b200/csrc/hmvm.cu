@@ -42,15 +42,10 @@ struct DevTPass {
     const TUnit* units = nullptr;
     const TSlab* slabs = nullptr;
     const TGroup* groups = nullptr;
-    int cls_begin[4] = {0, 0, 0, 0};
-    int ngroups = 0;
+    int nunits = 0, ngroups = 0;
     int in = V_X, out = V_T, mode = OUT_SET;
     int64_t bytes = 0, alg_bytes = 0;
-    int launches() const {
-        int n = ngroups > 0 ? 1 : 0;
-        for (int c = 0; c < 3; ++c) n += cls_begin[c + 1] > cls_begin[c] ? 1 : 0;
-        return n;
-    }
+    int launches() const { return (nunits > 0 ? 1 : 0) + (ngroups > 0 ? 1 : 0); }
 };
 
 struct DevNPass {
@@ -538,8 +533,7 @@ int plan_launches(const Plan& p, int op) {
     for (const Stage& st : p.stages_nf[op].empty() ? p.stages[op] : p.stages_nf[op]) {
         if (st.kind == 0) {
             const TPass& t = p.tpasses[size_t(st.idx)];
-            n += t.groups.empty() ? 0 : 1;
-            for (int c = 0; c < 3; ++c) n += t.cls_begin[c + 1] > t.cls_begin[c] ? 1 : 0;
+            n += (t.units.empty() ? 0 : 1) + (t.groups.empty() ? 0 : 1);
         } else if (st.kind == 1) {
             const NPass& q = p.npasses[size_t(st.idx)];
             const int k = formats(q.segs);
@@ -1200,8 +1194,7 @@ void plan_flow(hlrc_hmat_s* h) {
                 push(FLOW_FINISH, tp.groups, nullptr, tp.ngroups, false, tp.in, part, tp.out, tp.mode);
             } else {
                 const DevTPass& tp = h->t[size_t(st.idx)];
-                ok = ok && tp.cls_begin[1] == tp.cls_begin[3];   // 8-column units only
-                push(FLOW_T, tp.units, tp.slabs, tp.cls_begin[3], false, tp.in, 4, tp.out, tp.mode);
+                push(FLOW_T, tp.units, tp.slabs, tp.nunits, false, tp.in, 4, tp.out, tp.mode);
                 push(FLOW_TFINISH, tp.groups, nullptr, tp.ngroups, false, tp.in, 4, tp.out, tp.mode);
             }
         }
@@ -1351,7 +1344,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         d.units = reinterpret_cast<const TUnit*>(hp->arena + o_tu[i]);
         d.slabs = reinterpret_cast<const TSlab*>(hp->arena + o_ts[i]);
         d.groups = reinterpret_cast<const TGroup*>(hp->arena + o_tg[i]);
-        std::memcpy(d.cls_begin, tp.cls_begin, sizeof(d.cls_begin));
+        d.nunits = int(tp.units.size());
         d.ngroups = int(tp.groups.size());
         d.in = tp.in; d.out = tp.out; d.mode = tp.mode; d.bytes = tp.bytes; d.alg_bytes = tp.alg_bytes;
         hp->t.push_back(d);
@@ -2039,7 +2032,7 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
             const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
             if (ws.profile) prof_begin(M, stage_name(M, 0, st.idx), tp.alg_bytes, s);
             static_assert(TCOLS == 8, "T-form units are launched with the 8-column kernel");
-            if (const int nu = tp.cls_begin[3]; nu > 0)   // unit T-form: FP64 plans only
+            if (const int nu = tp.nunits; nu > 0)   // unit T-form: FP64 plans only
                 L(launch_k(ov, k_tform_f64<TCOLS>, unsigned((nu + 7) / 8), 256, 0, s, tp.units, nu, tp.slabs,
                            reinterpret_cast<const double*>(M->store), vin, vout, ws.part, alpha, add));
             if (tp.ngroups > 0)
@@ -2167,7 +2160,7 @@ hlrc_status run_dw(hlrc_hmat M, const Workspace& ws, double alpha_in, int op, co
             const int add = tp.mode != OUT_SET;
             const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
             const OutMap om = omap(tp.out);
-            const int nu = tp.cls_begin[3];
+            const int nu = tp.nunits;
             if (ws.profile) prof_begin(M, stage_name(M, 0, st.idx), tp.alg_bytes, s);
             if (nu > 0) {
                 L(launch_k(ov, k_tform_dw<NT>, unsigned((nu * NG + 7) / 8), 256, 0, s, tp.units, nu, tp.slabs, A,

@@ -75,13 +75,11 @@ constexpr int WIDE_THREADS = 224;     // 4 epilogue warps, 1 MMA warp, 2 produce
 constexpr int WIDE_PRODUCERS = 64;
 constexpr int WIDE_NS_N = 6;          // N-form stages (32 columns each): 2 CTAs per SM
 constexpr int WIDE_FLUSH = 2;         // N-form stages per FP32 accumulation (64 columns), then added in FP64
-// Column-cluster T-form stages (one tile each).  Most units have one tile or a
+// The column-cluster T-form has one stage (one tile).  Most units have one tile or a
 // few, so a unit is a chain of latencies and CTAs per SM count for more than
 // stages: 361 us with three stages and two CTAs (n = 20011, BF16, 40 vectors),
 // 258 us with two and three, 216 us with one and four (all of the tensor memory).
-constexpr int WIDE_NS_C = 1;
 constexpr int WIDE_LAG_N = WIDE_NS_N - 2;   // copy groups a producer keeps in flight
-constexpr int WIDE_LAG_C = WIDE_NS_C - 1;
 constexpr int WIDE_PF = WIDE_LAG_N + 1;     // N-form: column-table entries prefetched this many stages ahead
 constexpr int WIDE_WQ = WIDE_PF + WIDE_LAG_N + 1;   // ring of prefetched column-table entries
 constexpr int WIDE_ERR_WAIT = 2;      // device error word bit: a wait of a wide kernel ran out
@@ -99,10 +97,9 @@ constexpr int WIDE_BAR_BYTES = 256;   // mbarriers and the TMEM address
 constexpr int wide_smem_n() {
     return 1024 + WIDE_NS_N * WIDE_N_STAGE + WIDE_WQ_BYTES + WIDE_BAR_BYTES;
 }
-constexpr int wide_smem_c() { return 1024 + WIDE_NS_C * WIDE_C_STAGE + WIDE_C_TABLES + WIDE_BAR_BYTES; }
+constexpr int wide_smem_c() { return 1024 + WIDE_C_STAGE + WIDE_C_TABLES + WIDE_BAR_BYTES; }
 // the T-form epilogue transposes this many columns at a time through the stages
-constexpr int WIDE_C_ROUND = WIDE_NS_C * WIDE_C_STAGE / (WIDE_TERMS * 4) < WT_MAXN
-                                 ? WIDE_NS_C * WIDE_C_STAGE / (WIDE_TERMS * 4) : WT_MAXN;
+constexpr int WIDE_C_ROUND = WIDE_C_STAGE / (WIDE_TERMS * 4) < WT_MAXN ? WIDE_C_STAGE / (WIDE_TERMS * 4) : WT_MAXN;
 
 template <int FMT> struct WideT;
 template <> struct WideT<FMT_F16> {
@@ -327,15 +324,15 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
     pdl_wait(xs);
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-    WTBlk* sblk = reinterpret_cast<WTBlk*>(sm + WIDE_NS_C * WIDE_C_STAGE);
+    WTBlk* sblk = reinterpret_cast<WTBlk*>(sm + WIDE_C_STAGE);
     uint32_t* scol = reinterpret_cast<uint32_t*>(sblk + WT_MAXB);           // stacked column -> (block << 16) | column
     uint32_t* sdst = scol + WT_MAXN;                                        // its output entry,
     int* sexp = reinterpret_cast<int*>(sdst + WT_MAXN);                     // static exponent
     float* sscl = reinterpret_cast<float*>(sexp + WT_MAXN);                 // and scale
     uint32_t* sslab = reinterpret_cast<uint32_t*>(sscl + WT_MAXN);          // [tile][block] store offsets / 16
     uint64_t* full = reinterpret_cast<uint64_t*>(sslab + WT_MAXT * WT_MAXB);
-    uint64_t* empty = full + WIDE_NS_C;
-    uint64_t* accf = empty + WIDE_NS_C;
+    uint64_t* empty = full + 1;
+    uint64_t* accf = empty + 1;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(accf + 1);
 
     const WTUnit u = units[blockIdx.x];
@@ -345,10 +342,8 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
     for (int j = threadIdx.x; j < nb; j += WIDE_THREADS) sblk[j] = blks[u.blk0 + j];
     for (int i = threadIdx.x; i < nt * nb; i += WIDE_THREADS) sslab[i] = slabs[u.slab0 + i];
     if (threadIdx.x == 0) {
-        for (int i = 0; i < WIDE_NS_C; ++i) {
-            mbar_init(full + i, WIDE_PRODUCERS);
-            mbar_init(empty + i, 1);
-        }
+        mbar_init(full, WIDE_PRODUCERS);
+        mbar_init(empty, 1);
         mbar_init(accf, 1);
         mbar_init_fence();
     }
@@ -383,13 +378,10 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
         // ---------------------------------------------------- producers
         const int p = threadIdx.x - 160;
         const uint32_t s0 = smem_u32(sm);
-        bool ok = true;
-        for (int q = 0; q < nt && ok; ++q) {
-            const int slot = q % WIDE_NS_C;
-            if (q >= WIDE_NS_C) ok = wide_wait(empty + slot, uint32_t((q / WIDE_NS_C) - 1) & 1u, err, wc.limit_ns);
-            if (!ok) break;
+        for (int q = 0; q < nt; ++q) {
+            if (q > 0 && !wide_wait(empty, uint32_t(q - 1) & 1u, err, wc.limit_ns)) break;
             const WTTile tl = tiles[u.tile0 + q];
-            const uint32_t sa = s0 + uint32_t(slot) * WIDE_C_STAGE, sb = sa + 16384u;
+            const uint32_t sa = s0, sb = sa + 16384u;
             // A: split row k (tile entry), unit v -> M-atom v / 8 (8 KB apart), K-atom k / 8, row k % 8
             for (int i = p; i < 1024; i += WIDE_PRODUCERS) {
                 const int k = i >> 4, v = i & 15;
@@ -410,32 +402,24 @@ k_ctform_wide(const WTUnit* __restrict__ units, const WTBlk* __restrict__ blks, 
                 tc5::cp16(sb + uint32_t(n >> 3) * 1024u + swz(n & 7, jj), src, in ? 16u : 0u);
             }
             tc5::cp_commit();
-            if (q >= WIDE_LAG_C) {
-                tc5::cp_wait<WIDE_LAG_C>();
-                fence_async_smem();
-                if (!(wc.skip && q == WIDE_LAG_C)) mbar_arrive(full + (q - WIDE_LAG_C) % WIDE_NS_C);
-            }
+            tc5::cp_wait<0>();
+            fence_async_smem();
+            if (!(wc.skip && q == 0)) mbar_arrive(full);
         }
-        tc5::cp_wait<0>();
-        fence_async_smem();
-        if (ok)
-            for (int q = max(0, nt - WIDE_LAG_C); q < nt; ++q)
-                if (!(wc.skip && q == 0)) mbar_arrive(full + q % WIDE_NS_C);
     } else if (warp == 4) {
         // ------------------------------------------------------- MMA issue
         if (lane == 0) {
             const uint32_t id = tc5::idesc_f16(128, npad, WideT<FMT>::bf16, true, false);
             const uint32_t s0 = smem_u32(sm);
             for (int q = 0; q < nt; ++q) {
-                const int slot = q % WIDE_NS_C;
-                if (!wide_wait(full + slot, uint32_t(q / WIDE_NS_C) & 1u, err, wc.limit_ns)) break;
+                if (!wide_wait(full, uint32_t(q) & 1u, err, wc.limit_ns)) break;
                 tc_fence_after();
-                const uint32_t sa = s0 + uint32_t(slot) * WIDE_C_STAGE, sb = sa + 16384u;
+                const uint32_t sa = s0, sb = sa + 16384u;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     mma_f16(tmem, sdesc(sa + 2048u * j, 8192u, 1024u), sdesc(sb + 32u * j, 16u, 1024u), id,
                             (q > 0 || j > 0) ? 1u : 0u);
-                mma_commit(empty + slot);
+                mma_commit(empty);
             }
             // every MMA issued has completed before the epilogue reads TMEM
             // and before TMEM is freed (this wait does not give up on the

@@ -331,7 +331,7 @@ struct Store {
 
 struct TBuilder {
     TPass& P;
-    std::vector<std::pair<int64_t, TUnit>> tmp[3];  // (cost, unit) per class
+    std::vector<std::pair<int64_t, TUnit>> tmp;  // (cost, unit)
     explicit TBuilder(TPass& p) : P(p) {}
 
     // one output of `ncols` columns at `out`, fed by `slabs`
@@ -355,13 +355,13 @@ struct TBuilder {
             if (sb != uint32_t(P.slabs.size()) || runs.empty()) runs.push_back({sb, uint32_t(P.slabs.size())});
             if (runs.size() == 1) {
                 TUnit u{runs[0].first, runs[0].second, uint32_t(out + c0), uint16_t(c0), uint8_t(nc), TU_DIRECT};
-                tmp[0].push_back({cost(u), u});
+                tmp.push_back({cost(u), u});
             } else {
                 TGroup g{P.nslots, uint32_t(runs.size()), uint32_t(out + c0), uint32_t(nc)};
                 P.groups.push_back(g);
                 for (auto& r : runs) {
                     TUnit u{r.first, r.second, P.nslots++, uint16_t(c0), uint8_t(nc), 0};
-                    tmp[0].push_back({cost(u), u});
+                    tmp.push_back({cost(u), u});
                 }
             }
         }
@@ -373,16 +373,11 @@ struct TBuilder {
     }
     void finish() {
         P.units.clear();
-        for (int c = 0; c < 3; ++c) {
-            std::stable_sort(tmp[c].begin(), tmp[c].end(),
-                             [](const auto& a, const auto& b) { return a.first > b.first; });
-            P.cls_begin[c] = int(P.units.size());
-            for (auto& e : tmp[c]) {
-                P.units.push_back(e.second);
-                P.bytes += e.first * int64_t(sizeof(double));
-            }
+        std::stable_sort(tmp.begin(), tmp.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+        for (auto& e : tmp) {
+            P.units.push_back(e.second);
+            P.bytes += e.first * int64_t(sizeof(double));
         }
-        P.cls_begin[3] = int(P.units.size());
     }
 };
 

@@ -43,8 +43,7 @@ constexpr uint8_t GC_PACK2 = 0x80;
 
 struct TPass {
     std::vector<TSlab> slabs;
-    std::vector<TUnit> units;      // ordered by column class, then cost
-    int cls_begin[4] = {0, 0, 0, 0};  // units of class c: [cls_begin[c], cls_begin[c+1]); classes nc<=8,16,32
+    std::vector<TUnit> units;      // by cost (descending)
     std::vector<TGroup> groups;    // outputs with several units
     uint32_t nslots = 0;
     int in = V_X, out = V_T, mode = OUT_SET;
