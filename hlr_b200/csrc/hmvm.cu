@@ -2302,16 +2302,22 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 const double alpha = tp.mode == OUT_ADD ? 1.0 : alpha_in;   // plain adds pass coefficients down a tree
                 const OutMap om = omap(tp.out);
                 if (ws.profile) prof_begin(M, stage_name(M, 2, st.idx), tp.alg_bytes, s);
+                // The T-forms are launched plainly: their CTAs, started while
+                // the predecessor drains, crowd the SMs that empty first (8
+                // vectors, early -> plain, adjoint: FP32 n = 20011 286 -> 256 us,
+                // FP16/FP32 219 -> 201, FP16 182 -> 174, BFP 248 -> 246; op N of
+                // FP16/FP32 n = 9001 106 -> 103, n = 20011 177 -> 173; the other way
+                // FP16/FP32 n = 3001, adjoint, 53 -> 56)
                 if (M->precision == HLRC_PREC_BFP) {
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     if (tp.nmseg[FMT_I24] > 0) {
-                        L(launch_k(ov, k_ttform_bfp<true>, dim3(unsigned(tp.nmseg[FMT_I24]), unsigned(tp.msplit)), TC_WARPS * 32,
+                        L(launch_k(false, k_ttform_bfp<true>, dim3(unsigned(tp.nmseg[FMT_I24]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    bq_smem_t(true), s, tp.mseg[FMT_I24], tp.mcol, M->store, vec(tp.in), om, fpart,
                                    alpha, add));
                         ++nl;
                     }
                     if (tp.nmseg[FMT_I16] > 0) {
-                        L(launch_k(ov, k_ttform_bfp<false>, dim3(unsigned(tp.nmseg[FMT_I16]), unsigned(tp.msplit)), TC_WARPS * 32,
+                        L(launch_k(false, k_ttform_bfp<false>, dim3(unsigned(tp.nmseg[FMT_I16]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    bq_smem_t(false), s, tp.mseg[FMT_I16], tp.mcol, M->store, vec(tp.in), om, fpart,
                                    alpha, add));
                         ++nl;
@@ -2320,12 +2326,12 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                     const int n32 = tp.nmseg[FMT_F32];
                     float* fpart = reinterpret_cast<float*>(ws.mr_part);
                     if (tp.nmseg[FMT_BF16] > 0) {
-                        L(launch_k(ov, k_ttform_mr<FMT_BF16>, dim3(unsigned(n32 + tp.nmseg[FMT_BF16]), unsigned(tp.msplit)), TC_WARPS * 32,
+                        L(launch_k(false, k_ttform_mr<FMT_BF16>, dim3(unsigned(n32 + tp.nmseg[FMT_BF16]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s, tp.mseg[FMT_F32], n32,
                                    tp.mseg[FMT_BF16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add));
                         ++nl;
                     } else if (n32 + tp.nmseg[FMT_F16] > 0) {
-                        L(launch_k(ov, k_ttform_mr<FMT_F16>, dim3(unsigned(n32 + tp.nmseg[FMT_F16]), unsigned(tp.msplit)), TC_WARPS * 32,
+                        L(launch_k(false, k_ttform_mr<FMT_F16>, dim3(unsigned(n32 + tp.nmseg[FMT_F16]), unsigned(tp.msplit)), TC_WARPS * 32,
                                    tc_smem_bytes(TC_STAGE_TT, TC_STAGES_TT), s, tp.mseg[FMT_F32], n32,
                                    tp.mseg[FMT_F16], tp.mcol, M->store, vec(tp.in), om, fpart, alpha, add));
                         ++nl;
@@ -2359,15 +2365,16 @@ hlrc_status run_multi(hlrc_hmat M, const Workspace& ws, double alpha_in, int op,
                 const OutMap om = omap(np.out);
                 // the formats of one output tile run as separate grids, each
                 // adding its share to the output in a fixed launch order.
-                // Whole tiles of the FP32 and 16-bit kernels are launched
+                // The FP32 kernel and whole tiles of the 16-bit one are launched
                 // plainly: their one or two waves, started while the
                 // predecessor drains, crowd the SMs that empty first (FP32
-                // n = 20011 226 -> 250 us, FP16/FP32 n = 32768 adjoint
-                // 263 -> 274, batch of 4, 2 vectors 115 -> 121; the other way
+                // n = 20011 226 -> 250 us early, FP16/FP32 n = 32768 adjoint
+                // 263 -> 274, batch of 4, 2 vectors 115 -> 121; FP32 in clusters,
+                // n = 13001 105 -> 117, FP16/FP32 n = 9001 97 -> 103; the other way
                 // n = 65536 437 -> 432, BFP n = 20011 234 -> 229)
                 const bool early = ov && np.msplit > 1;
                 if (np.nmseg[FMT_F32] > 0) {
-                    L(launch_n(early, k_nform_d32<false>, k_nform_d32<true>,
+                    L(launch_n(false, k_nform_d32<false>, k_nform_d32<true>,
                                np.nmseg[FMT_F32], np.msplit, TC_WARPS * 32,
                                tc_smem_bytes(TC_STAGE_N32, TC_STAGES_D32), s, np.mseg[FMT_F32], np.mcol, M->store,
                                vec(np.vx), vec(np.vt), om, alpha, add));
