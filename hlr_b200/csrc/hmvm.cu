@@ -62,6 +62,7 @@ struct DevNPass {
     const MSeg* mseg_cp = nullptr;    // 64-vector N-form with cp.async: the other tiles
     int nmseg_cp = 0;
     int nseg2 = 0;
+    size_t ntiles = 0;                // tiles
     int warps = 8;                    // of the FP64 one-vector kernel at the default setting (nform_default)
     int split = 1;                    // CTAs per tile at the default setting (tile_split)
     int msplit = 1;                   // the same of the 8- to 32-vector kernels
@@ -94,6 +95,7 @@ struct DevTTPass {
     const TGroup* groups1 = nullptr;  // first finish level (long outputs), into the partial array
     int ngroups1 = 0;
     int64_t npart = 0;
+    size_t ntiles = 0;                // tiles (of every format)
     int warps = 8;                    // of the FP64 one-vector kernel at the default setting
     int split = 1;                    // CTAs per tile at the default setting (tile_split)
     int msplit = 1;                   // the same of the 8- to 32-vector kernels
@@ -270,6 +272,7 @@ struct hlrc_hmat_s {
     // run on the side stream beside the other passes (near_t_stage; -1: not),
     // and the partial sums it needs of its own
     int near_t[3] = {-1, -1, -1};
+    bool near_eager[3] = {false, false, false};   // beside in eager calls too (near_eager())
     double* part2 = nullptr;
     int64_t n_part2 = 0;
     bool nf_multi = false;             // multi-vector products take stages_nf too
@@ -463,7 +466,14 @@ int near_t_stage(const Plan& p, int op) {
     if (t.in != V_X || t.out != V_Y || t.mode != OUT_ADD_ALPHA || t.chunks.empty()) return -1;
     for (const GChunk& c : t.chunks)
         if (c.flags & TT_DIRECT) return -1;
-    return int(l.size()) - 1;
+    bool others = false;   // a pass to run beside (none in a matrix of dense leaves)
+    for (size_t i = 0; i + 1 < l.size(); ++i) {
+        const Stage& st = l[i];
+        others = others || (st.kind == 0 ? !p.tpasses[size_t(st.idx)].units.empty()
+                                         : st.kind == 1 ? !p.npasses[size_t(st.idx)].chunks.empty()
+                                                        : !p.ttpasses[size_t(st.idx)].chunks.empty());
+    }
+    return others ? int(l.size()) - 1 : -1;
 }
 
 ArenaLayout arena_layout(const Plan& p) {
@@ -1114,6 +1124,33 @@ hlrc_status plan_h_leaves(const hlrc_h_desc& d, hlrc_options o, Plan& p, double 
     return plan_h(hd, o, p, area);
 }
 
+// Does the transposed near field of an eager product run beside the chain?  The
+// fork and join are four calls of the host, which are saved only where the product
+// takes longer on the device than the host's calls, about 25 us: 2.5 us a launch, a
+// CTA 25 KB/us (stored in FP64; 17 otherwise) and all CTAs 5 MB/us, in line.  Adjoint,
+// eager, in line -> beside (estimate in brackets): 1D log n = 9001 (18) 30.5 -> 32 us,
+// n = 20011 (23) 25.5 -> 30.4, FP16/FP32 n = 9001 21.8 -> 24.5; exponential n = 1100 FP16/FP32
+// (23) 24.2 -> 26.6, sphere of 2048 triangles (24) 19.8 -> 23.7; the other way n = 24001 (26)
+// 28.1 -> 24.9, n = 28001 (29) 29.8 -> 26.8, exponential n = 1100 FP64 (28) 29.1 -> 27.2,
+// n = 3001 FP16/FP32 (34) 32.5 -> 26.6, n = 7001 FP64 56.6 -> 47.7.  A graph has no such calls.
+bool near_eager(hlrc_hmat_s* h, int op) {
+    if (h->near_t[op] < 0) return false;
+    const double rate = h->precision == HLRC_PREC_F64 ? 25e3 : 17e3;
+    double us = 0.0;
+    for (const Stage& st : h->stages[op]) {
+        const bool t = st.kind == 0, n = st.kind == 1;
+        const int launches = t ? h->t[size_t(st.idx)].launches()
+                               : n ? h->n[size_t(st.idx)].launches() : h->tt[size_t(st.idx)].launches();
+        const double bytes = double(t ? h->t[size_t(st.idx)].bytes
+                                      : n ? h->n[size_t(st.idx)].bytes : h->tt[size_t(st.idx)].bytes);
+        size_t ctas = t ? size_t(h->t[size_t(st.idx)].nunits) / 8 : 0;
+        if (n) ctas = h->n[size_t(st.idx)].ntiles * size_t(h->n[size_t(st.idx)].split);
+        if (st.kind == 2) ctas = h->tt[size_t(st.idx)].ntiles * size_t(h->tt[size_t(st.idx)].split);
+        us += 2.5 * launches + std::max(bytes / double(std::max<size_t>(1, ctas)) / rate, bytes / 5e6);
+    }
+    return us > 25.0;
+}
+
 // The passes of one-launch products (kernels_flow.cuh): the one-vector stages
 // of each op, with the finishes as passes of their own.  Only products whose
 // passes have at most FLOW_TILES tiles run this way, and none with tree sweeps:
@@ -1127,7 +1164,11 @@ hlrc_status plan_h_leaves(const hlrc_h_desc& d, hlrc_options o, Plan& p, double 
 // several CTAs (tile_split): n = 4096 exponential (62 MB of it) 45 us as one launch,
 // 23 us so split; where only the near field or little of the chain does, one launch
 // wins (sphere of 2048 triangles, 15 MB in all: 16 against 24 us), and its sums are
-// those of whole tiles in separate launches too.
+// those of whole tiles in separate launches too.  Op T / C of a
+// matrix of dense leaves, a T-form and its finish, is two launches (sphere of 512
+// triangles, two -> one: 11.6 -> 12.6 us).  At 256 tiles one launch of op T / C takes
+// 22.7 us on the device whatever the host, separate launches as long as the host's
+// calls: 1D log n = 9001 20.1 us with one host, 28.9 with another.
 constexpr int FLOW_TILES = 296;
 constexpr int64_t FLOW_SPLIT_BYTES = 16 << 20;
 void plan_flow(hlrc_hmat_s* h) {
@@ -1198,6 +1239,7 @@ void plan_flow(hlrc_hmat_s* h) {
                 push(FLOW_TFINISH, tp.groups, nullptr, tp.ngroups, false, tp.in, 4, tp.out, tp.mode);
             }
         }
+        if (op != HLRC_OP_N && F.nst <= 2) continue;
         if (!ok || F.nst == 0 || split_bytes > FLOW_SPLIT_BYTES) continue;
         h->flow[op] = F;
         for (const Stage& st : list)   // the same sums in separate launches
@@ -1365,6 +1407,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (f64) d.warps = nform_default(np.segs[FMT_F64].size(), np.chunks.size());
         size_t tiles = 0;   // a tile has one CTA for all formats
         for (int f = 0; f < NFMT; ++f) tiles = std::max(tiles, np.segs[f].size());
+        d.ntiles = tiles;
         if (np.cta_begin.empty()) d.split = tile_split(tiles, np.bytes, SPLIT_BYTES);
         d.msplit = tile_split(tiles, np.bytes, msplit_bytes(f64));
         d.vx = np.vx; d.vt = np.vt; d.out = np.out; d.mode = np.mode; d.bytes = np.bytes; d.alg_bytes = np.alg_bytes;
@@ -1459,6 +1502,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         if (f64) d.warps = ttform_default(tp.segs[FMT_F64].size(), tp.chunks.size());
         size_t tiles = 0;   // a CTA for each format of a tile
         for (int f = 0; f < NFMT; ++f) tiles += tp.segs[f].size();
+        d.ntiles = tiles;
         d.split = tile_split(tiles, tp.bytes, SPLIT_BYTES);
         d.msplit = tile_split(tiles, tp.bytes, msplit_bytes(f64));
         d.groups = reinterpret_cast<const TGroup*>(hp->arena + L.ttg[i]);
@@ -1507,6 +1551,7 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
 
     fill_info(p, L, hp->info);
     plan_flow(hp);
+    for (int op = 0; op < 3; ++op) hp->near_eager[op] = near_eager(hp, op);
     // Without room for the group T-forms' tables, products of more than 8 vectors
     // go in blocks of 8.
     const int64_t no_groups = hp->info.device_bytes;
@@ -2012,7 +2057,8 @@ hlrc_status run_single(hlrc_hmat M, const Workspace& ws, double alpha_in, int op
     // vector, adjoint, in line -> beside: uniform-H sphere of 32768 triangles
     // 87 -> 76 us, as H^2 102 -> 82 us; exponential n = 20011 FP64 208 -> 186, BFP
     // 116 -> 107, n = 50021 FP64 530 -> 506 us; 1D log n = 50000 44.7 -> 39.0 us).
-    const int beside = ws.part2 && ws.side && !ws.profile ? M->near_t[op] : -1;
+    const int beside = ws.part2 && ws.side && !ws.profile && M->near_t[op] >= 0 && (M->near_eager[op] || capturing(s0))
+                           ? M->near_t[op] : -1;
     if (beside >= 0) {
         L(cudaEventRecord(ws.ev_fork, s0));
         L(cudaStreamWaitEvent(ws.side, ws.ev_fork, 0));
