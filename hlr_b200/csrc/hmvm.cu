@@ -1542,6 +1542,13 @@ hlrc_status upload_plan(Plan& p, const hlrc_options& o, hlrc_hmat* out) {
         hp->near_t[op] = near_t_stage(p, op);
     }
     hp->nf_multi = p.nf_multi;
+    // an H^2 near field runs beside a chain of short dependent passes, which is
+    // longer: several CTAs a tile take SMs from it (sphere of 8192 triangles, op N,
+    // 30.4 us whole, 31.5 us split)
+    if (p.kind == 2)
+        for (const std::vector<Stage>& l : hp->stages_nf)
+            for (const Stage& st : l)
+                if (st.side) hp->n[size_t(st.idx)].split = 1;
     if (has_side(hp->stages_nf)) {
         if (const hlrc_status ss = side_create(hp->side_ws); ss != HLRC_OK) {
             cleanup();
