@@ -172,7 +172,7 @@ __device__ __forceinline__ void npack_q(const QNPack& pk, const uint8_t* A, cons
     const uint32_t vo = second ? pk.p[1].v_off : pk.p[0].v_off;
     const float sc = second ? pk.p[1].scale : pk.p[0].scale;
     const double* v = (vo & VEC_T) ? vt + (vo & ~VEC_T) : vx + vo;
-    const float vl = lane < ntot ? float(__ldca(v + (second ? lane - n0 : lane)) * double(sc)) : 0.f;
+    const float vl = lane < ntot ? float(ld_ordered(v + (second ? lane - n0 : lane)) * double(sc)) : 0.f;
     uint4 m[8];
     uint2 ml[FMT == FMT_I24 ? 8 : 1];
     load_pack<FMT>(A, pk.p[0].a16, pk.p[1].a16, n0, ntot, ld, lane, m, ml);
@@ -239,13 +239,13 @@ __device__ __forceinline__ void nflush_add_q(double* acc, int lane, double* red_
 }
 
 // a warp's share (packs cb + warp, cb + warp + W, ...) of one format's packs
-// of a tile, with the next descriptor read ahead
-template <int W, int FMT>
-__device__ __forceinline__ void npacks_q(uint32_t cb, uint32_t ce, int ld, const QNPack* __restrict__ packs,
+// of a tile, with the next descriptor read ahead (nxt: the first one, if it is
+// there: GOT)
+template <int W, int FMT, bool GOT>
+__device__ __forceinline__ void npacks_q(QNPack nxt, uint32_t cb, uint32_t ce, int ld, const QNPack* __restrict__ packs,
                                          const uint8_t* __restrict__ A, const double* vx, const double* vt, int warp, int lane, double* acc) {
     uint32_t c = cb + warp;
-    QNPack nxt{};
-    if (c < ce) nxt = ld_pack(packs + c);
+    if (!GOT && c < ce) nxt = ld_pack(packs + c);
     for (; c < ce; c += W) {
         const QNPack pk = nxt;
         if (c + W < ce) nxt = ld_pack(packs + c + W);
@@ -266,7 +266,13 @@ k_nform_q(const NSeg2* __restrict__ segs, const QNPack* __restrict__ packs, cons
     const NSeg2 sg = segs[blockIdx.x / S];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = int(blockIdx.x % S) * W + warp;
-    pdl_wait(vx, vt);
+    // the first descriptors before the wait (n = 20011 FP16 79.5 -> 78.7 us, n = 13001
+    // 46.1 -> 45.3; the 24-bit kernel has no registers for them, n = 6007 32.4 -> 35.4)
+    constexpr bool GOT = WIDE != FMT_I24;
+    QNPack first32{}, first16{};
+    if (GOT && sg.cb32 + slot < sg.ce32) first32 = ld_pack(packs + sg.cb32 + slot);
+    if (GOT && sg.cb16 + slot < sg.ce16) first16 = ld_pack(packs + sg.cb16 + slot);
+    pdl_wait();   // ld_ordered behind it
     if constexpr (WIDE == FMT_I24) {
         // the wide packs flushed before the 16-bit ones start: fewer live
         // registers next to the 24-bit loads
@@ -274,13 +280,13 @@ k_nform_q(const NSeg2* __restrict__ segs, const QNPack* __restrict__ packs, cons
             double a32[QFmt<WIDE>::R];
 #pragma unroll
             for (int r = 0; r < QFmt<WIDE>::R; ++r) a32[r] = 0.0;
-            npacks_q<S * W, WIDE>(sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, slot, lane, a32);
+            npacks_q<S * W, WIDE, GOT>(first32, sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, slot, lane, a32);
             nflush_q<WIDE>(a32, lane, red[warp]);
         }
         double a16[QFmt<F16>::R];
 #pragma unroll
         for (int r = 0; r < QFmt<F16>::R; ++r) a16[r] = 0.0;
-        npacks_q<S * W, F16>(sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, slot, lane, a16);
+        npacks_q<S * W, F16, GOT>(first16, sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, slot, lane, a16);
         __syncwarp();
         nflush_add_q<F16>(a16, lane, red[warp]);
     } else {
@@ -289,8 +295,8 @@ k_nform_q(const NSeg2* __restrict__ segs, const QNPack* __restrict__ packs, cons
         for (int r = 0; r < QFmt<WIDE>::R; ++r) a32[r] = 0.0;
 #pragma unroll
         for (int r = 0; r < QFmt<F16>::R; ++r) a16[r] = 0.0;
-        npacks_q<S * W, WIDE>(sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, slot, lane, a32);
-        npacks_q<S * W, F16>(sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, slot, lane, a16);
+        npacks_q<S * W, WIDE, GOT>(first32, sg.cb32, sg.ce32, sg.ld32, packs, A, vx, vt, slot, lane, a32);
+        npacks_q<S * W, F16, GOT>(first16, sg.cb16, sg.ce16, sg.ld16, packs, A, vx, vt, slot, lane, a16);
         nflush_q<WIDE>(a32, lane, red[warp]);
         __syncwarp();
         nflush_add_q<F16>(a16, lane, red[warp]);
@@ -423,9 +429,11 @@ k_ttform_qs(const MSeg* __restrict__ segs32, int n32, const MSeg* __restrict__ s
             const uint8_t* __restrict__ A, const double* vin, double* __restrict__ out, double* __restrict__ part,
             double alpha, int add) {
     pdl_trigger();
+    const bool wide = int(blockIdx.x) < n32;
+    const MSeg sg = wide ? segs32[blockIdx.x] : segs16[blockIdx.x - n32];
     pdl_wait(vin);
-    if (int(blockIdx.x) < n32) ttform_qs<W, WIDE>(segs32[blockIdx.x], cols, A, vin, out, part, alpha, add);
-    else ttform_qs<W, F16>(segs16[blockIdx.x - n32], cols, A, vin, out, part, alpha, add);
+    if (wide) ttform_qs<W, WIDE>(sg, cols, A, vin, out, part, alpha, add);
+    else ttform_qs<W, F16>(sg, cols, A, vin, out, part, alpha, add);
 }
 
 }  // namespace hlrc
