@@ -2983,7 +2983,7 @@ extern "C" hlrc_status hlrc_check_device_error(hlrc_hmat M, int* code) {
     DeviceGuard g(M->device);
     if (!g.ok) return fail(HLRC_ERR_CUDA, "cannot select device %d", M->device);
     HLRC_CUDA(cudaMemcpy(code, M->dev_err, sizeof(int), cudaMemcpyDeviceToHost));
-    HLRC_CUDA(zero_now(M->dev_err, sizeof(int)));
+    if (*code != 0) HLRC_CUDA(zero_now(M->dev_err, sizeof(int)));
     return HLRC_OK;
 }
 
